@@ -85,8 +85,7 @@ Batch::~Batch() {
     if (join_ != nullptr) cudaEventDestroy(join_);
     if (done_ != nullptr) cudaEventDestroy(done_);
     if (start_ != nullptr) cudaEventDestroy(start_);
-    if (host_args_ != nullptr) cudaFreeHost(host_args_);
-    if (device_args_ != nullptr) cudaFree(device_args_);
+    if (device_args_ != nullptr) cudaFreeAsync(device_args_, nullptr);
     if (wirelength_ != nullptr) cudaStreamDestroy(wirelength_);
     if (split_ != nullptr) cudaStreamDestroy(split_);
     if (stream_ != nullptr) cudaStreamDestroy(stream_);
@@ -97,13 +96,13 @@ void Batch::reserve(std::size_t bytes) {
     const std::size_t grown = std::max(bytes, 2 * capacity_);
     // The previous round has completed (rounds end with a synchronisation), so
     // neither buffer is in use.
-    if (host_args_ != nullptr) checkCuda(cudaFreeHost(host_args_), "Free batch staging");
-    if (device_args_ != nullptr) checkCuda(cudaFree(device_args_), "Free batch arguments");
-    host_args_ = nullptr;
+    if (device_args_ != nullptr) checkCuda(cudaFreeAsync(device_args_, stream_), "Free batch arguments");
     device_args_ = nullptr;
     capacity_ = 0;
-    checkCuda(cudaMallocHost(reinterpret_cast<void**>(&host_args_), grown), "Allocate batch staging");
-    checkCuda(cudaMalloc(reinterpret_cast<void**>(&device_args_), grown), "Allocate batch arguments");
+    staging_ = PinnedBlock(grown, "Allocate batch staging");
+    host_args_ = staging_.data();
+    checkCuda(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&device_args_), grown, devicePool(device_), stream_),
+              "Allocate batch arguments");
     capacity_ = grown;
 }
 

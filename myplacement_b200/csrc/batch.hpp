@@ -75,7 +75,8 @@ private:
     cudaEvent_t split_fork_ = nullptr, split_join_ = nullptr;
     cudaEvent_t fork_ = nullptr, join_ = nullptr;
     cudaEvent_t start_ = nullptr, done_ = nullptr;  // timed: the round's device time
-    unsigned char* host_args_ = nullptr;  // pinned staging of a round's argument blocks
+    PinnedBlock staging_;                // pinned staging of a round's argument blocks
+    unsigned char* host_args_ = nullptr;  // its bytes
     unsigned char* device_args_ = nullptr;
     std::size_t capacity_ = 0;
 

@@ -131,15 +131,20 @@ Engine::Engine(const Grid& grid, int device, uint64_t budget_bytes, Batch* batch
     const uint64_t uploaded_before = g_uploaded_bytes;
     buildBasis();
     h2d_bytes_ += g_uploaded_bytes - uploaded_before;
-    // The reduction publishes the scalars and the error flag into mapped pinned
-    // memory; the host polls it, with no copy or stream synchronisation on the
-    // evaluation's critical path.
-    checkCuda(cudaMallocHost(reinterpret_cast<void**>(&host_scalars_), sizeof(EvalScalars)), "pinned scalars");
-    std::memset(host_scalars_, 0, sizeof(EvalScalars));
-    const std::size_t slot_bytes = static_cast<std::size_t>(kRecords) * kRecordSlots * sizeof(unsigned long long);
-    checkCuda(cudaHostAlloc(reinterpret_cast<void**>(&host_slots_), slot_bytes, cudaHostAllocMapped),
-              "pinned evaluation record");
-    std::memset(host_slots_, 0, slot_bytes);
+}
+
+// The reduction publishes the scalars and the error flag into mapped pinned
+// memory; the host polls it, with no copy or stream synchronisation on the
+// evaluation's critical path.
+void Engine::reserveRecord() {
+    constexpr std::size_t kSlotBytes = static_cast<std::size_t>(kRecords) * kRecordSlots * sizeof(unsigned long long);
+    constexpr std::size_t kRudyBytes = 5 * sizeof(double);
+    record_ = PinnedBlock(kSlotBytes + kRudyBytes + sizeof(int), "pinned evaluation record");
+    // A sequence of 0 marks an empty record, whatever an earlier engine left in the block.
+    std::memset(record_.data(), 0, kSlotBytes + kRudyBytes + sizeof(int));
+    host_slots_ = reinterpret_cast<unsigned long long*>(record_.data());
+    host_rudy_ = reinterpret_cast<double*>(record_.data() + kSlotBytes);
+    host_error_ = reinterpret_cast<int*>(record_.data() + kSlotBytes + kRudyBytes);
 }
 
 void Engine::load(const Problem& p) {
@@ -191,10 +196,6 @@ Engine::~Engine() {
     }
     if (fork_ != nullptr) cudaEventDestroy(fork_);
     if (join_ != nullptr) cudaEventDestroy(join_);
-    if (host_scalars_ != nullptr) cudaFreeHost(host_scalars_);
-    if (host_rudy_ != nullptr) cudaFreeHost(host_rudy_);
-    if (host_error_ != nullptr) cudaFreeHost(host_error_);
-    if (host_slots_ != nullptr) cudaFreeHost(host_slots_);
     for (cudaEvent_t e : events_) cudaEventDestroy(e);
 }
 
@@ -388,8 +389,7 @@ void Engine::buildTensorCoreBasis(double max_scale) {
     checkCuda(cudaStreamSynchronize(stream_), "upload field scales");  // host_scales leaves scope
     tc_error_ = arena_.array<int>(1, "contraction error flag");
     checkCuda(cudaMemsetAsync(tc_error_, 0, sizeof(int), stream_), "clear error flag");
-    checkCuda(cudaMallocHost(reinterpret_cast<void**>(&host_error_), sizeof(int)), "pinned error flag");
-    *host_error_ = 0;
+    reserveRecord();
 
     // Output bounds |C| <= gain * max |data operand|, with a margin for FP32 rounding.
     constexpr double kMargin = 1.02;
@@ -1051,7 +1051,7 @@ const EvalScalars& Engine::sync(uint64_t ticket) {
     for (uint32_t m = expected_mask; m != 0; m &= m - 1) {
         const int k = __builtin_ctz(m);
         const unsigned long long bits = (slots[2 * k] & 0xffffffffULL) | ((slots[2 * k + 1] & 0xffffffffULL) << 32);
-        std::memcpy(&host_scalars_->v[k], &bits, sizeof(double));
+        std::memcpy(&host_scalars_.v[k], &bits, sizeof(double));
     }
     synced_ticket_ = std::max(synced_ticket_, ticket);
     // Profiling events are read once no later evaluation is in flight (reading them
@@ -1060,7 +1060,7 @@ const EvalScalars& Engine::sync(uint64_t ticket) {
     if ((slots[2 * kScalarCount] & 0xffffffffULL) != 0) {
         fail(MPGP_ERR_TIMEOUT, "A tcgen05 field contraction timed out waiting on its pipeline.");
     }
-    return *host_scalars_;
+    return host_scalars_;
 }
 
 void Engine::densityMetrics(const EvalScalars& s, bool with, mpgp_density_metrics& out) const {
@@ -1151,7 +1151,6 @@ void Engine::enableRudy(const mpgp_options& o) {
     rudy_pin_gradient_ =
         arena_.array<double2>(std::max<std::size_t>(1, static_cast<std::size_t>(wl_pin_count_)), "RUDY pin gradients");
     rudy_scalars_ = arena_.array<double>(5, "RUDY scalars");
-    checkCuda(cudaMallocHost(reinterpret_cast<void**>(&host_rudy_), 5 * sizeof(double)), "pinned RUDY scalars");
     checkCuda(cudaStreamSynchronize(stream_), "RUDY set-up");
 }
 

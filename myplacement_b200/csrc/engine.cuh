@@ -11,6 +11,7 @@
 #include "dct_tc.cuh"
 #include "field_tc.cuh"
 #include "kernels.cuh"
+#include "pinned.hpp"
 #include "setup.hpp"
 
 namespace mpgp {
@@ -278,7 +279,7 @@ private:
     double* rudy_net_weight_ = nullptr;
     double2* rudy_pin_gradient_ = nullptr;
     double* rudy_scalars_ = nullptr;
-    double* host_rudy_ = nullptr;
+    double* host_rudy_ = nullptr;          // in the pinned record
     int wl_net_count_ = 0;
     int wl_pin_count_ = 0;
 
@@ -361,14 +362,17 @@ private:
     int* tc_row_exp_ = nullptr;
     TcScales* tc_scales_ = nullptr;
     int* tc_error_ = nullptr;
-    int* host_error_ = nullptr;
+    int* host_error_ = nullptr;            // in the pinned record
     // Evaluation results published by the reduction into mapped pinned memory
     // (ReduceArgs::host_slots), the scalars the current evaluation writes, and
     // the cache of the latest value of every scalar.
     // kRecords records of kRecordSlots slots; launch k publishes into record k % kRecords.
     static constexpr int kRecords = 2;
     static constexpr int kRecordSlots = 2 * (kScalarCount + 1);
+    // One pinned block holds them, the error flag's and the RUDY scalars' copies.
+    PinnedBlock record_;
     unsigned long long* host_slots_ = nullptr;
+    void reserveRecord();
     uint32_t record_mask_[kRecords] = {};       // the scalars the record's evaluation writes
     uint32_t record_sequence_[kRecords] = {};   // its sequence (the record's tag)
     uint64_t record_ticket_[kRecords] = {};     // its ticket
@@ -401,7 +405,7 @@ private:
     double* partials_e_ = nullptr;
     double* partials_g_ = nullptr;
     double* scalars_ = nullptr;
-    EvalScalars* host_scalars_ = nullptr;
+    EvalScalars host_scalars_{};
     bool last_gradient_ = false;
     bool last_propose_ = false;
 
