@@ -270,23 +270,14 @@ int mpgp_backend_rudy(mpgp_backend* b, const mpgp_options* options, const double
                                    r.maximum_utilization, r.p95_utilization, r.energy};
         std::copy(values, values + 10, metrics);
         if (calculate_gradient) {
-            mpgp::EvalRequest q;
-            q.mode = mpgp::kGiven;
-            q.positions = e.scratchPositions();
-            q.smoothing = 1.0;
-            q.gradient = true;
-            q.wire_out = b->wire;
-            q.density_out = b->density;
-            q.rudy_out = b->rudy;
-            q.rudy = true;
-            q.rudy_weight = 1.0;
-            const mpgp::EvalScalars& s = e.evaluate(q);
-            *energy = s.v[mpgp::kRudyEnergy];
+            // The maps, adjoints and energy are those that rudyEvaluate just formed.
+            e.rudyGradient(e.scratchPositions(), b->rudy);
+            *energy = r.energy;
             if (b->particles > 0) {
                 mpgp::checkCuda(cudaMemcpyAsync(gradient, b->rudy, bytes, cudaMemcpyDeviceToHost, e.stream()),
                                 "Download RUDY gradients");
-                mpgp::checkCuda(cudaStreamSynchronize(e.stream()), "Synchronize RUDY evaluation");
             }
+            e.requireHealthy();
         }
     });
 }

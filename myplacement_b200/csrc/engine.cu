@@ -1163,6 +1163,8 @@ RudyArgs Engine::rudyArgs(const RudyGrid& g, const double2* positions, bool with
     a.net_start = net_start_;
     a.net_weight = rudy_net_weight_;
     a.net_count = wl_net_count_;
+    a.work = block_work_;
+    a.work_count = wl_blocks_;
     a.pin_slot = pin_slot_;
     a.pin_gradient = rudy_pin_gradient_;
     a.llx = region_.llx;
@@ -1246,6 +1248,24 @@ RudyReport Engine::rudyEvaluate(const double2* positions, bool validation) {
         r.p95_utilization = utilization[index];
     }
     return r;
+}
+
+void Engine::rudyGradient(const double2* positions, double2* out) {
+    const RudyGrid& g = rudy_main_;
+    require(g.columns > 0 && g.capacity_h > 0.0 && g.capacity_v > 0.0, "A RUDY gradient needs positive capacities.");
+    const RudyArgs ra = rudyArgs(g, positions, true);
+    launchRudyTables(ra, stream_);
+    launchRudyGradient(ra, stream_);
+    launchRudyGather(particle_pin_start_, rudy_pin_gradient_, static_cast<int>(movable_count_),
+                     static_cast<int>(particle_count_), out, stream_);
+    launches_ += 4;
+}
+
+void Engine::requireHealthy() {
+    checkCuda(cudaMemcpyAsync(host_error_, tc_error_, sizeof(int), cudaMemcpyDeviceToHost, stream_),
+              "Download contraction status");
+    checkCuda(cudaStreamSynchronize(stream_), "Synchronize the engine");
+    if (*host_error_ != 0) fail(MPGP_ERR_TIMEOUT, "A tcgen05 field contraction timed out waiting on its pipeline.");
 }
 
 void Engine::depositLayers(const double2* positions, int64_t* movable, int64_t* macro, int64_t* filler) {

@@ -216,6 +216,11 @@ public:
     void setRudyModel(int model, double temperature);
     [[nodiscard]] double rudyMinimumSpan() const { return rudy_minimum_span_; }
     RudyReport rudyEvaluate(const double2* positions, bool validation);
+    // The subgradient per particle (device array) of the energy whose maps the last
+    // rudyEvaluate of the main grid formed, at the same positions; launched, not waited for.
+    void rudyGradient(const double2* positions, double2* out);
+    // Waits for the engine stream and fails if a field contraction has ever timed out.
+    void requireHealthy();
     [[nodiscard]] int rudyBins() const { return rudy_main_.columns * rudy_main_.rows; }
 
     // Solves the field of an arbitrary FP64 deviation map (parity hook).

@@ -158,6 +158,8 @@ struct RudyArgs {
     const int* net_start;
     const double* net_weight;     // FP64 weights in bucket order
     int net_count;
+    const int4* work;             // the wirelength pass's work items (WirelengthArgs::block_work)
+    int work_count;
     const int* pin_slot;
     double2* pin_gradient;        // particle-ordered pin slots (gradient pass)
     double llx, lly, urx, ury;    // core region
@@ -177,12 +179,14 @@ struct RudyArgs {
     double* table;                  // 2 x (rows + 1) x (columns + 1) summed-area tables of the adjoints
     double* partials;               // per block: energy, H total, V total, proxy, max utilisation
 };
-int rudyBlocks(int count);
 void launchRudyDeposit(const RudyArgs& args, cudaStream_t stream);
 void launchRudyPrefix(const RudyArgs& args, cudaStream_t stream);
 void launchRudyMetrics(const RudyArgs& args, int blocks, cudaStream_t stream);
 void launchRudyTables(const RudyArgs& args, cudaStream_t stream);
 void launchRudyGradient(const RudyArgs& args, cudaStream_t stream);
+// out[i]: the sum of particle i's RUDY pin slots (zero for fillers).
+void launchRudyGather(const int* particle_pin_start, const double2* pin_gradient, int movable_count,
+                      int particle_count, double2* out, cudaStream_t stream);
 
 // ---- deterministic reduction of all partials into the scalar block ----------------------
 // Source row r is partials[r * stride + column]; the producers write their
