@@ -20,6 +20,7 @@
 #include "session.hpp"
 #include "server.hpp"
 #include "setup.hpp"
+#include "transfer.hpp"
 
 namespace {
 
@@ -51,12 +52,12 @@ int guarded(F&& body) {
 
 struct mpgp_backend {
     std::unique_ptr<mpgp::Engine> engine;
+    std::unique_ptr<mpgp::HostTransfer> transfer;  // on the engine's stream; none without particles
     double2* wire = nullptr;
     double2* density = nullptr;
     double2* rudy = nullptr;
     int rudy_columns = 0, rudy_rows = 0;
     int64_t particles = 0;
-    std::vector<double2> host;
 };
 
 struct mpgp_session {
@@ -131,7 +132,10 @@ int mpgp_backend_create(const mpgp_layout* layout, int device, uint64_t maximum_
         backend->particles = problem.particle_count;
         backend->wire = backend->engine->newParticleArray("wire gradients");
         backend->density = backend->engine->newParticleArray("density gradients");
-        backend->host.resize(static_cast<std::size_t>(problem.particle_count));
+        if (backend->particles > 0) {
+            backend->transfer = std::make_unique<mpgp::HostTransfer>(
+                backend->engine->stream(), sizeof(double2) * static_cast<std::size_t>(backend->particles));
+        }
         *out = backend.release();
     });
     if (rc != MPGP_OK) {
@@ -154,14 +158,21 @@ int mpgp_backend_evaluate(mpgp_backend* b, const double* positions, double smoot
         mpgp::Engine& e = *b->engine;
         mpgp::checkCuda(cudaSetDevice(e.device()), "Select CUDA device for evaluation");
         const std::size_t bytes = sizeof(double2) * static_cast<std::size_t>(b->particles);
-        for (int64_t i = 0; i < 2 * b->particles; ++i) {
-            if (!std::isfinite(positions[i])) {
-                mpgp::fail(MPGP_ERR_NON_FINITE, "CUDA placement positions must be finite.");
-            }
-        }
+        const std::size_t values = 2 * static_cast<std::size_t>(b->particles);
+        const mpgp::HostTransfer::Call call(b->transfer.get());
         if (b->particles > 0) {
-            mpgp::checkCuda(cudaMemcpyAsync(e.scratchPositions(), positions, bytes, cudaMemcpyHostToDevice, e.stream()),
-                      "Upload CUDA particle positions");
+            // Positions that are not finite are refused with the positions of the last
+            // evaluation left in place: small arrays are checked first, larger ones while they
+            // are copied to the wire gradient's array, from which a kernel takes them.
+            mpgp::HostTransfer& t = *b->transfer;
+            const bool finite = t.large() ? t.upload(positions, reinterpret_cast<double*>(b->wire), values, true)
+                                           : mpgp::HostTransfer::allFinite(positions, values);
+            if (!finite) mpgp::fail(MPGP_ERR_NON_FINITE, "CUDA placement positions must be finite.");
+            if (t.large()) {
+                mpgp::launchCopyPositions(b->wire, e.scratchPositions(), static_cast<int>(b->particles), e.stream());
+            } else {
+                t.upload(positions, reinterpret_cast<double*>(e.scratchPositions()), values, false);
+            }
         }
         mpgp::EvalRequest q;
         q.mode = mpgp::kGiven;
@@ -170,19 +181,17 @@ int mpgp_backend_evaluate(mpgp_backend* b, const double* positions, double smoot
         q.gradient = calculate_gradient != 0;
         q.wire_out = b->wire;
         q.density_out = b->density;
-        const mpgp::EvalScalars& s = e.evaluate(q);
+        const uint64_t ticket = e.launch(q);
+        const bool download = calculate_gradient && b->particles > 0;
+        if (download) b->transfer->startDownload({{b->wire, wire_gradient, bytes}, {b->density, density_gradient, bytes}});
+        const mpgp::EvalScalars& s = e.sync(ticket);
         out->hpwl = s.v[mpgp::kHpwl];
         out->smooth_wirelength = s.v[mpgp::kSmooth];
         out->electrostatic_energy = e.energy(s);
         e.densityMetrics(s, true, out->optimizer_density);
         e.densityMetrics(s, false, out->design_density);
-        if (calculate_gradient && b->particles > 0) {
-            mpgp::checkCuda(cudaMemcpyAsync(wire_gradient, b->wire, bytes, cudaMemcpyDeviceToHost, e.stream()),
-                      "Download CUDA wire gradients");
-            mpgp::checkCuda(cudaMemcpyAsync(density_gradient, b->density, bytes, cudaMemcpyDeviceToHost, e.stream()),
-                      "Download CUDA density gradients");
-            mpgp::checkCuda(cudaStreamSynchronize(e.stream()), "Synchronize CUDA placement evaluation");
-        }
+        if (download) b->transfer->finishDownload();
+        if (b->transfer != nullptr) b->transfer->settled();  // the evaluation came after the upload
         if (!std::isfinite(out->smooth_wirelength) || !std::isfinite(out->hpwl) ||
             !std::isfinite(out->electrostatic_energy)) {
             mpgp::fail(MPGP_ERR_NON_FINITE, "CUDA global-placement evaluation produced a non-finite metric.");
@@ -259,9 +268,10 @@ int mpgp_backend_rudy(mpgp_backend* b, const mpgp_options* options, const double
                       "The backend's RUDY grid is fixed by its first use.");
         e.setRudyModel(options->rudy_penalty_model, options->rudy_softplus_temperature);
         const std::size_t bytes = sizeof(double2) * static_cast<std::size_t>(b->particles);
+        const mpgp::HostTransfer::Call call(b->transfer.get());
         if (b->particles > 0) {
-            mpgp::checkCuda(cudaMemcpyAsync(e.scratchPositions(), positions, bytes, cudaMemcpyHostToDevice, e.stream()),
-                            "Upload CUDA particle positions");
+            b->transfer->upload(positions, reinterpret_cast<double*>(e.scratchPositions()),
+                                2 * static_cast<std::size_t>(b->particles), false);
         }
         e.setRudyCapacity(false, horizontal_capacity, vertical_capacity);
         const mpgp::RudyReport r = e.rudyEvaluate(e.scratchPositions(), false);
@@ -273,12 +283,11 @@ int mpgp_backend_rudy(mpgp_backend* b, const mpgp_options* options, const double
             // The maps, adjoints and energy are those that rudyEvaluate just formed.
             e.rudyGradient(e.scratchPositions(), b->rudy);
             *energy = r.energy;
-            if (b->particles > 0) {
-                mpgp::checkCuda(cudaMemcpyAsync(gradient, b->rudy, bytes, cudaMemcpyDeviceToHost, e.stream()),
-                                "Download RUDY gradients");
-            }
+            if (b->particles > 0) b->transfer->startDownload({{b->rudy, gradient, bytes}});
             e.requireHealthy();
+            if (b->particles > 0) b->transfer->finishDownload();
         }
+        if (b->transfer != nullptr) b->transfer->settled();  // rudyEvaluate waits for the stream
     });
 }
 

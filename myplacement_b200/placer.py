@@ -270,8 +270,9 @@ class CudaPlacementBackend:
         if positions.shape[0] != 2 * self.particle_count:
             raise ValueError("CUDA placement positions do not match the particle count.")
         out = _abi.Evaluation()
-        wire = np.zeros(2 * self.particle_count)
-        density = np.zeros(2 * self.particle_count)
+        # The engine writes every component; a candidate evaluation needs no arrays at all.
+        wire = np.empty(2 * self.particle_count) if calculate_gradient else None
+        density = np.empty(2 * self.particle_count) if calculate_gradient else None
         check(self.lib.mpgp_backend_evaluate(self.handle, _ptr(positions, _d), smoothing, int(calculate_gradient),
                                              C.byref(out), _ptr(wire, _d), _ptr(density, _d)))
         result = {
@@ -312,7 +313,7 @@ class CudaPlacementBackend:
         positions = np.ascontiguousarray(positions, np.float64).reshape(-1)
         metrics = np.empty(10)
         energy = C.c_double(0.0)
-        grad = np.zeros(positions.size)
+        grad = np.empty(positions.size) if gradient else None
         check(self.lib.mpgp_backend_rudy(self.handle, C.byref(options), _ptr(positions, _d), float(capacity[0]),
                                          float(capacity[1]), int(gradient), _ptr(metrics, _d), C.byref(energy),
                                          _ptr(grad, _d)))
