@@ -858,6 +858,26 @@ __global__ void __launch_bounds__(kThreads) basisRangeKernel(BasisShape b, unsig
     }
 }
 
+// The spectral divide (ElectrostaticField.cpp:212-221): 1/(4 Nx Ny) / (kx^2 + ky^2), DC removed,
+// and its largest value (of non-negative floats, so their bits compare alike).
+__global__ void __launch_bounds__(kThreads) spectralScaleKernel(BasisShape b, float* scale, unsigned long long* top) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int l = blockIdx.y;
+    float v = 0.0f;
+    if (k < b.nx) {
+        constexpr double kHalfTurn = 3.141592653589793238462643383279502884;
+        const double normalization = 1.0 / (4.0 * static_cast<double>(b.nx) * static_cast<double>(b.ny));
+        const double wave_y = kHalfTurn * static_cast<double>(l) / b.height;
+        const double wave_x = kHalfTurn * static_cast<double>(k) / b.width;
+        const double denominator = wave_x * wave_x + wave_y * wave_y;
+        v = denominator <= kEpsilon ? 0.0f : static_cast<float>(normalization / denominator);
+        scale[static_cast<size_t>(l) * b.nx + k] = v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(top, static_cast<unsigned long long>(__float_as_uint(v)));
+}
+
 struct BasisPlanes {
     __half* data[kBasisCount];
     int ld[kBasisCount];
@@ -883,16 +903,25 @@ __global__ void __launch_bounds__(kThreads) basisPlanesKernel(BasisShape b, Basi
 }
 
 void buildBasisPlanes(int nx, int ny, double width, double height, const SplitMatrix (&out)[kBasisCount],
-                      unsigned long long* scratch, int (&exponents)[kBasisCount],
-                      double (&max_row_l1)[kBasisCount], cudaStream_t stream) {
+                      float* scale, unsigned long long* scratch, int (&exponents)[kBasisCount],
+                      double (&max_row_l1)[kBasisCount], double& max_scale, cudaStream_t stream) {
     const BasisShape shape{nx, ny, width, height};
     const dim3 grid(static_cast<unsigned>(std::max(nx, ny)), kBasisCount);
-    checkCuda(cudaMemsetAsync(scratch, 0, 2 * kBasisCount * sizeof(unsigned long long), stream), "basis ranges");
+    checkCuda(cudaMemsetAsync(scratch, 0, kBasisRanges * sizeof(unsigned long long), stream), "basis ranges");
+    spectralScaleKernel<<<dim3(static_cast<unsigned>(ceilDiv(nx, kThreads)), static_cast<unsigned>(ny)), kThreads, 0,
+                          stream>>>(shape, scale, scratch + 2 * kBasisCount);
+    checkCuda(cudaGetLastError(), "Launch the spectral scale");
     basisRangeKernel<<<grid, kThreads, 0, stream>>>(shape, scratch);
     checkCuda(cudaGetLastError(), "Launch the basis range pass");
-    unsigned long long ranges[2 * kBasisCount] = {};
+    unsigned long long ranges[kBasisRanges] = {};
     checkCuda(cudaMemcpyAsync(ranges, scratch, sizeof(ranges), cudaMemcpyDeviceToHost, stream), "basis ranges");
     checkCuda(cudaStreamSynchronize(stream), "basis ranges");
+    {
+        const uint32_t bits = static_cast<uint32_t>(ranges[2 * kBasisCount]);
+        float top = 0.0f;
+        std::memcpy(&top, &bits, sizeof(float));
+        max_scale = static_cast<double>(top);
+    }
     BasisPlanes planes{};
     for (int t = 0; t < kBasisCount; ++t) {
         double top = 0.0, row = 0.0;

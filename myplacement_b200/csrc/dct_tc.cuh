@@ -139,10 +139,12 @@ int splitHost(const std::vector<double>& values, int rows, int cols, int ld, std
 //   5 syw[r][l]  = (pi l / height) 2 sin(pi l (2r+1) / 2ny) DST-III along y times the wave number
 // The planes go to out[t]; exponents[t] and max_row_l1[t] (the largest row sum
 // of |values|, which bounds |A x| / max |x|) come back to the host.
+// `scale` (ny x nx) receives the spectral divide and max_scale its largest value.
 constexpr int kBasisCount = 6;
-void buildBasisPlanes(int nx, int ny, double width, double height, const SplitMatrix (&out)[kBasisCount],
+constexpr int kBasisRanges = 2 * kBasisCount + 1;  // scratch words
+void buildBasisPlanes(int nx, int ny, double width, double height, const SplitMatrix (&out)[kBasisCount], float* scale,
                       unsigned long long* scratch, int (&exponents)[kBasisCount],
-                      double (&max_row_l1)[kBasisCount], cudaStream_t stream);
+                      double (&max_row_l1)[kBasisCount], double& max_scale, cudaStream_t stream);
 // Splits the FP32 source S with one exponent per row (row_exp), folds max |S| into
 // scales->max_source and clears the magnitudes the forward contractions fold into.
 void launchSplitSource(const float* source, const SplitMatrix& out, int cols, int* row_exp, TcScales* scales,

@@ -397,6 +397,25 @@ __global__ void copyPositionsKernel(const double2* source, double2* destination,
     }
 }
 
+// applyPositions' clamp (AdaptiveGlobalPlacer.cpp:185-198) of `count` positions.
+__global__ void clampPositionsKernel(const double2* source, const double2* size, double2* destination, int count,
+                                     double llx, double lly, double urx, double ury) {
+    releaseNext();
+    waitForPrior();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const auto clamp = [](double value, double extent, double low, double high) {
+        const double least = low + extent * 0.5;
+        const double most = high - extent * 0.5;
+        if (!(least <= most)) return (low + high) * 0.5;
+        const double below = most < value ? most : value;
+        return least < below ? below : least;
+    };
+    const double2 p = source[i];
+    const double2 s = size[i];
+    destination[i] = make_double2(clamp(p.x, s.x, llx, urx), clamp(p.y, s.y, lly, ury));
+}
+
 }  // namespace
 
 void launchScatter(const ScatterArgs& args, int blocks, cudaStream_t stream) {
@@ -435,6 +454,13 @@ void launchCopyPositions(const double2* source, double2* destination, int count,
     const int blocks = std::max(1, std::min(ceilDiv(count, kThreads), 4 * sms));
     launchChained("Launch the checkpoint copy", copyPositionsKernel, dim3(blocks), dim3(kThreads), 0, stream, source,
                   destination, count);
+}
+
+void launchClampPositions(const double2* source, const double2* size, double2* destination, int count, double llx,
+                          double lly, double urx, double ury, cudaStream_t stream) {
+    if (count <= 0) return;
+    launchChained("Launch the position clamp", clampPositionsKernel, dim3(ceilDiv(count, kThreads)), dim3(kThreads), 0,
+                  stream, source, size, destination, count, llx, lly, urx, ury);
 }
 
 void launchVelocity(const double2* next, const double2* previous, double2* velocity, int count, cudaStream_t stream) {

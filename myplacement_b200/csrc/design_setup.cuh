@@ -1,0 +1,86 @@
+// A session's problem built on the device from the caller's design (design_setup.cu): the module
+// map, the pin CSR's source, the static density layers, the fillers' sizes and the particle
+// arrays.  Every value is the one setup.cpp forms (the same operations in the same order), so
+// a session is the same whichever path set it up.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <cstdint>
+#include <functional>
+
+#include "ingest.cuh"
+#include "setup.hpp"
+
+namespace mpgp {
+
+// The rule of a session's set-up: the device takes designs of at least this many modules and
+// pins whose scratch fits the budget (deviceSetupBytes).  Whole placements of two iterations
+// on a B200 with 16 host CPUs, host set-up against device set-up: 25,000 items 1.7 / 1.8 ms,
+// 51,000 1.96 / 1.72, 101,000 2.57 / 2.17, 226,000 5.9 / 2.8, 1.06 million 20.2 / 6.5.  The
+// host's part that is left is the validation, the module lists and sums that must be added in
+// order; below the line both are launch and allocation latency.
+constexpr int64_t kDeviceSetupItems = int64_t{1} << 15;
+
+// More than the set-up's transient device memory and the net layout's lasting arrays together.
+uint64_t deviceSetupBytes(const mpgp_design& design, int bins);
+
+// The design's modules on the device: scratch that lives until the set-up is done.
+struct DeviceModules {
+    int count = 0;
+    double* width = nullptr;
+    double* height = nullptr;
+    double* x = nullptr;
+    double* y = nullptr;
+    int* orientation = nullptr;      // null: all N
+    int* movable = nullptr;          // particle -> module
+    int* particle = nullptr;         // module -> particle, -1 for fixed modules
+    int* pins = nullptr;             // pins per module
+};
+void launchMapModules(const DeviceModules& modules, int movable, cudaStream_t stream);
+void launchCountPins(const int* pin_module, int pins, int* count, cudaStream_t stream);
+
+// What the host needs to know of the static layers: their sums in bin order.
+struct StaticSums {
+    double fixed = 0.0;      // physical areas
+    double dark = 0.0;
+    double placeable = 0.0;  // sum of bin area - dark
+    double charge = 0.0;     // sum of t * (fixed + dark), DensityMap::metrics(false) of the static map
+};
+
+// The static layers (staticDensity) formed per bin; static_charge (device, per bin) receives
+// t * (fixed + dark).  Waits for the stream.
+StaticSums staticLayersOnDevice(const mpgp_design& design, const DerivedDesign& derived, int bins_x, int bins_y,
+                                double target_density, double* static_charge, const BudgetHeadroom& headroom,
+                                cudaStream_t stream);
+
+// The movable modules' areas inside the core in ascending order (createFillers), in `sorted`
+// (device, `movable` doubles); areas of at most kEpsilon come last, as infinities.  Launched,
+// not waited for.
+void sortAreasOnDevice(const DeviceModules& modules, int movable, const Rect2& core, double* sorted,
+                       const BudgetHeadroom& headroom, cudaStream_t stream);
+
+// Hands `count` doubles of a device array to consume(values, count) piece by piece in order,
+// through two pinned slots: the next piece comes down while one is consumed.
+void readDown(const double* device, std::size_t count, const std::function<void(const double*, std::size_t)>& consume,
+              cudaStream_t stream);
+
+// The particle arrays (buildProblemParticles) and initial positions: movable modules, then fillers.
+struct ParticleArrays {
+    double2* size = nullptr;
+    unsigned char* layer = nullptr;
+    double* charge = nullptr;
+    double* precond = nullptr;
+    double2* position = nullptr;
+    const double2* filler_position = nullptr;  // device
+    double filler_width = 0.0, filler_height = 0.0;
+    int movable = 0;
+    int count = 0;
+    double target_density = 0.0;
+    double nominal_row_height = 0.0;
+    double average_area = 0.0;  // of the movable modules
+};
+void launchParticles(const DeviceModules& modules, const ParticleArrays& arrays, cudaStream_t stream);
+
+}  // namespace mpgp

@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <mutex>
 #include <string>
 #include <atomic>
@@ -22,7 +23,9 @@
 
 #include "batch.hpp"
 #include "common.cuh"
+#include "design_setup.cuh"
 #include "ingest.cuh"
+#include "transfer.hpp"
 
 namespace mpgp {
 
@@ -168,7 +171,6 @@ void Engine::loadParticles(const Problem& p) {
     particle_count_ = p.particle_count;
     const uint64_t uploaded_before = g_uploaded_bytes;
     uploadStatic(p);
-    allocateGroups();
     h2d_bytes_ += g_uploaded_bytes - uploaded_before;
     checkCuda(cudaStreamSynchronize(stream_), "Engine setup");
     if (batch_ != nullptr) {
@@ -214,24 +216,16 @@ double2* Engine::newParticleArray(const char* what) {
     return p;
 }
 
-void Engine::uploadStatic(const Problem& p) {
+void Engine::allocateParticles() {
     const std::size_t n = static_cast<std::size_t>(std::max<int64_t>(1, particle_count_));
-    std::vector<double2> size(static_cast<std::size_t>(particle_count_));
-    std::vector<unsigned char> layer(static_cast<std::size_t>(particle_count_));
-    for (int64_t i = 0; i < particle_count_; ++i) {
-        size[i] = make_double2(p.width[i], p.height[i]);
-        layer[i] = static_cast<unsigned char>(p.layer[i]);
-    }
     size_ = arena_.array<double2>(n, "particle sizes");
     layer_ = arena_.array<unsigned char>(n, "particle layers");
     charge_ = arena_.array<double>(n, "particle charge areas");
     precond_ = arena_.array<double>(n, "preconditioner");
     scratch_positions_ = arena_.array<double2>(n, "uploaded positions");
-    upload(size_, size, stream_);
-    upload(layer_, layer, stream_);
-    upload(charge_, p.charge, stream_);
-    if (!p.precond_base.empty()) upload(precond_, p.precond_base, stream_);
+}
 
+void Engine::allocateDensity() {
     const std::size_t bins = static_cast<std::size_t>(bin_count_);
     layers_ = arena_.array<unsigned long long>(3 * bins, "fixed-point density layers");
     totals_ = arena_.array<unsigned long long>(4, "density layer totals");
@@ -239,6 +233,36 @@ void Engine::uploadStatic(const Problem& p) {
     source_ = arena_.array<float>(bins, "density source");
     checkCuda(cudaMemsetAsync(layers_, 0, 3 * bins * sizeof(unsigned long long), stream_), "clear layers");
     checkCuda(cudaMemsetAsync(totals_, 0, 4 * sizeof(unsigned long long), stream_), "clear totals");
+}
+
+void Engine::allocatePartials() {
+    scatter_blocks_ = ceilDiv(std::max<int64_t>(1, particle_count_), kThreads);
+    gather_blocks_ = gatherBlocks(static_cast<int>(std::min<int64_t>(particle_count_, 1 << 30)));
+    metrics_fused_ = metricsSplitFits(bins_x_);
+    metrics_blocks_ = metrics_fused_ ? bins_y_ : std::min(ceilDiv(bin_count_, 2 * kThreads), 148 * 2);
+    partials_sc_ = arena_.array<double>(2 * static_cast<std::size_t>(scatter_blocks_), "scatter partials");
+    partials_m_ = arena_.array<double>(9 * static_cast<std::size_t>(metrics_blocks_), "metric partials");
+    partials_g_ = arena_.array<double>(8 * static_cast<std::size_t>(gather_blocks_), "gather partials");
+    scalars_ = arena_.array<double>(kScalarCount, "evaluation scalars");
+    checkCuda(cudaMemsetAsync(scalars_, 0, kScalarCount * sizeof(double), stream_), "clear scalars");
+    allocateGroups();
+}
+
+void Engine::uploadStatic(const Problem& p) {
+    std::vector<double2> size(static_cast<std::size_t>(particle_count_));
+    std::vector<unsigned char> layer(static_cast<std::size_t>(particle_count_));
+    for (int64_t i = 0; i < particle_count_; ++i) {
+        size[i] = make_double2(p.width[i], p.height[i]);
+        layer[i] = static_cast<unsigned char>(p.layer[i]);
+    }
+    allocateParticles();
+    upload(size_, size, stream_);
+    upload(layer_, layer, stream_);
+    upload(charge_, p.charge, stream_);
+    if (!p.precond_base.empty()) upload(precond_, p.precond_base, stream_);
+
+    const std::size_t bins = static_cast<std::size_t>(bin_count_);
+    allocateDensity();
     {
         // t * (fixed + dark): the part of every bin's charge area that never moves.
         std::vector<double> static_charge(bins);
@@ -259,24 +283,167 @@ void Engine::uploadStatic(const Problem& p) {
             static_placeable_sum_ += area - p.static_dark[b];
         }
     }
-    scatter_blocks_ = ceilDiv(std::max<int64_t>(1, particle_count_), kThreads);
-    gather_blocks_ = gatherBlocks(static_cast<int>(std::min<int64_t>(particle_count_, 1 << 30)));
-    metrics_fused_ = metricsSplitFits(bins_x_);
-    metrics_blocks_ = metrics_fused_ ? bins_y_ : std::min(ceilDiv(bin_count_, 2 * kThreads), 148 * 2);
-    partials_sc_ = arena_.array<double>(2 * static_cast<std::size_t>(scatter_blocks_), "scatter partials");
-    partials_m_ = arena_.array<double>(9 * static_cast<std::size_t>(metrics_blocks_), "metric partials");
-    partials_g_ = arena_.array<double>(8 * static_cast<std::size_t>(gather_blocks_), "gather partials");
-    scalars_ = arena_.array<double>(kScalarCount, "evaluation scalars");
-    checkCuda(cudaMemsetAsync(scalars_, 0, kScalarCount * sizeof(double), stream_), "clear scalars");
+    allocatePartials();
+}
+
+bool Engine::setsUpOnDevice(const mpgp_design& d) const {
+    return static_cast<int64_t>(d.module_count) + d.pin_count >= kDeviceSetupItems &&
+           deviceSetupBytes(d, bin_count_) <= arena_.headroom();
+}
+
+// The session's set-up on the device (design_setup.cuh).  The caller's arrays are uploaded as
+// they are; this thread lays the nets out while a second one forms the static layers and the
+// movable areas on the device and, from their sums, the fillers, and a third sums the movable
+// areas on the host (in module order, as the reference does).
+void Engine::loadDesign(const mpgp_design& d, const DerivedDesign& derived, const mpgp_options& o) {
+    require(!nets_loaded_, "The engine's nets are loaded once.");
+    const std::size_t modules = static_cast<std::size_t>(d.module_count);
+    const std::size_t pins = static_cast<std::size_t>(d.pin_count);
+    const std::size_t nets = static_cast<std::size_t>(d.net_count);
+    const int movable = static_cast<int>(derived.movable.size());
+    movable_count_ = movable;
+    const uint64_t headroom = arena_.headroom();
+    const BudgetHeadroom fixed_headroom = [headroom] { return headroom; };
+
+    MovableAreas areas;
+    FillerNumbers numbers(o.seed);
+    std::vector<double> centres;
+    FillerPlan plan;
+    StaticSums sums;
+    std::exception_ptr areas_error, side_error;
+    struct Join {
+        std::thread t;
+        ~Join() { join(); }
+        void join() {
+            if (t.joinable()) t.join();
+        }
+    };
+    // Declared before the threads that use it.
+    Scratch scratch(stream_, [this] { return arena_.headroom(); });
+    DeviceModules m;
+    m.count = d.module_count;
+    Join areas_thread{std::thread([&] {
+        try {
+            areas = movableAreas(d, derived);
+            // The fillers' random numbers, ahead of their count (more are drawn if it is larger).
+            numbers.extend(static_cast<std::size_t>(std::min<uint64_t>(o.maximum_fillers, derived.movable.size())));
+        } catch (...) {
+            areas_error = std::current_exception();
+        }
+    })};
+
+    HostTransfer transfer(stream_, std::max(modules, pins) * sizeof(double));
+    const HostTransfer::Call call(&transfer);
+    const auto put = [&](const auto* host, std::size_t count) {
+        using T = std::remove_const_t<std::remove_pointer_t<decltype(host)>>;
+        T* device = scratch.array<T>(count);
+        transfer.send(host, device, count * sizeof(T));
+        h2d_bytes_ += count * sizeof(T);
+        return device;
+    };
+    m.width = put(d.module_width, modules);
+    m.height = put(d.module_height, modules);
+    m.x = put(d.module_x, modules);
+    m.y = put(d.module_y, modules);
+    if (d.module_orientation != nullptr) m.orientation = put(d.module_orientation, modules);
+    m.movable = put(derived.movable.data(), static_cast<std::size_t>(movable));
+    m.particle = scratch.array<int>(modules);
+    m.pins = scratch.array<int>(modules);
+    double* ascending = scratch.array<double>(static_cast<std::size_t>(movable));
+    checkCuda(cudaMemsetAsync(m.pins, 0, modules * sizeof(int), stream_), "Clear the pin counts");
+    launchMapModules(m, movable, stream_);
+    allocateDensity();
+    const cudaStream_t side = stream_wl_ != nullptr ? stream_wl_ : stream_;
+    checkCuda(cudaEventRecord(fork_, stream_), "Modules on the device");
+    checkCuda(cudaStreamWaitEvent(side, fork_, 0), "Modules on the device");
+    Join side_thread{std::thread([&] {
+        try {
+            checkCuda(cudaSetDevice(device_), "Select CUDA device");
+            sortAreasOnDevice(m, movable, derived.core, ascending, fixed_headroom, side);
+            sums = staticLayersOnDevice(d, derived, bins_x_, bins_y_, target_density_, static_charge_, fixed_headroom, side);
+            areas_thread.join();
+            if (areas_error) std::rethrow_exception(areas_error);
+            const auto trimmed_sum = [&](std::size_t lower, std::size_t upper) {
+                double sum = 0.0;
+                readDown(ascending + lower, upper - lower,
+                         [&](const double* v, std::size_t count) {
+                             for (std::size_t k = 0; k < count; ++k) sum += v[k];
+                         },
+                         side);
+                return sum;
+            };
+            plan = planFillers(derived.core, areas, sums.charge, trimmed_sum, o);
+            centres = fillerCentres(derived.core, plan, numbers);
+        } catch (...) {
+            side_error = std::current_exception();
+        }
+    })};
+
+    // The nets, as buildNetLayout lays them out from a Problem.
+    const int* pin_module = put(d.pin_module, pins);
+    launchCountPins(pin_module, static_cast<int>(pins), m.pins, stream_);
+    static_assert(sizeof(long long) == sizeof(int64_t), "64-bit offsets");
+    const long long* net_pin_start =
+        reinterpret_cast<const long long*>(put(d.net_pin_start, nets + 1));
+    const double* net_weight = put(d.net_weight, nets);
+    const double* offset_x = put(d.pin_offset_x, pins);
+    const double* offset_y = put(d.pin_offset_y, pins);
+    adoptNetLayout(buildNetLayoutOnDevice(
+        DesignPins{pin_module, offset_x, offset_y, m.particle, m.orientation, m.x, m.y}, net_pin_start, net_weight,
+        static_cast<int>(nets), movable,
+        [this](std::size_t bytes, const char* what) { return arena_.allocate(bytes, what); },
+        [&] { return arena_.headroom() - std::min(arena_.headroom(), scratch.held()); }, stream_));
+    nets_loaded_ = true;
+
+    side_thread.join();
+    if (side_error) std::rethrow_exception(side_error);
+    require(static_cast<std::size_t>(movable) + plan.count < static_cast<std::size_t>(std::numeric_limits<int32_t>::max()),
+            "The engine indexes particles with 32-bit integers.");
+    particle_count_ = static_cast<int64_t>(movable) + static_cast<int64_t>(plan.count);
+    static_fixed_sum_ = sums.fixed;
+    static_dark_sum_ = sums.dark;
+    static_placeable_sum_ = sums.placeable;
+    allocateParticles();
+    ParticleArrays p;
+    p.size = size_;
+    p.layer = layer_;
+    p.charge = charge_;
+    p.precond = precond_;
+    p.position = scratch_positions_;
+    p.filler_position = reinterpret_cast<const double2*>(put(centres.data(), centres.size()));
+    p.filler_width = plan.width;
+    p.filler_height = plan.height;
+    p.movable = movable;
+    p.count = static_cast<int>(particle_count_);
+    p.target_density = target_density_;
+    p.nominal_row_height = derived.nominal_row_height;
+    p.average_area = areas.total / static_cast<double>(std::max<std::size_t>(1U, derived.movable.size()));
+    launchParticles(m, p, stream_);
+    allocatePartials();
+    checkCuda(cudaStreamSynchronize(stream_), "Engine setup");  // the scratch is released on this stream
+    transfer.settled();
+    if (batch_ != nullptr) {
+        batch_->attach(this);
+        attached_ = true;
+    }
+}
+
+void Engine::clampPositions(const double2* positions, double2* out) {
+    launchClampPositions(positions, size_, out, static_cast<int>(particle_count_), region_.llx, region_.lly, region_.urx,
+                         region_.ury, stream_);
+    launches_ += 1;
 }
 
 void Engine::buildNetLayout(const Problem& p) {
     // The bucketed layout and the particle pin lists are built on the device
     // (ingest.cu); the host only turns the bucket sizes into the work list.
-    const NetLayout layout = buildNetLayoutOnDevice(
+    adoptNetLayout(buildNetLayoutOnDevice(
         p, static_cast<int>(movable_count_),
         [this](std::size_t bytes, const char* what) { return arena_.allocate(bytes, what); },
-        [this]() { return arena_.headroom(); }, stream_);
+        [this]() { return arena_.headroom(); }, stream_));
+}
+
+void Engine::adoptNetLayout(const NetLayout& layout) {
     pin_particle_ = layout.pin_particle;
     pin_offset_ = layout.pin_offset;
     static_pins_ = layout.static_pins;
@@ -318,19 +485,6 @@ void Engine::buildNetLayout(const Problem& p) {
 
 void Engine::buildBasis() {
     const int nx = bins_x_, ny = bins_y_;
-    const double width = region_.width(), height = region_.height();
-    // Spectral divide (ElectrostaticField.cpp:212-221): 1/(4 Nx Ny) / (kx^2 + ky^2), DC removed.
-    std::vector<float> scale(static_cast<std::size_t>(ny) * nx);
-    const double normalization = 1.0 / (4.0 * static_cast<double>(nx) * static_cast<double>(ny));
-    for (int l = 0; l < ny; ++l) {
-        const double wave_y = kPi * static_cast<double>(l) / height;
-        for (int k = 0; k < nx; ++k) {
-            const double wave_x = kPi * static_cast<double>(k) / width;
-            const double denominator = wave_x * wave_x + wave_y * wave_y;
-            scale[static_cast<std::size_t>(l) * nx + k] =
-                denominator <= kEpsilon ? 0.0f : static_cast<float>(normalization / denominator);
-        }
-    }
     std::vector<float> wy(static_cast<std::size_t>(ny), 1.0f), wx(static_cast<std::size_t>(nx), 1.0f);
     wy[0] = 0.5f;
     wx[0] = 0.5f;
@@ -340,12 +494,9 @@ void Engine::buildBasis() {
     weight_x_ = arena_.array<float>(wx.size(), "Parseval weights");
     field_ = arena_.array<float2>(bins, "electric field");
     potential_ = arena_.array<float>(bins, "potential");
-    upload(spectral_scale_, scale, stream_);
     upload(weight_y_, wy, stream_);
     upload(weight_x_, wx, stream_);
-    double max_scale = 0.0;
-    for (float v : scale) max_scale = std::max(max_scale, static_cast<double>(v));
-    buildTensorCoreBasis(max_scale);
+    buildTensorCoreBasis();
     checkCuda(cudaStreamSynchronize(stream_), "basis upload");
 }
 
@@ -360,7 +511,7 @@ SplitMatrix Engine::newSplit(int rows, int cols, const char* what) {
 }
 
 
-void Engine::buildTensorCoreBasis(double max_scale) {
+void Engine::buildTensorCoreBasis() {
     const int nx = bins_x_, ny = bins_y_;
     TcScales host_scales{};
     enum { kCx = 0, kCy, kDy, kDxc, kSxwt, kSyw };
@@ -371,10 +522,12 @@ void Engine::buildTensorCoreBasis(double max_scale) {
     tc_sxwt_ = newSplit(nx, nx, "DST basis planes");
     tc_syw_ = newSplit(ny, ny, "DST basis planes");
     const SplitMatrix basis_planes[kBasisCount] = {tc_cx_, tc_cy_, tc_dy_, tc_dxc_, tc_sxwt_, tc_syw_};
-    unsigned long long* ranges = arena_.array<unsigned long long>(2 * kBasisCount, "basis ranges");
+    unsigned long long* ranges = arena_.array<unsigned long long>(kBasisRanges, "basis ranges");
     int exponents[kBasisCount] = {};
     double row_l1[kBasisCount] = {};
-    buildBasisPlanes(nx, ny, region_.width(), region_.height(), basis_planes, ranges, exponents, row_l1, stream_);
+    double max_scale = 0.0;
+    buildBasisPlanes(nx, ny, region_.width(), region_.height(), basis_planes, spectral_scale_, ranges, exponents, row_l1,
+                     max_scale, stream_);
     for (int t = 0; t < kBasisCount; ++t) host_scales.exp_basis[t] = exponents[t];
     tc_source_ = newSplit(ny, nx, "source planes");
     tc_x1t_ = newSplit(nx, ny, "DCT stage planes");

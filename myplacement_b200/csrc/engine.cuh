@@ -10,6 +10,7 @@
 
 #include "dct_tc.cuh"
 #include "field_tc.cuh"
+#include "ingest.cuh"
 #include "kernels.cuh"
 #include "pinned.hpp"
 #include "setup.hpp"
@@ -170,6 +171,13 @@ public:
     void load(const Problem& problem);
     void loadNets(const Problem& problem, int64_t movable_count);
     void loadParticles(const Problem& problem);
+    // Or from a session's design, set up on the device where setsUpOnDevice says so; the
+    // initial positions are then in scratchPositions().
+    [[nodiscard]] bool setsUpOnDevice(const mpgp_design& design) const;
+    void loadDesign(const mpgp_design& design, const DerivedDesign& derived, const mpgp_options& options);
+    // out = positions moved into the region as far as the particles' sizes allow (applyPositions,
+    // AdaptiveGlobalPlacer.cpp:185-198).
+    void clampPositions(const double2* positions, double2* out);
     ~Engine();
     Engine(const Engine&) = delete;
     Engine& operator=(const Engine&) = delete;
@@ -295,6 +303,10 @@ private:
     void runStagedField(bool gradient, bool potential, bool forward, bool split_source);
     void runWirelengthPass(const EvalPlan& p);
     void uploadStatic(const Problem& problem);
+    void allocateParticles();
+    void allocateDensity();
+    void allocatePartials();
+    void adoptNetLayout(const NetLayout& layout);
     void buildNetLayout(const Problem& problem);
     void buildBasis();
 
@@ -385,7 +397,7 @@ private:
     bool nets_loaded_ = false;
     uint64_t synced_ticket_ = 0;
     unsigned long long sequence_ = 0;
-    void buildTensorCoreBasis(double max_scale);
+    void buildTensorCoreBasis();
     SplitMatrix newSplit(int rows, int cols, const char* what);
 
     // partials and scalars

@@ -40,6 +40,18 @@ __global__ void netKeysKernel(const long long* net_pin_start, int nets, int* key
     values[n] = n;
 }
 
+// Pins of a flat CSR (Problem): the particle (negative: static) and its offset or position.
+struct FlatPins {
+    const int* pin_particle;
+    const double* pin_x;
+    const double* pin_y;
+    __device__ __forceinline__ int pin(long long k, double& x, double& y) const {
+        x = pin_x[k];
+        y = pin_y[k];
+        return pin_particle[k];
+    }
+};
+
 // Kept degree per sorted net and the first sorted position of every bucket.
 __global__ void sortedNetsKernel(const long long* net_pin_start, const int* keys, const int* order, int nets,
                                  int* degree, int* bucket_first) {
@@ -51,9 +63,9 @@ __global__ void sortedNetsKernel(const long long* net_pin_start, const int* keys
     if (k == 0 || keys[k - 1] != key) bucket_first[key] = k;
 }
 
-__global__ void copyPinsKernel(const long long* net_pin_start, const int* order, const int* net_start, int kept,
-                               const int* pin_particle, const double* pin_x, const double* pin_y,
-                               const double* net_weight, int movable, int* out_particle, float2* out_offset,
+template <class Source>
+__global__ void copyPinsKernel(Source source, const long long* net_pin_start, const int* order, const int* net_start,
+                               int kept, const double* net_weight, int movable, int* out_particle, float2* out_offset,
                                double2* out_static, int* is_static, float* out_weight, double* out_weight64,
                                int* error) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -63,10 +75,9 @@ __global__ void copyPinsKernel(const long long* net_pin_start, const int* order,
     const int dst = net_start[k];
     const int degree = net_start[k + 1] - dst;
     for (int j = 0; j < degree; ++j) {
-        const int particle = pin_particle[src + j];
+        double x, y;
+        const int particle = source.pin(src + j, x, y);
         if (particle >= movable) atomicExch(error, 1);
-        const double x = pin_x[src + j];
-        const double y = pin_y[src + j];
         out_particle[dst + j] = particle;
         out_offset[dst + j] = particle >= 0 ? make_float2(static_cast<float>(x), static_cast<float>(y))
                                             : make_float2(0.0f, 0.0f);
@@ -112,40 +123,6 @@ int bitsFor(int value) {
     return bits;
 }
 
-// Stream-ordered scratch, released when the ingest returns.  While it lives it
-// counts against the engine's device-memory budget like the lasting arrays.
-class Scratch {
-public:
-    Scratch(cudaStream_t stream, const BudgetHeadroom& headroom) : stream_(stream), headroom_(headroom) {}
-    ~Scratch() {
-        for (void* p : blocks_) cudaFreeAsync(p, stream_);
-    }
-    // Fails unless `bytes` more fit in the budget beside the scratch held now.
-    void check(std::size_t bytes) const {
-        if (held_ + bytes > headroom_()) {
-            fail(MPGP_ERR_BUDGET, "CUDA allocation budget exceeded while ingesting the design.");
-        }
-    }
-    template <typename T>
-    T* array(std::size_t count) {
-        const std::size_t bytes = std::max<std::size_t>(1, count) * sizeof(T);
-        check(bytes);
-        void* p = nullptr;
-        int device = 0;
-        checkCuda(cudaGetDevice(&device), "Query the current device");
-        checkCuda(cudaMallocFromPoolAsync(&p, bytes, devicePool(device), stream_), "ingest scratch");
-        blocks_.push_back(p);
-        held_ += bytes;
-        return static_cast<T*>(p);
-    }
-
-private:
-    cudaStream_t stream_;
-    const BudgetHeadroom& headroom_;
-    std::vector<void*> blocks_;
-    uint64_t held_ = 0;
-};
-
 template <typename T>
 void uploadVector(T* device, const std::vector<T>& host, cudaStream_t stream) {
     if (!host.empty()) {
@@ -156,32 +133,17 @@ void uploadVector(T* device, const std::vector<T>& host, cudaStream_t stream) {
 
 }  // namespace
 
-NetLayout buildNetLayoutOnDevice(const Problem& p, int movable, const DeviceAllocator& lasting,
-                                 const BudgetHeadroom& headroom, cudaStream_t stream) {
-    const int nets = static_cast<int>(p.net_weight.size());
-    const int pins_in = static_cast<int>(p.pin_particle.size());
+namespace {
+
+template <class Source>
+NetLayout layOutNets(const Source& source, const long long* net_pin_start, const double* weight, int nets, int movable,
+                     const DeviceAllocator& lasting, Scratch& scratch, cudaStream_t stream) {
     NetLayout out;
-    Scratch scratch(stream, headroom);
     // The layout's lasting arrays, checked against the budget beside the scratch.
     const auto allocate = [&](std::size_t bytes, const char* what) {
         scratch.check(bytes);
         return lasting(bytes, what);
     };
-
-    // The flat CSR on the device.
-    long long* net_pin_start = scratch.array<long long>(static_cast<std::size_t>(nets) + 1);
-    int* pin_particle = scratch.array<int>(static_cast<std::size_t>(pins_in));
-    double* pin_x = scratch.array<double>(static_cast<std::size_t>(pins_in));
-    double* pin_y = scratch.array<double>(static_cast<std::size_t>(pins_in));
-    double* weight = scratch.array<double>(static_cast<std::size_t>(nets));
-    static_assert(sizeof(long long) == sizeof(int64_t), "64-bit offsets");
-    checkCuda(cudaMemcpyAsync(net_pin_start, p.net_pin_start.data(), (static_cast<std::size_t>(nets) + 1) * 8,
-                              cudaMemcpyHostToDevice, stream),
-              "ingest upload");
-    uploadVector(pin_particle, p.pin_particle, stream);
-    uploadVector(pin_x, p.pin_x, stream);
-    uploadVector(pin_y, p.pin_y, stream);
-    uploadVector(weight, p.net_weight, stream);
 
     // 1-2: buckets, stable sort of the nets.
     int* keys = scratch.array<int>(static_cast<std::size_t>(nets));
@@ -243,8 +205,8 @@ NetLayout buildNetLayoutOnDevice(const Problem& p, int movable, const DeviceAllo
     checkCuda(cudaMemsetAsync(is_static + out.kept_pins, 0, sizeof(int), stream), "ingest");
     if (out.kept_nets > 0) {
         copyPinsKernel<<<blocksFor(out.kept_nets), kThreads, 0, stream>>>(
-            net_pin_start, order, out.net_start, out.kept_nets, pin_particle, pin_x, pin_y, weight, movable,
-            out.pin_particle, out.pin_offset, staged_static, is_static, out.net_weight, out.net_weight64, error);
+            source, net_pin_start, order, out.net_start, out.kept_nets, weight, movable, out.pin_particle, out.pin_offset,
+            staged_static, is_static, out.net_weight, out.net_weight64, error);
         checkCuda(cudaGetLastError(), "Launch the pin copy");
     }
 
@@ -305,6 +267,38 @@ NetLayout buildNetLayoutOnDevice(const Problem& p, int movable, const DeviceAllo
     }
     checkCuda(cudaStreamSynchronize(stream), "net layout");
     return out;
+}
+
+}  // namespace
+
+NetLayout buildNetLayoutOnDevice(const Problem& p, int movable, const DeviceAllocator& lasting,
+                                 const BudgetHeadroom& headroom, cudaStream_t stream) {
+    const int nets = static_cast<int>(p.net_weight.size());
+    const int pins_in = static_cast<int>(p.pin_particle.size());
+    Scratch scratch(stream, headroom);
+    // The flat CSR on the device.
+    long long* net_pin_start = scratch.array<long long>(static_cast<std::size_t>(nets) + 1);
+    int* pin_particle = scratch.array<int>(static_cast<std::size_t>(pins_in));
+    double* pin_x = scratch.array<double>(static_cast<std::size_t>(pins_in));
+    double* pin_y = scratch.array<double>(static_cast<std::size_t>(pins_in));
+    double* weight = scratch.array<double>(static_cast<std::size_t>(nets));
+    static_assert(sizeof(long long) == sizeof(int64_t), "64-bit offsets");
+    checkCuda(cudaMemcpyAsync(net_pin_start, p.net_pin_start.data(), (static_cast<std::size_t>(nets) + 1) * 8,
+                              cudaMemcpyHostToDevice, stream),
+              "ingest upload");
+    uploadVector(pin_particle, p.pin_particle, stream);
+    uploadVector(pin_x, p.pin_x, stream);
+    uploadVector(pin_y, p.pin_y, stream);
+    uploadVector(weight, p.net_weight, stream);
+    return layOutNets(FlatPins{pin_particle, pin_x, pin_y}, net_pin_start, weight, nets, movable, lasting, scratch,
+                      stream);
+}
+
+NetLayout buildNetLayoutOnDevice(const DesignPins& pins, const long long* net_pin_start, const double* weight, int nets,
+                                 int movable, const DeviceAllocator& lasting, const BudgetHeadroom& headroom,
+                                 cudaStream_t stream) {
+    Scratch scratch(stream, headroom);
+    return layOutNets(pins, net_pin_start, weight, nets, movable, lasting, scratch, stream);
 }
 
 }  // namespace mpgp

@@ -268,6 +268,8 @@ int gatherBlocks(int particle_count);
 // ---- small vector kernels ---------------------------------------------------------
 // A device-to-device copy of positions as a chained kernel (programmatic launch, no copy engine).
 void launchCopyPositions(const double2* source, double2* destination, int count, cudaStream_t stream);
+void launchClampPositions(const double2* source, const double2* size, double2* destination, int count, double llx,
+                          double lly, double urx, double ury, cudaStream_t stream);
 void launchVelocity(const double2* next, const double2* previous, double2* velocity, int count,
                     cudaStream_t stream);
 

@@ -20,6 +20,7 @@
 #include <thread>
 
 #include "common.cuh"
+#include "design_setup.cuh"
 
 namespace mpgp {
 namespace {
@@ -103,59 +104,74 @@ Session::Session(const mpgp_design& design, const mpgp_options& options, Batch* 
         validateOptions(options_);
     }
     rudy_requested_ = options_.rudy_penalty_model != MPGP_RUDY_DISABLED;
-    derived_ = deriveDesign(design);
     module_x_.assign(design.module_x, design.module_x + design.module_count);
     module_y_.assign(design.module_y, design.module_y + design.module_count);
-    module_w_.assign(design.module_width, design.module_width + design.module_count);
-    module_h_.assign(design.module_height, design.module_height + design.module_count);
     result_.compute_backend_used = MPGP_BACKEND_CUDA;
+    // A large design is set up on the device, which counts its modules' pins itself.
+    const bool large = static_cast<int64_t>(design.module_count) + design.pin_count >= kDeviceSetupItems;
+    derived_ = deriveDesign(design, !large);
     if (derived_.movable.empty()) {  // AdaptiveGlobalPlacer.cpp:653
         empty_ = true;
         done_ = true;
         result_ = mpgp_result{};
         return;
     }
-    // The host problem is built on two threads while this one sets up the engine's grid
-    // part on the device (the field solve's bases and buffers need only the grid): the
-    // pin and net arrays, whose device layout then starts at once, and the static
-    // layers, fillers and particle arrays, which are uploaded last.
-    std::exception_ptr pins_error, particles_error;
-    std::thread pins_thread([&] {
-        try {
-            buildProblemPins(design, derived_, problem_);
-        } catch (...) {
-            pins_error = std::current_exception();
-        }
-    });
-    std::thread particles_thread([&] {
-        try {
-            buildProblemParticles(design, derived_, options_, problem_, fillers_);
-        } catch (...) {
-            particles_error = std::current_exception();
-        }
-    });
-    struct Join {
-        std::thread& t;
-        ~Join() {
-            if (t.joinable()) t.join();
-        }
-    } join_pins{pins_thread}, join_particles{particles_thread};
-    int device_count = 0;
-    const cudaError_t count_status = cudaGetDeviceCount(&device_count);
-    if (count_status != cudaSuccess || device_count <= 0) {
-        fail(MPGP_ERR_UNAVAILABLE, std::string("CUDA device discovery failed: ") + cudaGetErrorString(count_status));
-    }
-    require(options_.cuda_device >= 0 && options_.cuda_device < device_count,
-            "Requested CUDA device does not exist on this host.");
     const Engine::Grid grid{options_.bins_x, options_.bins_y, derived_.core, options_.target_density};
-    engine_ = std::make_unique<Engine>(grid, options_.cuda_device, options_.maximum_cuda_memory_bytes,
-                                       rudy_requested_ ? nullptr : batch);
-    pins_thread.join();
-    if (pins_error) std::rethrow_exception(pins_error);
-    engine_->loadNets(problem_, static_cast<int64_t>(derived_.movable.size()));
-    particles_thread.join();
-    if (particles_error) std::rethrow_exception(particles_error);
-    engine_->loadParticles(problem_);
+    const auto makeEngine = [&] {
+        int device_count = 0;
+        const cudaError_t count_status = cudaGetDeviceCount(&device_count);
+        if (count_status != cudaSuccess || device_count <= 0) {
+            fail(MPGP_ERR_UNAVAILABLE, std::string("CUDA device discovery failed: ") + cudaGetErrorString(count_status));
+        }
+        require(options_.cuda_device >= 0 && options_.cuda_device < device_count,
+                "Requested CUDA device does not exist on this host.");
+        engine_ = std::make_unique<Engine>(grid, options_.cuda_device, options_.maximum_cuda_memory_bytes,
+                                           rudy_requested_ ? nullptr : batch);
+    };
+    bool on_device = false;
+    if (large) {
+        makeEngine();
+        on_device = engine_->setsUpOnDevice(design);
+        if (on_device) {
+            engine_->loadDesign(design, derived_, options_);
+        } else {
+            derived_ = deriveDesign(design);  // with the pin counts
+        }
+    }
+    if (!on_device) {
+        // The host problem is built on two threads while this one sets up the engine's grid
+        // part on the device (the field solve's bases and buffers need only the grid): the
+        // pin and net arrays, whose device layout then starts at once, and the static
+        // layers, fillers and particle arrays, which are uploaded last.
+        std::exception_ptr pins_error, particles_error;
+        std::thread pins_thread([&] {
+            try {
+                buildProblemPins(design, derived_, problem_);
+            } catch (...) {
+                pins_error = std::current_exception();
+            }
+        });
+        std::thread particles_thread([&] {
+            try {
+                buildProblemParticles(design, derived_, options_, problem_, fillers_);
+            } catch (...) {
+                particles_error = std::current_exception();
+            }
+        });
+        struct Join {
+            std::thread& t;
+            ~Join() {
+                if (t.joinable()) t.join();
+            }
+        } join_pins{pins_thread}, join_particles{particles_thread};
+        if (engine_ == nullptr) makeEngine();
+        pins_thread.join();
+        if (pins_error) std::rethrow_exception(pins_error);
+        engine_->loadNets(problem_, static_cast<int64_t>(derived_.movable.size()));
+        particles_thread.join();
+        if (particles_error) std::rethrow_exception(particles_error);
+        engine_->loadParticles(problem_);
+    }
     if (rudy_requested_) engine_->enableRudy(options_);
     result_.cuda_device_used = options_.cuda_device;
 
@@ -184,17 +200,22 @@ Session::Session(const mpgp_design& design, const mpgp_options& options, Batch* 
 
     // capturePositions (AdaptiveGlobalPlacer.cpp:174-183): movable centres, then fillers.
     const std::size_t particles = static_cast<std::size_t>(engine_->particleCount());
-    std::vector<double2> initial(particles);
-    for (std::size_t i = 0; i < derived_.movable.size(); ++i) {
-        initial[i] = make_double2(module_x_[derived_.movable[i]], module_y_[derived_.movable[i]]);
+    if (on_device) {
+        launchCopyPositions(engine_->scratchPositions(), cur_, static_cast<int>(particles), engine_->stream());
+        engine_->countLaunches(1);
+    } else {
+        std::vector<double2> initial(particles);
+        for (std::size_t i = 0; i < derived_.movable.size(); ++i) {
+            initial[i] = make_double2(module_x_[derived_.movable[i]], module_y_[derived_.movable[i]]);
+        }
+        for (std::size_t i = 0; i < fillers_.size(); ++i) {
+            initial[derived_.movable.size() + i] = make_double2(fillers_[i].x, fillers_[i].y);
+        }
+        checkCuda(cudaMemcpyAsync(cur_, initial.data(), particles * sizeof(double2), cudaMemcpyHostToDevice,
+                                  engine_->stream()),
+                  "Upload initial positions");
+        engine_->addTransfer(particles * sizeof(double2), 0);
     }
-    for (std::size_t i = 0; i < fillers_.size(); ++i) {
-        initial[derived_.movable.size() + i] = make_double2(fillers_[i].x, fillers_[i].y);
-    }
-    checkCuda(cudaMemcpyAsync(cur_, initial.data(), particles * sizeof(double2), cudaMemcpyHostToDevice,
-                              engine_->stream()),
-              "Upload initial positions");
-    engine_->addTransfer(particles * sizeof(double2), 0);
 
     // Initial evaluations and the penalty normalisation (AdaptiveGlobalPlacer.cpp:672-733).
     smoothing_ = options_.initial_smoothing * max_bin_;
@@ -694,6 +715,14 @@ void Session::currentPositions(double* xy) const {
     checkCuda(cudaStreamSynchronize(engine_->stream()), "Download positions");
 }
 
+void Session::downloadPlaced(double2* placed, std::size_t count) {
+    const std::size_t bytes = count * sizeof(double2);
+    checkCuda(cudaMemcpyAsync(placed, cand_, bytes, cudaMemcpyDeviceToHost, engine_->stream()),
+              "Download final positions");
+    checkCuda(cudaStreamSynchronize(engine_->stream()), "Download final positions");
+    engine_->addTransfer(0, bytes);
+}
+
 void Session::finish(double* module_x, double* module_y, mpgp_result* result, mpgp_history_row* history,
                      int capacity) {
     if (!empty_) {
@@ -706,34 +735,21 @@ void Session::finish(double* module_x, double* module_y, mpgp_result* result, mp
             result_.best_checkpoint_hpwl = chosen.hpwl;
             result_.best_checkpoint_overflow = chosen.overflow;
         }
-        const std::size_t particles = static_cast<std::size_t>(engine_->particleCount());
-        std::vector<double2> host(particles);
-        checkCuda(cudaMemcpyAsync(host.data(), final_positions, particles * sizeof(double2), cudaMemcpyDeviceToHost,
-                                  engine_->stream()),
-                  "Download final positions");
-        checkCuda(cudaStreamSynchronize(engine_->stream()), "Download final positions");
-        engine_->addTransfer(0, particles * sizeof(double2));
-        // applyPositions (AdaptiveGlobalPlacer.cpp:185-198) for the movable modules.
-        const Rect2& core = derived_.core;
-        std::vector<double2> clamped(particles);
-        for (std::size_t i = 0; i < particles; ++i) {
-            const double w = i < derived_.movable.size() ? module_w_[derived_.movable[i]] : fillers_[i - derived_.movable.size()].width;
-            const double h = i < derived_.movable.size() ? module_h_[derived_.movable[i]] : fillers_[i - derived_.movable.size()].height;
-            const double min_x = core.llx + w * 0.5, max_x = core.urx - w * 0.5;
-            const double min_y = core.lly + h * 0.5, max_y = core.ury - h * 0.5;
-            clamped[i].x = min_x <= max_x ? clampValue(host[i].x, min_x, max_x) : (core.llx + core.urx) * 0.5;
-            clamped[i].y = min_y <= max_y ? clampValue(host[i].y, min_y, max_y) : (core.lly + core.ury) * 0.5;
-            if (i < derived_.movable.size()) {
-                module_x_[derived_.movable[i]] = clamped[i].x;
-                module_y_[derived_.movable[i]] = clamped[i].y;
-            }
+        // applyPositions (AdaptiveGlobalPlacer.cpp:185-198); then calculateHpwl /
+        // calculateDensity at the restored placement (:938-940), which run while the movable
+        // modules' centres come back.
+        const std::size_t movable = derived_.movable.size();
+        engine_->clampPositions(final_positions, cand_);
+        EvalRequest q = givenRequest(cand_, false, penalty_, nullptr, nullptr, false, false, false, -1.0);
+        const uint64_t ticket = launchEvaluation(q);
+        const std::unique_ptr<double2[]> placed(new double2[movable]);  // not cleared: filled by the download
+        if (engine_->overlapsEvaluations()) downloadPlaced(placed.get(), movable);
+        const StateEval final_eval = collect(ticket, q, penalty_);
+        if (!engine_->overlapsEvaluations()) downloadPlaced(placed.get(), movable);  // a batched evaluation runs in collect
+        for (std::size_t i = 0; i < movable; ++i) {
+            module_x_[derived_.movable[i]] = placed[i].x;
+            module_y_[derived_.movable[i]] = placed[i].y;
         }
-        // calculateHpwl / calculateDensity at the restored placement (:938-940).
-        checkCuda(cudaMemcpyAsync(cand_, clamped.data(), particles * sizeof(double2), cudaMemcpyHostToDevice,
-                                  engine_->stream()),
-                  "Upload final positions");
-        engine_->addTransfer(particles * sizeof(double2), 0);
-        const StateEval final_eval = evaluateGiven(cand_, false, penalty_, nullptr, nullptr, false, false);
         result_.hpwl_after = final_eval.m.hpwl;
         result_.overflow_after = final_eval.m.design.normalized_overflow;
         if (rudy_active_) {

@@ -98,8 +98,8 @@ private:
     void iterate();
 
     mpgp_options options_{};
+    void downloadPlaced(double2* placed, std::size_t count);
     std::vector<double> module_x_, module_y_;
-    std::vector<double> module_w_, module_h_;
     DerivedDesign derived_;
     std::vector<Filler> fillers_;
     Problem problem_;

@@ -259,7 +259,7 @@ void validateOptions(const mpgp_options& o) {
     require(o.maximum_cuda_memory_bytes > 0, "The device memory budget must be non-zero.");
 }
 
-DerivedDesign deriveDesign(const mpgp_design& d) {
+DerivedDesign deriveDesign(const mpgp_design& d, bool with_pins) {
     DerivedDesign out;
     if (d.row_count > 0) {
         std::vector<double> heights(d.row_height, d.row_height + d.row_count);
@@ -280,10 +280,10 @@ DerivedDesign deriveDesign(const mpgp_design& d) {
         out.core = {core.llx, core.lly, core.urx, core.ury};
     }
     const std::size_t modules = static_cast<std::size_t>(d.module_count);
-    const std::size_t pins = static_cast<std::size_t>(d.pin_count);
+    const std::size_t pins = with_pins ? static_cast<std::size_t>(d.pin_count) : 0;
     out.is_fixed.resize(modules);
     out.is_macro.resize(modules);
-    out.pin_count.assign(modules, 0);
+    if (with_pins) out.pin_count.assign(modules, 0);
     // Module flags and the movable list (in module order: each piece's movable
     // modules go after those of the pieces before it), then the pin counts (integer
     // sums, so the pieces' order does not matter), on up to eight host threads.
@@ -313,12 +313,13 @@ DerivedDesign deriveDesign(const mpgp_design& d) {
         for (std::size_t m = bound(k, modules); m < bound(k + 1, modules); ++m) {
             if (!out.is_fixed[m]) out.movable[at++] = static_cast<int32_t>(m);
         }
-        if (pieces > 1) {
+        if (pieces > 1 && with_pins) {
             std::vector<int32_t>& mine = counts[k];
             mine.assign(modules, 0);
             for (std::size_t p = bound(k, pins); p < bound(k + 1, pins); ++p) ++mine[d.pin_module[p]];
         }
     });
+    if (!with_pins) return out;
     if (pieces <= 1) {
         for (std::size_t p = 0; p < pins; ++p) ++out.pin_count[d.pin_module[p]];
     } else {
@@ -389,60 +390,96 @@ void staticDensity(const mpgp_design& d, const DerivedDesign& derived, int bins_
     }
 }
 
+MovableAreas movableAreas(const mpgp_design& d, const DerivedDesign& derived) {
+    const R core{derived.core.llx, derived.core.lly, derived.core.urx, derived.core.ury};
+    MovableAreas out;
+    for (const int32_t m : derived.movable) {
+        const double area =
+            moduleRect(d.module_x[m], d.module_y[m], d.module_width[m], d.module_height[m]).intersection(core).area();
+        if (derived.is_macro[m]) {
+            out.macro += area;
+        } else {
+            out.standard += area;
+        }
+        if (area > kEpsilon) ++out.positive;
+        out.total += d.module_width[m] * d.module_height[m];
+    }
+    return out;
+}
+
+FillerPlan planFillers(const Rect2& core, const MovableAreas& movable, double static_charge_area,
+                       const std::function<double(std::size_t, std::size_t)>& trimmed_sum,
+                       const mpgp_options& options) {
+    const R region{core.llx, core.lly, core.urx, core.ury};
+    const double t = options.target_density;
+    const double movable_charge_area = movable.standard + t * movable.macro;
+    const double required_filler_charge_area =
+        std::max(0.0, t * region.area() - static_charge_area - movable_charge_area);
+    const double filler_area = required_filler_charge_area / std::max(t, kEpsilon);
+    const std::size_t n = movable.positive;
+    if (filler_area <= kEpsilon || n == 0 || options.maximum_fillers == 0U) return {};
+
+    const std::size_t lower = n / 10U;
+    const std::size_t upper = std::max(lower + 1U, n - n / 10U);
+    const double representative_area = trimmed_sum(lower, upper) / static_cast<double>(upper - lower);
+    FillerPlan plan;
+    plan.count = std::min<std::size_t>(
+        static_cast<std::size_t>(options.maximum_fillers),
+        std::max<std::size_t>(1U, static_cast<std::size_t>(std::ceil(filler_area / std::max(representative_area, kEpsilon)))));
+    const double area_per_filler = filler_area / static_cast<double>(plan.count);
+    const double aspect = std::max(core.width() / core.height(), 0.1);
+    plan.width = std::sqrt(area_per_filler * aspect);
+    plan.height = area_per_filler / std::max(plan.width, kEpsilon);
+    return plan;
+}
+
+void FillerNumbers::extend(std::size_t count) {
+    unit.reserve(2 * count);
+    while (unit.size() < 2 * count) unit.push_back(std::generate_canonical<double, 53>(generator));
+}
+
+std::vector<double> fillerCentres(const Rect2& core, const FillerPlan& plan, FillerNumbers& numbers) {
+    numbers.extend(plan.count);
+    const double least_x = core.llx + plan.width * 0.5, most_x = core.urx - plan.width * 0.5;
+    const double least_y = core.lly + plan.height * 0.5, most_y = core.ury - plan.height * 0.5;
+    std::vector<double> centres(2 * plan.count);
+    for (std::size_t index = 0; index < plan.count; ++index) {
+        centres[2 * index] = numbers.unit[2 * index] * (most_x - least_x) + least_x;
+        centres[2 * index + 1] = numbers.unit[2 * index + 1] * (most_y - least_y) + least_y;
+    }
+    return centres;
+}
+
 std::vector<Filler> createFillers(const mpgp_design& d, const DerivedDesign& derived, const std::vector<double>& fixed,
                                   const std::vector<double>& dark, int, int, const mpgp_options& options) {
     const R core{derived.core.llx, derived.core.lly, derived.core.urx, derived.core.ury};
-    double standard_cell_area = 0.0;
-    double macro_area = 0.0;
+    const MovableAreas movable = movableAreas(d, derived);
+    // static_density.metrics(false).total_charge_area (Metrics.cpp:101-119 with Metrics.hpp:25-29).
+    double static_charge_area = 0.0;
+    for (std::size_t index = 0; index < fixed.size(); ++index) {
+        const double scaled_area = fixed[index] + 0.0 + dark[index] + 0.0;
+        static_charge_area += 0.0 + options.target_density * scaled_area;
+    }
     std::vector<double> areas;
     areas.reserve(derived.movable.size());
     for (const int32_t m : derived.movable) {
         const double area =
             moduleRect(d.module_x[m], d.module_y[m], d.module_width[m], d.module_height[m]).intersection(core).area();
-        if (derived.is_macro[m]) {
-            macro_area += area;
-        } else {
-            standard_cell_area += area;
-        }
         if (area > kEpsilon) areas.push_back(area);
     }
-    // static_density.metrics(false).total_charge_area (Metrics.cpp:101-119 with Metrics.hpp:25-29).
-    double static_charge_area = 0.0;
-    const double t = options.target_density;
-    for (std::size_t index = 0; index < fixed.size(); ++index) {
-        const double scaled_area = fixed[index] + 0.0 + dark[index] + 0.0;
-        static_charge_area += 0.0 + t * scaled_area;
-    }
-    const double movable_charge_area = standard_cell_area + t * macro_area;
-    const double required_filler_charge_area =
-        std::max(0.0, t * core.area() - static_charge_area - movable_charge_area);
-    const double filler_area = required_filler_charge_area / std::max(t, kEpsilon);
-    if (filler_area <= kEpsilon || areas.empty() || options.maximum_fillers == 0U) return {};
-
     sortAscending(areas);
-    const std::size_t lower = areas.size() / 10U;
-    const std::size_t upper = std::max(lower + 1U, areas.size() - areas.size() / 10U);
-    const double representative_area =
-        std::accumulate(areas.begin() + static_cast<std::ptrdiff_t>(lower),
-                        areas.begin() + static_cast<std::ptrdiff_t>(upper), 0.0) /
-        static_cast<double>(upper - lower);
-    const std::size_t count = std::min<std::size_t>(
-        static_cast<std::size_t>(options.maximum_fillers),
-        std::max<std::size_t>(1U, static_cast<std::size_t>(std::ceil(filler_area / std::max(representative_area, kEpsilon)))));
-    const double area_per_filler = filler_area / static_cast<double>(count);
-    const double aspect = std::max(core.width() / core.height(), 0.1);
-    const double width = std::sqrt(area_per_filler * aspect);
-    const double height = area_per_filler / std::max(width, kEpsilon);
-
-    std::mt19937_64 generator(options.seed ^ 0x9e3779b97f4a7c15ULL);
-    std::uniform_real_distribution<double> x_distribution(core.llx + width * 0.5, core.urx - width * 0.5);
-    std::uniform_real_distribution<double> y_distribution(core.lly + height * 0.5, core.ury - height * 0.5);
+    const auto trimmed_sum = [&](std::size_t lower, std::size_t upper) {
+        return std::accumulate(areas.begin() + static_cast<std::ptrdiff_t>(lower),
+                               areas.begin() + static_cast<std::ptrdiff_t>(upper), 0.0);
+    };
+    const FillerPlan plan = planFillers(derived.core, movable, static_charge_area, trimmed_sum, options);
+    if (plan.count == 0) return {};
+    FillerNumbers numbers(options.seed);
+    const std::vector<double> centres = fillerCentres(derived.core, plan, numbers);
     std::vector<Filler> fillers;
-    fillers.reserve(count);
-    for (std::size_t index = 0; index < count; ++index) {
-        const double x = x_distribution(generator);
-        const double y = y_distribution(generator);
-        fillers.push_back({x, y, width, height});
+    fillers.reserve(plan.count);
+    for (std::size_t index = 0; index < plan.count; ++index) {
+        fillers.push_back({centres[2 * index], centres[2 * index + 1], plan.width, plan.height});
     }
     return fillers;
 }

@@ -9,7 +9,10 @@
 // layers and preconditioner are bit-identical to the reference's.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
+#include <functional>
+#include <random>
 #include <vector>
 
 #include "mpgp.h"
@@ -55,7 +58,8 @@ struct DerivedDesign {
     std::vector<int32_t> pin_count;  // per module
 };
 
-DerivedDesign deriveDesign(const mpgp_design& design);
+// Without `with_pins` the pin counts stay empty.
+DerivedDesign deriveDesign(const mpgp_design& design, bool with_pins = true);
 
 // Validates the design arrays (sizes, indices, finiteness).
 void validateDesign(const mpgp_design& design);
@@ -76,6 +80,34 @@ struct Filler {
 std::vector<Filler> createFillers(const mpgp_design& design, const DerivedDesign& derived,
                                   const std::vector<double>& fixed, const std::vector<double>& dark,
                                   int bins_x, int bins_y, const mpgp_options& options);
+
+// Its parts: the movable modules' areas summed in module order, the fillers' number and size
+// from the areas inside the core in ascending order (those above kEpsilon), and their seeded
+// centres in order.
+struct MovableAreas {
+    double standard = 0.0, macro = 0.0;  // inside the core
+    double total = 0.0;                  // of the whole modules (initializePreconditioner)
+    std::size_t positive = 0;            // modules with more than kEpsilon inside the core
+};
+MovableAreas movableAreas(const mpgp_design& design, const DerivedDesign& derived);
+struct FillerPlan {
+    std::size_t count = 0;
+    double width = 0.0, height = 0.0;
+};
+// trimmed_sum(lower, upper) sums the ascending areas [lower, upper) in order.
+FillerPlan planFillers(const Rect2& core, const MovableAreas& areas, double static_charge_area,
+                       const std::function<double(std::size_t, std::size_t)>& trimmed_sum,
+                       const mpgp_options& options);
+// The seeded uniform numbers in [0, 1) of the first `count` fillers (two each), and the centres
+// made of them: x0, y0, x1, y1, ...  (uniform_real_distribution's formula; `unit` holds as many
+// as are at hand and is extended as needed).
+struct FillerNumbers {
+    explicit FillerNumbers(uint64_t seed) : generator(seed ^ 0x9e3779b97f4a7c15ULL) {}
+    void extend(std::size_t count);
+    std::mt19937_64 generator;
+    std::vector<double> unit;
+};
+std::vector<double> fillerCentres(const Rect2& core, const FillerPlan& plan, FillerNumbers& numbers);
 
 // The whole session setup (AdaptiveGlobalPlacer.cpp:114-126 plus buildHostLayout,
 // CudaPlacementBackend.cu:784-839).  `fillers` receives the filler geometry.

@@ -163,6 +163,7 @@ HostTransfer::Call::Call(HostTransfer* transfer) : transfer_(transfer) {
     if (transfer_ == nullptr) return;
     HostTransfer& t = *transfer_;
     t.helped_ = t.hub_ != nullptr && t.hub_->acquire();
+    t.moved_ = 0;
     t.ring_ = t.helped_ ? t.hub_->ring() : t.own_.data();
     t.slots_ = t.helped_ ? kHubSlots : kOwnSlots;
     t.slot_bytes_ = t.helped_ ? kHubSlotBytes : t.own_slot_bytes_;
@@ -187,10 +188,30 @@ struct HostTransfer::Download {
 };
 
 bool HostTransfer::upload(const double* source, double* destination, std::size_t count, bool check) {
+    return move(reinterpret_cast<const unsigned char*>(source), reinterpret_cast<unsigned char*>(destination),
+                count * sizeof(double), check);
+}
+
+void HostTransfer::send(const void* source, void* destination, std::size_t bytes) {
+    if (bytes == 0) return;
+    if (helped_ && bytes >= kLargeBytes) {
+        move(static_cast<const unsigned char*>(source), static_cast<unsigned char*>(destination), bytes, false);
+    } else {
+        checkCuda(cudaMemcpyAsync(destination, source, bytes, cudaMemcpyHostToDevice, stream_), "Upload to the device");
+    }
+}
+
+bool HostTransfer::move(const unsigned char* source, unsigned char* destination, std::size_t bytes, bool check) {
+    // Slots that an earlier move of this call still uses: its last copies, from the last slots' events.
+    if (in_flight_) {
+        for (std::size_t k = 0; k < std::min(slots_, moved_); ++k) {
+            checkCuda(cudaEventSynchronize(events_[k]), "Wait for earlier transfers");
+        }
+    }
     in_flight_ = true;
-    const std::size_t per_slot = slot_bytes_ / sizeof(double);
-    const std::size_t chunks = (count + per_slot - 1) / per_slot;
-    const auto size = [&](std::size_t k) { return std::min(per_slot, count - k * per_slot); };
+    const std::size_t chunks = (bytes + slot_bytes_ - 1) / slot_bytes_;
+    moved_ = chunks;
+    const auto size = [&](std::size_t k) { return std::min(slot_bytes_, bytes - k * slot_bytes_); };
     std::atomic<bool> finite{true};
     // Chunks below `allowed` may use their slot and are claimed in order.
     std::atomic<std::size_t> next{0}, allowed{std::min(chunks, slots_)};
@@ -202,8 +223,11 @@ bool HostTransfer::upload(const double* source, double* destination, std::size_t
         do {
             if (k >= allowed.load(std::memory_order_acquire)) return false;
         } while (!next.compare_exchange_weak(k, k + 1, std::memory_order_relaxed));
-        std::memcpy(slot(k), source + k * per_slot, size(k) * sizeof(double));
-        if (check && !allFinite(source + k * per_slot, size(k))) finite.store(false, std::memory_order_relaxed);
+        const unsigned char* from = source + k * slot_bytes_;
+        std::memcpy(slot(k), from, size(k));
+        if (check && !allFinite(reinterpret_cast<const double*>(from), size(k) / sizeof(double))) {
+            finite.store(false, std::memory_order_relaxed);
+        }
         filled[k].store(1, std::memory_order_release);
         return true;
     };
@@ -224,8 +248,8 @@ bool HostTransfer::upload(const double* source, double* destination, std::size_t
     std::size_t sent = 0, done = 0;  // chunks given to the copy engine, and out of their slots
     while (sent < chunks) {
         if (filled[sent].load(std::memory_order_acquire) != 0) {
-            checkCuda(cudaMemcpyAsync(destination + sent * per_slot, slot(sent), size(sent) * sizeof(double),
-                                      cudaMemcpyHostToDevice, stream_),
+            checkCuda(cudaMemcpyAsync(destination + sent * slot_bytes_, slot(sent), size(sent), cudaMemcpyHostToDevice,
+                                      stream_),
                       "Upload to the device");
             checkCuda(cudaEventRecord(events_[sent % slots_], stream_), "Record an upload");
             ++sent;

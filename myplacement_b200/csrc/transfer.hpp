@@ -83,6 +83,9 @@ public:
     // Copies `count` doubles to the device on the stream.  With `check`, returns whether all
     // are finite.  The source has been read when this returns.
     bool upload(const double* source, double* destination, std::size_t count, bool check);
+    // Copies bytes to the device on the stream; the source has been read when this returns.
+    // Bytes that are few, or beside another thread's call, take the driver's own staging.
+    void send(const void* source, void* destination, std::size_t bytes);
 
     struct Piece {
         const void* device = nullptr;
@@ -105,6 +108,7 @@ private:
     };
     struct Download;
     [[nodiscard]] unsigned char* slot(std::size_t k) const { return ring_ + (k % slots_) * slot_bytes_; }
+    bool move(const unsigned char* source, unsigned char* destination, std::size_t bytes, bool check);
     void issue(std::size_t k);
     [[nodiscard]] bool arrived(std::size_t k);
     bool copyOne(Download& download);
@@ -122,6 +126,7 @@ private:
     std::vector<Chunk> chunks_;  // of the download in progress
     std::unique_ptr<Download> download_;
     std::size_t issued_ = 0;
+    std::size_t moved_ = 0;   // chunks of the call's last move
     bool in_flight_ = false;  // copies that nothing has waited for may still use the slots
 };
 
