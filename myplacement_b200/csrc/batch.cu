@@ -12,6 +12,7 @@
 
 #include "common.cuh"
 #include "dct_tc.cuh"
+#include "field_small.cuh"
 #include "field_tc.cuh"
 
 namespace mpgp {
@@ -38,6 +39,13 @@ constexpr int kInverseX = 4;           // the banded solve's inverse along x (En
 struct FieldGroup {
     FieldShape shape;
     std::vector<FieldItem> items;
+    std::size_t at = 0;
+};
+
+// The small-grid items of a round with one shape.
+struct SmallFieldGroup {
+    FieldSmallShape shape;
+    std::vector<FieldSmallItem> items;
     std::size_t at = 0;
 };
 
@@ -107,7 +115,12 @@ void Batch::reserve(std::size_t bytes) {
 }
 
 void Batch::attach(Engine* engine) {
-    engine->deviceBatches();  // the contraction descriptors the batched launches read
+    // The descriptors the batched launches read.
+    if (engine->smallField()) {
+        engine->deviceSmallField();
+    } else {
+        engine->deviceBatches();
+    }
     if (engine->banded()) engine->deviceField();
     std::lock_guard<std::mutex> lock(mutex_);
     ++attached_;
@@ -195,6 +208,7 @@ void Batch::execute(const std::vector<Request*>& round) {
     std::vector<int> scatter, metrics, gather;
     std::vector<TcItem> items[kContractionStages][kMaxSplit];
     std::vector<FieldGroup> fields;
+    std::vector<SmallFieldGroup> smalls;
     bool mixed_split = false;  // an instance whose stages use different splits (its stages must share a stream)
     int staged = 0;
     for (int i = 0; i < n; ++i) {
@@ -205,6 +219,17 @@ void Batch::execute(const std::vector<Request*>& round) {
         if (p.gather) gather.push_back(i);
         const int total = p.reduce_args.offsets[p.reduce_args.source_count];
         if (total <= p.reduce_args.staged_capacity) staged = std::max(staged, total);
+        if (engine->smallField()) {
+            if (!p.forward && !p.gradient) continue;
+            const FieldSmallShape& shape = engine->fieldSmall().shape;
+            auto group = std::find_if(smalls.begin(), smalls.end(), [&](const SmallFieldGroup& g) {
+                return g.shape.cluster == shape.cluster && g.shape.share_n == shape.share_n;
+            });
+            if (group == smalls.end()) group = smalls.insert(smalls.end(), SmallFieldGroup{shape, {}, 0});
+            const int mode = (p.forward ? kSmallForward : 0) | (p.gradient ? kSmallGradient : 0);
+            group->items.push_back(FieldSmallItem{engine->deviceSmallField(), mode});
+            continue;
+        }
         const TcBatch* device_batches = engine->deviceBatches();
         if (engine->banded()) {
             // The banded launch (as Engine::runDct), then the inverse along x with the
@@ -268,6 +293,7 @@ void Batch::execute(const std::vector<Request*>& round) {
         for (int k = 0; k < kMaxSplit; ++k) at_items[stage][k] = layout.add<TcItem>(items[stage][k].size());
     }
     for (FieldGroup& g : fields) g.at = layout.add<FieldItem>(g.items.size());
+    for (SmallFieldGroup& g : smalls) g.at = layout.add<FieldSmallItem>(g.items.size());
     reserve(layout.bytes);
 
     unsigned char* host = host_args_;
@@ -316,6 +342,9 @@ void Batch::execute(const std::vector<Request*>& round) {
         }
     }
     for (const FieldGroup& g : fields) std::memcpy(host + g.at, g.items.data(), g.items.size() * sizeof(FieldItem));
+    for (const SmallFieldGroup& g : smalls) {
+        std::memcpy(host + g.at, g.items.data(), g.items.size() * sizeof(FieldSmallItem));
+    }
 
     unsigned char* dev = device_args_;
     const auto on_device = [&](std::size_t at) { return dev + at; };
@@ -344,6 +373,24 @@ void Batch::execute(const std::vector<Request*>& round) {
         launchMetricsSplitBatch(reinterpret_cast<const MetricsArgs*>(on_device(at_metrics)),
                                 reinterpret_cast<const int*>(on_device(at_metrics_offsets)),
                                 static_cast<int>(metrics.size()), metrics_blocks, stream_);
+        ++launches;
+    }
+    // The small grids' one-launch solves depend on no other instance's launches: with more
+    // than one of them (one per shape), or banded or staged instances in the round, they are
+    // dealt to this stream and the second one.
+    bool others = !fields.empty();
+    for (const auto& stage : items) {
+        for (const auto& of_split : stage) others = others || !of_split.empty();
+    }
+    const bool aside = smalls.size() > (others ? 0U : 1U);
+    if (aside) {
+        checkCuda(cudaEventRecord(split_fork_, stream_), "Batch split fork");
+        checkCuda(cudaStreamWaitEvent(split_, split_fork_, 0), "Batch split fork");
+    }
+    for (std::size_t g = 0; g < smalls.size(); ++g) {
+        launchFieldSmallBatch(reinterpret_cast<const FieldSmallItem*>(on_device(smalls[g].at)),
+                              static_cast<int>(smalls[g].items.size()), smalls[g].shape,
+                              aside && (g % 2 == 0) == others ? split_ : stream_);
         ++launches;
     }
     // The banded field solves, one launch per cluster shape.
@@ -375,7 +422,7 @@ void Batch::execute(const std::vector<Request*>& round) {
             ++launches;
         }
     }
-    if (both) {
+    if (both || aside) {
         checkCuda(cudaEventRecord(split_join_, split_), "Batch split join");
         checkCuda(cudaStreamWaitEvent(stream_, split_join_, 0), "Batch split join");
     }

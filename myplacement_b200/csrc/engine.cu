@@ -530,11 +530,6 @@ void Engine::buildTensorCoreBasis() {
                      max_scale, stream_);
     for (int t = 0; t < kBasisCount; ++t) host_scales.exp_basis[t] = exponents[t];
     tc_source_ = newSplit(ny, nx, "source planes");
-    tc_x1t_ = newSplit(nx, ny, "DCT stage planes");
-    tc_phi_ = newSplit(ny, nx, "potential coefficient planes");
-    tc_phit_ = newSplit(nx, ny, "potential coefficient planes");
-    tc_t_ = newSplit(ny, nx, "DCT stage planes");
-    tc_ut_ = newSplit(nx, ny, "DCT stage planes");
     tc_row_exp_ = arena_.array<int>(static_cast<std::size_t>(ny), "source plane exponents");
     tc_scales_ = arena_.array<TcScales>(1, "field scales");
     checkCuda(cudaMemcpyAsync(tc_scales_, &host_scales, sizeof(TcScales), cudaMemcpyHostToDevice, stream_),
@@ -547,6 +542,45 @@ void Engine::buildTensorCoreBasis() {
     // Output bounds |C| <= gain * max |data operand|, with a margin for FP32 rounding.
     constexpr double kMargin = 1.02;
     TcScales* sc = tc_scales_;
+    // Grids of at most kFieldSmallMax rows and columns take the one-launch solve (field_small.cu);
+    // MPGP_FIELD_SOLVE=staged or =banded chooses another for every grid that one takes.
+    const char* solve = std::getenv("MPGP_FIELD_SOLVE");
+    const bool wants_staged = solve != nullptr && std::strcmp(solve, "staged") == 0;
+    const bool wants_banded = solve != nullptr && std::strcmp(solve, "banded") == 0;
+    const FieldSmallShape small_shape = wants_staged || wants_banded ? FieldSmallShape{} : fieldSmallShape(nx, ny);
+    if (small_shape.cluster > 0) {
+        FieldSmall& f = small_field_;
+        makeOperandMap(&f.map_s, tc_source_, kTileM);
+        makeOperandMap(&f.map_cy, tc_cy_, kTileM);
+        makeOperandMap(&f.map_dy, tc_dy_, kTileM);
+        makeOperandMap(&f.map_syw, tc_syw_, kTileM);
+        makeOperandMap(&f.map_cx, tc_cx_, small_shape.share_n);
+        makeOperandMap(&f.map_dxc, tc_dxc_, small_shape.share_n);
+        makeOperandMap(&f.map_sxwt, tc_sxwt_, small_shape.share_n);
+        f.nx = nx;
+        f.ny = ny;
+        f.shape = small_shape;
+        f.row_exp = tc_row_exp_;
+        f.scales = sc;
+        f.scale = spectral_scale_;
+        f.gain_x = static_cast<float>(row_l1[kCx] * kMargin);
+        f.gain_phi = static_cast<float>(row_l1[kCy] * max_scale * kMargin);
+        f.gain_t = static_cast<float>(row_l1[kDy] * kMargin);
+        f.gain_u = static_cast<float>(row_l1[kDxc] * kMargin);
+        f.field = field_;
+        f.potential = potential_;
+        f.phi_store = arena_.array<unsigned char>(fieldSmallStoreBytes(nx, ny), "kept field coefficients");
+        f.error_flag = tc_error_;
+        energy_blocks_ = small_shape.cluster;
+        partials_e_ = arena_.array<double>(static_cast<std::size_t>(energy_blocks_), "energy partials");
+        f.energy_partials = partials_e_;
+        return;
+    }
+    tc_x1t_ = newSplit(nx, ny, "DCT stage planes");
+    tc_phi_ = newSplit(ny, nx, "potential coefficient planes");
+    tc_phit_ = newSplit(nx, ny, "potential coefficient planes");
+    tc_t_ = newSplit(ny, nx, "DCT stage planes");
+    tc_ut_ = newSplit(nx, ny, "DCT stage planes");
     const auto task = [&](TcTask& t, const SplitMatrix& a, const SplitMatrix& b, int m, int n, int k, int mode) {
         std::memset(static_cast<void*>(&t), 0, sizeof(TcTask));
         makeOperandMap(&t.map_a, a, kTileM);
@@ -644,10 +678,7 @@ void Engine::buildTensorCoreBasis() {
     // Ey = M2 Dx^T and the potential M1 Dx^T over all bands.
     // The banded solve for grids taller than kFieldBandedMinRows rows (up to its limits);
     // MPGP_FIELD_SOLVE=staged or =banded chooses for every grid the banded solve takes.
-    const char* solve = std::getenv("MPGP_FIELD_SOLVE");
-    bool banded = ny > kFieldBandedMinRows;
-    if (solve != nullptr && std::strcmp(solve, "staged") == 0) banded = false;
-    if (solve != nullptr && std::strcmp(solve, "banded") == 0) banded = true;
+    const bool banded = wants_banded || (ny > kFieldBandedMinRows && !wants_staged);
     const FieldShape shape = banded ? fieldShape(nx, ny) : FieldShape{};
     banded_ = shape.cluster > 0;
     if (banded_) {
@@ -714,6 +745,7 @@ void Engine::setStallProbe(long long polls) {
         b->stall_polls = std::max(0LL, polls);
     }
     field_band_.stall_polls = std::max(0LL, polls);
+    small_field_.stall_polls = std::max(0LL, polls);
 }
 
 const char* kernelKindName(int kind) {
@@ -794,6 +826,17 @@ void Engine::runDct(bool gradient, bool potential, bool forward, bool split_sour
     runStagedField(gradient, potential, forward, split_source);
 }
 
+// One launch (field_small.cu); without the forward flag from the coefficients the last
+// forward launch kept.
+void Engine::runSmallField(bool gradient, bool potential, bool forward) {
+    if (!forward && !gradient) return;
+    const int mode = (forward ? kSmallForward : 0) | (gradient ? kSmallGradient : 0) | (potential ? kSmallPotential : 0);
+    beginKernel(!gradient ? kKindFieldForward : (forward ? kKindFieldGradient : kKindFieldInverse));
+    launchFieldSmall(small_field_, mode, stream_);
+    endKernel();
+    launches_ += 1;
+}
+
 void Engine::runBandedField(bool gradient, bool forward, bool split_source) {
     const int nx = bins_x_;
     if (forward && split_source) {
@@ -831,13 +874,17 @@ void Engine::runBandedInverseX(bool gradient, bool potential) {
 
 void Engine::runStagedField(bool gradient, bool potential, bool forward, bool split_source) {
     const int nx = bins_x_;
+    if (forward && split_source) {
+        beginKernel(kKindDctSplit);
+        launchSplitSource(source_, tc_source_, nx, tc_row_exp_, tc_scales_, stream_);
+        endKernel();
+        launches_ += 1;
+    }
+    if (smallField()) {
+        runSmallField(gradient, potential, forward);
+        return;
+    }
     if (forward) {
-        if (split_source) {
-            beginKernel(kKindDctSplit);
-            launchSplitSource(source_, tc_source_, nx, tc_row_exp_, tc_scales_, stream_);
-            endKernel();
-            launches_ += 1;
-        }
         beginKernel(kKindDctForward);
         launchTcGemm(tc_fwd1_, 1, stream_);
         endKernel();
@@ -1151,6 +1198,16 @@ const FieldBand* Engine::deviceField() {
         checkCuda(cudaStreamSynchronize(stream_), "Upload the field descriptor");
     }
     return device_field_;
+}
+
+const FieldSmall* Engine::deviceSmallField() {
+    if (device_small_field_ == nullptr) {
+        device_small_field_ = arena_.array<FieldSmall>(1, "batched field descriptor");
+        checkCuda(cudaMemcpyAsync(device_small_field_, &small_field_, sizeof(FieldSmall), cudaMemcpyHostToDevice, stream_),
+                  "Upload the field descriptor");
+        checkCuda(cudaStreamSynchronize(stream_), "Upload the field descriptor");
+    }
+    return device_small_field_;
 }
 
 const TcBatch& Engine::contraction(int stage) const {

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "dct_tc.cuh"
+#include "field_small.cuh"
 #include "field_tc.cuh"
 #include "ingest.cuh"
 #include "kernels.cuh"
@@ -140,9 +141,9 @@ enum KernelKind : int {
     kKindVector,
     kKindDctSplit,
     kKindRudy,
-    kKindFieldForward,   // the banded field solve without the inverse passes
-    kKindFieldGradient,  // the banded field solve with them
-    kKindFieldInverse,   // the banded field solve's inverse passes alone
+    kKindFieldForward,   // the banded or one-launch field solve without the inverse passes
+    kKindFieldGradient,  // with them
+    kKindFieldInverse,   // the inverse passes alone
     kKindCount
 };
 const char* kernelKindName(int kind);
@@ -197,10 +198,14 @@ public:
     // solve's descriptor, copied to device memory for batched launches; uploaded on first use.
     const TcBatch* deviceBatches();
     const FieldBand* deviceField();
+    const FieldSmall* deviceSmallField();
     [[nodiscard]] const TcBatch& contraction(int stage) const;
-    // The field solve is banded (field_tc.cu) rather than staged (four contraction launches).
+    // The field solve is banded (field_tc.cu) or, for a small grid, one launch
+    // (field_small.cu) rather than staged (four contraction launches).
     [[nodiscard]] bool banded() const { return banded_; }
     [[nodiscard]] const FieldBand& fieldBand() const { return field_band_; }
+    [[nodiscard]] bool smallField() const { return small_field_.shape.cluster > 0; }
+    [[nodiscard]] const FieldSmall& fieldSmall() const { return small_field_; }
     // Stops taking part in the batch's rounds (the placement has finished); a later
     // evaluation still runs through the batch.
     void leaveBatch();
@@ -300,6 +305,7 @@ private:
     void runDct(bool gradient, bool potential, bool forward, bool split_source = true);
     void runBandedField(bool gradient, bool forward, bool split_source);
     void runBandedInverseX(bool gradient, bool potential);
+    void runSmallField(bool gradient, bool potential, bool forward);
     void runStagedField(bool gradient, bool potential, bool forward, bool split_source);
     void runWirelengthPass(const EvalPlan& p);
     void uploadStatic(const Problem& problem);
@@ -374,6 +380,8 @@ private:
     bool banded_ = false;
     FieldBand field_band_{};
     FieldBand* device_field_ = nullptr;
+    FieldSmall small_field_{};
+    FieldSmall* device_small_field_ = nullptr;
     SplitMatrix tc_m1_, tc_m2_;
     TcBatch tc_invx_{}, tc_potx_{};
     int* tc_row_exp_ = nullptr;

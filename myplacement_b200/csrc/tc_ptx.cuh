@@ -1,4 +1,4 @@
-// Inline PTX shared by the tcgen05 contraction kernels (dct_tc.cu, field_tc.cu):
+// Inline PTX shared by the tcgen05 contraction kernels (dct_tc.cu, field_tc.cu, field_small.cu):
 // shared-memory and cluster addressing, mbarriers with bounded waits, TMA and
 // shared-to-shared bulk copies, UMMA descriptors and issue, TMEM loads, and the
 // plane split of eight values.
@@ -143,6 +143,21 @@ __device__ __forceinline__ void tmemLoad16(uint32_t address, uint32_t (&r)[16]) 
 __device__ __forceinline__ void tmemWait(uint32_t (&a)[16], uint32_t (&b)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]), "+r"(a[8]), "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15]), "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7]), "+r"(b[8]), "+r"(b[9]), "+r"(b[10]), "+r"(b[11]), "+r"(b[12]), "+r"(b[13]), "+r"(b[14]), "+r"(b[15])
+                 :
+                 : "memory");
+}
+
+// The eight-column form of tmemLoad16 and tmemWait.
+__device__ __forceinline__ void tmemLoad8(uint32_t address, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(address));
+}
+
+__device__ __forceinline__ void tmemWait(uint32_t (&a)[8], uint32_t (&b)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
+                   "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7])
                  :
                  : "memory");
 }
