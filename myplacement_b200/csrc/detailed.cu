@@ -15,14 +15,19 @@
 // arithmetic (products and sums rounded separately) against the placement the
 // earlier acceptances left.  A second kernel evaluates that rule
 // speculatively: every window's before and after values on the assumption
-// that each earlier window decided as the previous round said, for a few
-// rounds.  The host walks the windows in the reference's order and takes the
-// device's values unless a net of the window belongs to an earlier window
-// whose actual decision differed from the assumption; only those windows are
-// re-evaluated on the host.  The segment ends the reference keeps on the host
-// (two or three cells, every order by its exhaustive rule) go through a tail
-// kernel the same way, after the four-cell windows.  The result is the
-// reference's exactly.
+// that each earlier window decided as the previous round said.  The segment ends
+// the reference keeps on the host (two or three cells, every order by its
+// exhaustive rule) go through a tail kernel the same way, after the four-cell
+// windows.  The result is the reference's exactly.
+//
+// Whole passes run on the device (placeOnDevice): it builds the windows and
+// repeats the rounds until one changes no decision.  Where the host has to look,
+// it builds the windows (buildWindows), the device runs a few rounds, and the
+// host walks the windows in the reference's order: it takes the device's values
+// unless a net of the window belongs to an earlier window whose actual decision
+// differed from the assumption, and re-evaluates only those windows.
+#include <cub/device/device_radix_sort.cuh>
+#include <cub/device/device_scan.cuh>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,13 +36,19 @@
 #include <cstdint>
 #include <cstring>
 #include <limits>
+#include <memory>
 #include <numeric>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
+#include "design_setup.cuh"
 #include "detailed.hpp"
+#include "ingest.cuh"
+#include "pinned.hpp"
 #include "setup.hpp"
+#include "transfer.hpp"
 #include "workers.hpp"
 
 namespace mpgp {
@@ -47,7 +58,7 @@ constexpr int kWindow = 4;
 constexpr int kOrders = 24;
 constexpr int kCurrentLane = kOrders;  // the lane that evaluates the placement as it is
 constexpr int kWindowsPerBlock = 8;
-constexpr int kSpeculations = 3;  // rounds of speculative re-decision on the device
+constexpr int kSpeculations = 3;  // rounds of speculative re-decision beside the host's walk
 constexpr int kOrientationUnknown = 8;
 constexpr double kLargest = std::numeric_limits<double>::max();
 
@@ -95,15 +106,308 @@ struct WindowArrays {
     const int* nets;
 };
 
+// What a window of a pass is: evaluated as a four-cell window, as a tail (a segment end), or not.
+enum WindowKind : uint8_t { kNotEvaluated = 0, kFourCells = 1, kTail = 2 };
+
+// Rounds of re-decision until nothing changes (stamp != null): in round k a window is
+// evaluated again if a window that shares a net with it changed its decision in round k - 1
+// (every window in round 1), otherwise it decides as before.  A round after one without a
+// change does nothing.
+struct Rounds {
+    int round = 0;
+    int* stamp = nullptr;    // per net: the latest round that has to look at its windows again
+    int* changed = nullptr;  // per round: decisions that differ from the round's input
+};
+
+// Whether the warp's window has nothing new to decide in this round.
+__device__ __forceinline__ bool settledWindow(const Rounds& r, const int* nets, int first, int last) {
+    if (r.round <= 1) return false;
+    bool again = false;
+    for (int e = first + static_cast<int>(threadIdx.x & 31); e < last; e += 32) again = again || __ldcg(r.stamp + nets[e]) >= r.round;
+    return __any_sync(0xffffffffu, again ? 1 : 0) == 0;
+}
+
+// The window changed its decision in this round: its nets' windows are looked at in the next one.
+__device__ __forceinline__ void stampWindow(const Rounds& r, const int* nets, int first, int last) {
+    for (int e = first + static_cast<int>(threadIdx.x & 31); e < last; e += 32) __stcg(r.stamp + nets[e], r.round + 1);
+    if ((threadIdx.x & 31) == 0) atomicAdd(r.changed + r.round, 1);
+}
+
+constexpr int kPinChunk = 64;  // pins a warp loads at a time, two per lane
+
+// The pins of up to 32 nets one net after another, so that a warp's lanes load a pin each
+// whatever the nets' degrees: lane e holds net e's part.
+struct PinRun {
+    int offset = 0;  // of the net's first pin in the run
+    int degree = 0;
+    int shift = 0;   // first pin - offset
+    int count = 0;   // nets
+    int total = 0;   // pins
+};
+
+__device__ __forceinline__ PinRun pinRun(const int* nets, int count, const int* net_pin_start) {
+    const int lane = threadIdx.x & 31;
+    PinRun run;
+    run.count = count;
+    int first = 0;
+    if (lane < count) {
+        const int net = nets[lane];
+        first = net_pin_start[net];
+        run.degree = net_pin_start[net + 1] - first;
+    }
+    int end = run.degree;  // inclusive scan
+#pragma unroll
+    for (int step = 1; step < 32; step <<= 1) {
+        const int other = __shfl_up_sync(0xffffffffu, end, step);
+        if (lane >= step) end += other;
+    }
+    run.offset = end - run.degree;
+    run.shift = first - run.offset;
+    run.total = __shfl_sync(0xffffffffu, end, 31);
+    return run;
+}
+
+// The pin at place at + lane of the run (a whole warp calls it; past the end, some pin of the
+// run).  The nets of a window have a pin at least, so each begins at a place of its own.
+__device__ __forceinline__ int pinAt(const PinRun& run, int at) {
+    const int lane = threadIdx.x & 31;
+    const bool net = lane < run.count;
+    const int begun = __popc(__ballot_sync(0xffffffffu, net && run.offset < at ? 1 : 0));
+    const unsigned begins = __reduce_or_sync(
+        0xffffffffu, net && run.offset >= at && run.offset < at + 32 ? 1u << (run.offset - at) : 0u);
+    const int e = begun + __popc(begins & (0xffffffffu >> (31 - lane))) - 1;
+    return __shfl_sync(0xffffffffu, run.shift, e) + min(at + lane, run.total - 1);
+}
+
+// Up to 32 nets of a window, as the lanes that try the window's orders need them: of each net
+// the box of its pins on other cells, which no order moves, and its pins on the window's own
+// cells.  The chains of loads (pin, cell, centre) bound the kernels; a warp follows 64 of them
+// at once and every lane then has only the window's own pins to place.  Of 210,000 cells the
+// tails took 344 us with every lane walking every pin, 182 with a net per lane and 124 so; the
+// four-cell windows 745, 410 and 430, and 220 (with 50 for the extremes) from the nets'
+// extremes below: a window of the design touches 16 nets of 153 pins, 16 of them its own.
+constexpr int kOwnPins = 64;  // of a batch of nets (about 14 are common); more take the pin by pin walk
+struct WindowNets {
+    double2 point[kPinChunk];
+    double2 low[32];
+    double2 high[32];
+    double2 offset[kOwnPins];
+    uint8_t cell[kOwnPins];
+    uint8_t start[36];  // the nets' ranges of the own pins
+};
+
+__device__ __forceinline__ int slotOf(const int (&module)[kWindow], int m) {
+    int slot = -1;
+#pragma unroll
+    for (int i = 0; i < kWindow; ++i) slot = module[i] == m ? i : slot;  // a window's cells are distinct
+    return slot;
+}
+
+// Gathers `count` <= 32 nets (a whole warp); false, for every lane, with more than kOwnPins own
+// pins.  position(p, m): a pin of another cell; offset(p, m): an own pin's offset.
+template <typename Position, typename Offset>
+__device__ __forceinline__ bool gatherNets(WindowNets& g, const int* nets, int count, const int* net_pin_start,
+                                           const int* pin_module, const int (&module)[kWindow],
+                                           const Position& position, const Offset& offset) {
+    const int lane = threadIdx.x & 31;
+    const PinRun run = pinRun(nets, count, net_pin_start);
+    double2 low = make_double2(kLargest, kLargest);
+    double2 high = make_double2(-kLargest, -kLargest);
+    int own = 0;        // of the lane's net
+    int own_total = 0;  // so far
+    __syncwarp();       // the last batch has been read
+    for (int at = 0; at < run.total; at += kPinChunk) {
+        int p[2], m[2], slot[2];
+        double2 v[2];
+        unsigned mine[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) p[u] = pinAt(run, at + 32 * u);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) m[u] = pin_module[p[u]];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            slot[u] = slotOf(module, m[u]);
+            v[u] = slot[u] < 0 ? position(p[u], m[u]) : offset(p[u], m[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            mine[u] = __ballot_sync(0xffffffffu, slot[u] >= 0 && at + 32 * u + lane < run.total ? 1 : 0);
+            g.point[32 * u + lane] = v[u];
+            const int to = own_total + __popc(mine[u] & ((1u << lane) - 1u));
+            if ((mine[u] >> lane & 1u) != 0u && to < kOwnPins) {
+                g.offset[to] = v[u];
+                g.cell[to] = static_cast<uint8_t>(slot[u]);
+            }
+            own_total += __popc(mine[u]);
+        }
+        __syncwarp();
+        const int stop = min(run.offset + run.degree, at + kPinChunk);
+        for (int k = max(run.offset, at); k < stop; ++k) {
+            const int i = k - at;
+            if ((mine[i >> 5] >> (i & 31) & 1u) != 0u) {
+                ++own;
+                continue;
+            }
+            const double2 c = g.point[i];
+            low.x = c.x < low.x ? c.x : low.x;  // std::min / std::max
+            high.x = high.x < c.x ? c.x : high.x;
+            low.y = c.y < low.y ? c.y : low.y;
+            high.y = high.y < c.y ? c.y : high.y;
+        }
+        __syncwarp();
+    }
+    if (own_total > kOwnPins) return false;
+    int end = own;  // inclusive scan
+#pragma unroll
+    for (int step = 1; step < 32; step <<= 1) {
+        const int other = __shfl_up_sync(0xffffffffu, end, step);
+        if (lane >= step) end += other;
+    }
+    g.low[lane] = low;
+    g.high[lane] = high;
+    g.start[lane + 1] = static_cast<uint8_t>(end);
+    if (lane == 0) g.start[0] = 0;
+    __syncwarp();
+    return true;
+}
+
+// The half perimeter of gathered net `e` with the window's cells at (cx, cy).
+__device__ __forceinline__ double gatheredSpan(const WindowNets& g, int e, const double (&cx)[kWindow],
+                                               const double (&cy)[kWindow]) {
+    double2 low = g.low[e];
+    double2 high = g.high[e];
+    for (int k = g.start[e]; k < g.start[e + 1]; ++k) {
+        const double2 o = g.offset[k];
+        const int slot = g.cell[k];
+        double x = cx[0], y = cy[0];
+#pragma unroll
+        for (int i = 1; i < kWindow; ++i) {
+            x = slot == i ? cx[i] : x;
+            y = slot == i ? cy[i] : y;
+        }
+        x += o.x;
+        y += o.y;
+        low.x = x < low.x ? x : low.x;
+        high.x = high.x < x ? x : high.x;
+        low.y = y < low.y ? y : low.y;
+        high.y = high.y < y ? y : high.y;
+    }
+    return (high.x - low.x) + (high.y - low.y);
+}
+
+// The same pin by pin.
+template <typename Position, typename Offset>
+__device__ __forceinline__ double walkedSpan(int net, const int* net_pin_start, const int* pin_module,
+                                             const int (&module)[kWindow], const double (&cx)[kWindow],
+                                             const double (&cy)[kWindow], const Position& position,
+                                             const Offset& offset) {
+    double2 low = make_double2(kLargest, kLargest);
+    double2 high = make_double2(-kLargest, -kLargest);
+    for (int p = net_pin_start[net]; p < net_pin_start[net + 1]; ++p) {
+        const int m = pin_module[p];
+        double2 at;
+        if (slotOf(module, m) >= 0) {
+            at = offset(p, m);
+#pragma unroll
+            for (int i = 0; i < kWindow; ++i) {
+                if (module[i] == m) at = make_double2(cx[i] + at.x, cy[i] + at.y);
+            }
+        } else {
+            at = position(p, m);
+        }
+        low.x = at.x < low.x ? at.x : low.x;
+        high.x = high.x < at.x ? at.x : high.x;
+        low.y = at.y < low.y ? at.y : low.y;
+        high.y = high.y < at.y ? at.y : high.y;
+    }
+    return (high.x - low.x) + (high.y - low.y);
+}
+
+// Calls take(net, half perimeter) on lanes below `active` for the window's nets in order, with
+// the lane's cells at (cx, cy); gather(base, count, position, offset) fills `g` with up to 32
+// of them.  The whole warp calls it.
+template <typename Position, typename Offset, typename Take, typename Gather>
+__device__ __forceinline__ void forWindowNets(WindowNets& g, const int* nets, int first, int last, int active,
+                                              const int* net_pin_start, const int* pin_module,
+                                              const int (&module)[kWindow], const double (&cx)[kWindow],
+                                              const double (&cy)[kWindow], const Position& position,
+                                              const Offset& offset, const Take& take, const Gather& gather) {
+    const int lane = threadIdx.x & 31;
+    for (int base = first; base < last; base += 32) {
+        const int count = min(32, last - base);
+        const bool gathered = gather(base, count, position, offset);
+        if (lane >= active) continue;
+        for (int e = 0; e < count; ++e) {
+            const int net = nets[base + e];
+            take(net, gathered ? gatheredSpan(g, e, cx, cy)
+                               : walkedSpan(net, net_pin_start, pin_module, module, cx, cy, position, offset));
+        }
+    }
+}
+
+// The least and greatest pin coordinates of a net, each with the window that owns the pin's cell
+// (-1: none) and the same over the pins of every other window: the box of the pins on other
+// cells than a window's, for any window, without a walk over the net.
+struct NetExtremes {
+    double2 low, high;            // over all pins
+    double2 next_low, next_high;  // over the pins of other owners than those below
+    int2 low_owner, high_owner;
+};
+
+// What a pass on the device knows of its windows' nets beside WindowArrays: entry e of the nets
+// has own pins pin[own[e]] .. pin[own[e + 1] - 1].
+struct OwnPins {
+    const int* own = nullptr;
+    const int* pin = nullptr;
+    const NetExtremes* extremes = nullptr;
+};
+
+// Fills `g` for `count` <= 32 nets of window w from the nets' extremes (gatherNets otherwise).
+__device__ __forceinline__ bool gatherFromExtremes(WindowNets& g, const OwnPins& pins, int w, const int* nets, int base,
+                                                   int count, const int* pin_module, const int (&module)[kWindow],
+                                                   const double2* pin_offset) {
+    const int lane = threadIdx.x & 31;
+    const int first = pins.own[base];
+    const int total = pins.own[base + count] - first;
+    if (total > kOwnPins) return false;
+    __syncwarp();  // the last batch has been read
+    for (int k = lane; k < total; k += 32) {
+        const int p = pins.pin[first + k];
+        g.offset[k] = pin_offset[p];
+        g.cell[k] = static_cast<uint8_t>(slotOf(module, pin_module[p]));
+    }
+    if (lane < count) {
+        const NetExtremes x = pins.extremes[nets[base + lane]];
+        g.low[lane] = make_double2(x.low_owner.x == w ? x.next_low.x : x.low.x,
+                                   x.low_owner.y == w ? x.next_low.y : x.low.y);
+        g.high[lane] = make_double2(x.high_owner.x == w ? x.next_high.x : x.high.x,
+                                    x.high_owner.y == w ? x.next_high.y : x.high.y);
+        g.start[lane + 1] = static_cast<uint8_t>(pins.own[base + lane + 1] - first);
+    }
+    if (lane == 0) g.start[0] = 0;
+    __syncwarp();
+    return true;
+}
+
+// kKnown: the nets' extremes and the windows' own pins are known (a pass on the device).
+template <bool kKnown>
 __global__ void __launch_bounds__(32 * kWindowsPerBlock)
     windowOrdersKernel(const double2* __restrict__ center, const double2* __restrict__ size,
                        const int* __restrict__ pin_module, const double2* __restrict__ pin_offset,
                        const int* __restrict__ net_pin_start, const double* __restrict__ net_weight,
-                       WindowArrays windows, int window_count, double epsilon, int* __restrict__ best_order,
-                       uint8_t* __restrict__ decided, double2* __restrict__ moved_center) {
+                       WindowArrays windows, int window_count, const uint8_t* __restrict__ kind, double epsilon,
+                       int* __restrict__ best_order, uint8_t* __restrict__ decided,
+                       double2* __restrict__ moved_center, OwnPins own_pins) {
     const int lane = threadIdx.x & 31;
     const int w = blockIdx.x * kWindowsPerBlock + static_cast<int>(threadIdx.x >> 5);
     if (w >= window_count) return;  // whole warps leave together
+    if (kind != nullptr && kind[w] != kFourCells) {
+        if (lane == 0) {
+            best_order[w] = 0;
+            decided[w] = 0;
+        }
+        return;
+    }
     const int4 m4 = windows.modules[w];
     const int module[kWindow] = {m4.x, m4.y, m4.z, m4.w};
 
@@ -142,37 +446,32 @@ __global__ void __launch_bounds__(32 * kWindowsPerBlock)
         }
     }
 
+    __shared__ WindowNets gathered[kWindowsPerBlock];
     double fused = 0.0;
     double plain = 0.0;
-    if (lane <= kCurrentLane) {
-        for (int e = windows.net_start[w]; e < windows.net_start[w + 1]; ++e) {
-            const int net = windows.nets[e];
-            double fmin_x = kLargest, fmax_x = -kLargest, fmin_y = kLargest, fmax_y = -kLargest;
-            double min_x = kLargest, max_x = -kLargest, min_y = kLargest, max_y = -kLargest;
-            for (int p = net_pin_start[net]; p < net_pin_start[net + 1]; ++p) {
-                const int m = pin_module[p];
-                double2 c = center[m];
-#pragma unroll
-                for (int i = 0; i < kWindow; ++i) {  // a window's cells are distinct: one match at most
-                    if (module[i] == m) c = make_double2(cx[i], cy[i]);
-                }
-                const double2 o = pin_offset[p];
-                const double x = c.x + o.x;
-                const double y = c.y + o.y;
-                fmin_x = fmin(fmin_x, x);
-                fmax_x = fmax(fmax_x, x);
-                fmin_y = fmin(fmin_y, y);
-                fmax_y = fmax(fmax_y, y);
-                min_x = x < min_x ? x : min_x;  // std::min / std::max
-                max_x = max_x < x ? x : max_x;
-                min_y = y < min_y ? y : min_y;
-                max_y = max_y < y ? y : max_y;
-            }
+    forWindowNets(
+        gathered[threadIdx.x >> 5], windows.nets, windows.net_start[w], windows.net_start[w + 1], kCurrentLane + 1,
+        net_pin_start, pin_module, module, cx, cy,
+        [&](int p, int m) {
+            const double2 c = center[m];
+            const double2 o = pin_offset[p];
+            return make_double2(c.x + o.x, c.y + o.y);
+        },
+        [&](int p, int) { return pin_offset[p]; },
+        [&](int net, double span) {
             const double weight = net_weight[net];
-            fused = fma(weight, (fmax_x - fmin_x) + (fmax_y - fmin_y), fused);
-            plain = __dadd_rn(plain, __dmul_rn(weight, (max_x - min_x) + (max_y - min_y)));
-        }
-    }
+            fused = fma(weight, span, fused);
+            plain = __dadd_rn(plain, __dmul_rn(weight, span));
+        },
+        [&](int base, int count, const auto& position, const auto& offset) {
+            WindowNets& g = gathered[threadIdx.x >> 5];
+            if constexpr (kKnown) {
+                return gatherFromExtremes(g, own_pins, w, windows.nets, base, count, pin_module, module, pin_offset);
+            } else {
+                return gatherNets(g, windows.nets + base, count, net_pin_start, pin_module, module, position, offset);
+            }
+        });
+    __syncwarp();
 
     // The smallest fused value, the lowest order on ties, to every lane.
     double best = lane < kOrders ? fused : kLargest;
@@ -216,8 +515,10 @@ __host__ __device__ inline double2 transformed(double2 o, int orientation) {
 // `decided_in` says, and the decisions they give.  A cell of an earlier window
 // assumed accepted sits where that window's best order puts it, with the
 // orientation of its row; every other cell is where the pass found it.  One
-// warp per window: each lane takes one net and forms its two terms (products
-// rounded separately), and the warp adds them in net order, as the host does.
+// warp per window: its lanes load the nets' pins (PinRun), each lane then forms
+// the two terms of one net (products rounded separately), and the warp adds them
+// in net order, as the host does: 490 us in the first round with a net per lane, 276 so
+// (51,000 windows of 210,000 cells).
 __global__ void __launch_bounds__(32 * kWindowsPerBlock)
     speculativeValuesKernel(const double2* __restrict__ center, const double2* __restrict__ moved_center,
                             const int* __restrict__ owner, const int8_t* __restrict__ moved_orientation,
@@ -226,74 +527,96 @@ __global__ void __launch_bounds__(32 * kWindowsPerBlock)
                             const double* __restrict__ net_weight, WindowArrays windows, int window_count,
                             const int* __restrict__ best_order, double epsilon, const uint8_t* __restrict__ decided_in,
                             uint8_t* __restrict__ decided_out, double* __restrict__ value_before,
-                            double* __restrict__ value_after) {
+                            double* __restrict__ value_after, Rounds rounds) {
     const int lane = threadIdx.x & 31;
     const int w = blockIdx.x * kWindowsPerBlock + static_cast<int>(threadIdx.x >> 5);
     if (w >= window_count) return;  // whole warps leave together
+    if (rounds.round > 1 && rounds.changed[rounds.round - 1] == 0) return;  // in and out agree
     const int best = best_order[w];
     if (best <= 0 || best >= kOrders) {
         if (lane == 0) decided_out[w] = 0;
         return;
     }
-    const int4 m4 = windows.modules[w];
     const int first = windows.net_start[w];
     const int last = windows.net_start[w + 1];
+    if (rounds.stamp != nullptr && settledWindow(rounds, windows.nets, first, last)) {
+        if (lane == 0) decided_out[w] = decided_in[w];
+        return;
+    }
+    __shared__ double4 chunk[kWindowsPerBlock][kPinChunk];
+    double4* const points = chunk[threadIdx.x >> 5];
     double before = 0.0;
     double after = 0.0;
     for (int base = first; base < last; base += 32) {
+        const int count = min(32, last - base);
+        const PinRun run = pinRun(windows.nets + base, count, net_pin_start);
+        double min_b = kLargest, max_b = -kLargest, min_by = kLargest, max_by = -kLargest;
+        double min_a = kLargest, max_a = -kLargest, min_ay = kLargest, max_ay = -kLargest;
+        for (int at = 0; at < run.total; at += kPinChunk) {
+            int p[2], m[2], own[2];
+            double2 now_c[2], offset[2];
+            bool moved[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) p[u] = pinAt(run, at + 32 * u);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) m[u] = pin_module[p[u]];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                now_c[u] = center[m[u]];
+                own[u] = owner[m[u]];
+                offset[u] = pin_offset[p[u]];
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) moved[u] = own[u] >= 0 && own[u] < w && decided_in[max(own[u], 0)] != 0;
+            __syncwarp();  // the last chunk has been read
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                double2 then_c = now_c[u];  // with this window's best order applied
+                if (own[u] == w) {
+                    then_c = moved_center[m[u]];  // its orientation changes only once accepted
+                } else if (moved[u]) {
+                    now_c[u] = moved_center[m[u]];
+                    then_c = now_c[u];
+                    offset[u] = transformed(raw_offset[p[u]], moved_orientation[m[u]]);
+                }
+                points[32 * u + lane] =
+                    make_double4(now_c[u].x + offset[u].x, now_c[u].y + offset[u].y, then_c.x + offset[u].x,
+                                 then_c.y + offset[u].y);
+            }
+            __syncwarp();
+            const int stop = min(run.offset + run.degree, at + kPinChunk);
+            for (int k = max(run.offset, at); k < stop; ++k) {
+                const double4 v = points[k - at];
+                min_b = v.x < min_b ? v.x : min_b;
+                max_b = max_b < v.x ? v.x : max_b;
+                min_by = v.y < min_by ? v.y : min_by;
+                max_by = max_by < v.y ? v.y : max_by;
+                min_a = v.z < min_a ? v.z : min_a;
+                max_a = max_a < v.z ? v.z : max_a;
+                min_ay = v.w < min_ay ? v.w : min_ay;
+                max_ay = max_ay < v.w ? v.w : max_ay;
+            }
+        }
         double term_before = 0.0;
         double term_after = 0.0;
-        const int e = base + lane;
-        if (e < last) {
-            const int net = windows.nets[e];
-            double min_b = kLargest, max_b = -kLargest, min_by = kLargest, max_by = -kLargest;
-            double min_a = kLargest, max_a = -kLargest, min_ay = kLargest, max_ay = -kLargest;
-            for (int p = net_pin_start[net]; p < net_pin_start[net + 1]; ++p) {
-                const int m = pin_module[p];
-                double2 offset = pin_offset[p];
-                double2 now_c;   // the cell now (before)
-                double2 then_c;  // the cell with this window's best order applied (after)
-                if (m == m4.x || m == m4.y || m == m4.z || m == m4.w) {
-                    now_c = center[m];
-                    then_c = moved_center[m];  // its orientation changes only once accepted
-                } else {
-                    const int j = owner[m];
-                    if (j >= 0 && j < w && decided_in[j] != 0) {
-                        now_c = moved_center[m];
-                        offset = transformed(raw_offset[p], moved_orientation[m]);
-                    } else {
-                        now_c = center[m];
-                    }
-                    then_c = now_c;
-                }
-                const double bx = now_c.x + offset.x;
-                const double by = now_c.y + offset.y;
-                const double ax = then_c.x + offset.x;
-                const double ay = then_c.y + offset.y;
-                min_b = bx < min_b ? bx : min_b;
-                max_b = max_b < bx ? bx : max_b;
-                min_by = by < min_by ? by : min_by;
-                max_by = max_by < by ? by : max_by;
-                min_a = ax < min_a ? ax : min_a;
-                max_a = max_a < ax ? ax : max_a;
-                min_ay = ay < min_ay ? ay : min_ay;
-                max_ay = max_ay < ay ? ay : max_ay;
-            }
-            const double weight = net_weight[net];
+        if (lane < count) {
+            const double weight = net_weight[windows.nets[base + lane]];
             term_before = __dmul_rn(weight, (max_b - min_b) + (max_by - min_by));
             term_after = __dmul_rn(weight, (max_a - min_a) + (max_ay - min_ay));
         }
-        const int terms = min(32, last - base);
-        for (int j = 0; j < terms; ++j) {
+        for (int j = 0; j < count; ++j) {
             before = __dadd_rn(before, __shfl_sync(0xffffffffu, term_before, j));
             after = __dadd_rn(after, __shfl_sync(0xffffffffu, term_after, j));
         }
     }
-    if (lane == 0) {
+    const uint8_t decision = after < before - epsilon ? 1 : 0;
+    if (rounds.stamp != nullptr) {
+        if (decision != decided_in[w]) stampWindow(rounds, windows.nets, first, last);
+    } else if (lane == 0) {
         value_before[w] = before;
         value_after[w] = after;
-        decided_out[w] = after < before - epsilon ? 1 : 0;
     }
+    if (lane == 0) decided_out[w] = decision;
 }
 
 // The windows the reference keeps on the host (segment ends of two or three
@@ -311,9 +634,10 @@ struct TailArrays {
 // Where each tail window's assumed order (-1: none) puts its cells.
 __global__ void __launch_bounds__(256)
     tailPlacementKernel(TailArrays tail, int tail_count, const double2* __restrict__ size,
-                        const int8_t* __restrict__ assumed, double2* __restrict__ moved_center) {
+                        const int8_t* __restrict__ assumed, double2* __restrict__ moved_center, Rounds rounds) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= tail_count || assumed[t] < 0) return;
+    if (rounds.round > 1 && rounds.changed[rounds.round - 1] == 0) return;
     const int n = tail.count[t];
     const int4 m4 = tail.modules[t];
     const int module[kWindow] = {m4.x, m4.y, m4.z, m4.w};
@@ -346,50 +670,28 @@ __global__ void __launch_bounds__(32 * kWindowsPerBlock)
                      const int8_t* __restrict__ moved_orientation, const double2* __restrict__ raw_offset,
                      const double2* __restrict__ size, const int* __restrict__ pin_module,
                      const int* __restrict__ net_pin_start, const double* __restrict__ net_weight, TailArrays tail,
-                     int tail_count, double epsilon, const int8_t* __restrict__ assumed_in,
-                     int8_t* __restrict__ order_out) {
+                     int tail_count, const uint8_t* __restrict__ kind, double epsilon,
+                     const int8_t* __restrict__ assumed_in, int8_t* __restrict__ order_out, Rounds rounds) {
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * kWindowsPerBlock + static_cast<int>(threadIdx.x >> 5);
     if (t >= tail_count) return;  // whole warps leave together
+    if (rounds.round > 1 && rounds.changed[rounds.round - 1] == 0) return;  // in and out agree
+    if (kind != nullptr && kind[t] != kTail) {
+        if (lane == 0) order_out[t] = -1;
+        return;
+    }
+    const int first = tail.net_start[t];
+    const int last = tail.net_start[t + 1];
+    if (rounds.stamp != nullptr && settledWindow(rounds, tail.nets, first, last)) {
+        if (lane == 0) order_out[t] = assumed_in[t];
+        return;
+    }
     const int n = tail.count[t];
     const int orders = factorialOf(n);
     const int4 m4 = tail.modules[t];
     const int module[kWindow] = {m4.x, m4.y, m4.z, m4.w};
     double cx[kWindow];
     double cy[kWindow];
-    // The window's weighted HPWL with its own cells at (cx, cy).
-    const auto value = [&]() {
-        double sum = 0.0;
-        for (int e = tail.net_start[t]; e < tail.net_start[t + 1]; ++e) {
-            const int net = tail.nets[e];
-            double min_x = kLargest, max_x = -kLargest, min_y = kLargest, max_y = -kLargest;
-            for (int p = net_pin_start[net]; p < net_pin_start[net + 1]; ++p) {
-                const int m = pin_module[p];
-                double2 c = center[m];
-                int turn = orientation[m];
-#pragma unroll
-                for (int i = 0; i < kWindow; ++i) {
-                    if (module[i] == m) c = make_double2(cx[i], cy[i]);
-                }
-                if (m != module[0] && m != module[1] && m != module[2] && m != module[3]) {
-                    const int j = owner[m] - tail_base;
-                    if (j >= 0 && j < t && assumed_in[j] >= 0) {
-                        c = moved_center[m];
-                        turn = moved_orientation[m];
-                    }
-                }
-                const double2 o = transformed(raw_offset[p], turn);
-                const double x = c.x + o.x;
-                const double y = c.y + o.y;
-                min_x = x < min_x ? x : min_x;
-                max_x = max_x < x ? x : max_x;
-                min_y = y < min_y ? y : min_y;
-                max_y = max_y < y ? y : max_y;
-            }
-            sum = __dadd_rn(sum, __dmul_rn(net_weight[net], (max_x - min_x) + (max_y - min_y)));
-        }
-        return sum;
-    };
 #pragma unroll
     for (int i = 0; i < kWindow; ++i) {
         const double2 c = module[i] >= 0 ? center[module[i]] : make_double2(0.0, 0.0);
@@ -417,7 +719,29 @@ __global__ void __launch_bounds__(32 * kWindowsPerBlock)
             cursor = __dadd_rn(cursor, roundedWidthDevice(s.x, tail.spacing[t]));
         }
     }
-    const double mine = lane <= orders ? value() : 0.0;
+    // The window's weighted HPWL with its own cells at (cx, cy).
+    __shared__ WindowNets gathered[kWindowsPerBlock];
+    double mine = 0.0;
+    forWindowNets(
+        gathered[threadIdx.x >> 5], tail.nets, first, last, orders + 1, net_pin_start, pin_module, module, cx, cy,
+        [&](int p, int m) {
+            double2 c = center[m];
+            int turn = orientation[m];
+            const int j = owner[m] - tail_base;
+            if (j >= 0 && j < t && assumed_in[j] >= 0) {
+                c = moved_center[m];
+                turn = moved_orientation[m];
+            }
+            const double2 o = transformed(raw_offset[p], turn);
+            return make_double2(c.x + o.x, c.y + o.y);
+        },
+        [&](int p, int m) { return transformed(raw_offset[p], orientation[m]); },
+        [&](int net, double span) { mine = __dadd_rn(mine, __dmul_rn(net_weight[net], span)); },
+        [&](int base, int count, const auto& position, const auto& offset) {
+            return gatherNets(gathered[threadIdx.x >> 5], tail.nets + base, count, net_pin_start, pin_module, module,
+                              position, offset);
+        });
+    __syncwarp();
     double best = __shfl_sync(0xffffffffu, mine, orders);
     int taken = -1;
     for (int k = 0; k < orders; ++k) {
@@ -427,6 +751,7 @@ __global__ void __launch_bounds__(32 * kWindowsPerBlock)
             taken = k;
         }
     }
+    if (rounds.stamp != nullptr && taken != assumed_in[t]) stampWindow(rounds, tail.nets, first, last);
     if (lane == 0) order_out[t] = static_cast<int8_t>(taken);
 }
 
@@ -497,6 +822,18 @@ public:
 
 private:
     cudaStream_t stream_ = nullptr;
+};
+
+class Event {
+public:
+    Event() { checkCuda(cudaEventCreateWithFlags(&event_, cudaEventDisableTiming), "cudaEventCreate"); }
+    ~Event() { cudaEventDestroy(event_); }
+    Event(const Event&) = delete;
+    Event& operator=(const Event&) = delete;
+    [[nodiscard]] cudaEvent_t get() const { return event_; }
+
+private:
+    cudaEvent_t event_ = nullptr;
 };
 
 // The placement state the passes change, with the design's fixed data.
@@ -764,6 +1101,805 @@ void buildWindows(const Placement& s, const std::vector<uint8_t>& standard, int 
     }
 }
 
+// ---- the whole pass on the device ------------------------------------------------------------
+//
+// From the host's lists above, a pass over 210,000 cells spent 23 ms around 2.4 ms of kernels:
+// rows, segments, windows and their nets (7 ms), the lists of each kind and the owners (4.5),
+// uploads (3.3), the walk over the decisions (4) and the tails (1.6); and a call 30 ms more for
+// the pin lists (10), 30 allocations (5) and the uploads of the design (6).  Here the design goes
+// up once and the passes are kernels: the cells are sorted by row and x, cut into segments and
+// windows by scans, and the windows' nets come from one stable sort of the pins by window.  The
+// decisions are re-evaluated until a round changes none: the k-th window's decision no longer
+// changes after k rounds (it rests on earlier windows only), so the rounds end, and the only
+// decisions that reproduce themselves are the ones the walk takes one after another.  After the
+// first round only windows with a net of a window that changed are evaluated.  Two passes over
+// 210,000 cells: 76.6 ms, and 5.8 so, of which the uploads take 1.5 and the kernels 2.5.
+
+constexpr int kMaxRounds = 1000;
+constexpr int kRoundsPerCheck = 4;  // launched before the host looks whether the last one changed anything
+constexpr double kSegmentEpsilon = 1e-6;
+
+int threadBlocks(std::size_t count) { return static_cast<int>((std::max<std::size_t>(count, 1) + kThreads - 1) / kThreads); }
+
+// The rows on the device: in bottom order for the search, and by index.
+struct DeviceRows {
+    int count = 0;
+    const double* centre = nullptr;  // sorted
+    const int* index = nullptr;      // sorted -> row
+    const double* bottom = nullptr;
+    const double* spacing = nullptr;
+    const int* turn = nullptr;       // orientation a moved cell takes, kOrientationUnknown: its own
+};
+
+// Counts of a pass that the host needs.
+struct PassCounts {
+    int windows = 0;
+    int ties = 0;  // cells at the same x of a row: the host sort's order of them is not ours to know
+    int four = 0;
+    int tails = 0;
+    unsigned long long permutations = 0;
+    unsigned long long accepted = 0;
+};
+
+__device__ __forceinline__ double lowerLeft(double centre, double extent) {
+    return __dsub_rn(centre, __dmul_rn(extent, 0.5));
+}
+
+// The caller's arrays on the device.
+struct RawDesign {
+    int modules = 0, nets = 0, pins = 0;
+    const double* x = nullptr;
+    const double* y = nullptr;
+    const double* width = nullptr;
+    const double* height = nullptr;
+    const int* flags = nullptr;
+    const int* orientation = nullptr;  // null: all N
+    const long long* net_start = nullptr;
+    const double* net_weight = nullptr;
+    const int* pin_module = nullptr;
+    const double* offset_x = nullptr;
+    const double* offset_y = nullptr;
+};
+
+// Raises *bad where validateDesign, or the check of the orientations, would refuse an entry.
+__global__ void __launch_bounds__(kThreads) checkDesignKernel(RawDesign d, int* bad) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    bool good = true;
+    if (i < d.nets) good = d.net_start[i + 1] >= d.net_start[i] && isfinite(d.net_weight[i]);
+    if (i < d.pins) {
+        const int m = d.pin_module[i];
+        good = good && m >= 0 && m < d.modules && isfinite(d.offset_x[i]) && isfinite(d.offset_y[i]);
+    }
+    if (i < d.modules) {
+        const double w = d.width[i], h = d.height[i];
+        good = good && w >= 0.0 && h >= 0.0 && isfinite(w) && isfinite(h) && isfinite(d.x[i]) && isfinite(d.y[i]);
+        if (d.orientation != nullptr) good = good && d.orientation[i] >= 0 && d.orientation[i] <= kOrientationUnknown;
+    }
+    if (!good) *bad = 1;
+}
+
+// deriveDesign's fixed and macro rules: a standard cell is neither.
+__global__ void __launch_bounds__(kThreads) detailedModulesKernel(RawDesign d, double nominal_row_height, double2* center,
+                                                                  double2* size, int8_t* turn, uint8_t* standard) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= d.modules) return;
+    const double height = d.height[m];
+    center[m] = make_double2(d.x[m], d.y[m]);
+    size[m] = make_double2(d.width[m], height);
+    turn[m] = d.orientation != nullptr ? static_cast<int8_t>(d.orientation[m]) : 0;
+    const bool terminal = (d.flags[m] & MPGP_MODULE_TERMINAL) != 0;
+    const bool fixed = terminal || (d.flags[m] & MPGP_MODULE_FIXED) != 0;
+    const bool macro = !terminal && nominal_row_height > kEpsilon && fabs(height - nominal_row_height) > kEpsilon;
+    standard[m] = !fixed && !macro ? 1 : 0;
+}
+
+__global__ void __launch_bounds__(kThreads) detailedNetsKernel(int count, const long long* start, int* start32,
+                                                               int* pin_net, int* pin_index) {
+    const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;  // eight lanes per net
+    if (n > count) return;
+    const long long first = start[n];
+    if ((threadIdx.x & 7) == 0) start32[n] = static_cast<int>(first);
+    if (n == count) return;
+    for (long long p = first + (threadIdx.x & 7); p < start[n + 1]; p += 8) {
+        pin_net[p] = n;
+        pin_index[p] = static_cast<int>(p);
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) rawOffsetsKernel(int count, const double* x, const double* y, double2* raw) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < count) raw[p] = make_double2(x[p], y[p]);
+}
+
+__global__ void __launch_bounds__(kThreads) turnedOffsetsKernel(int count, const double2* raw, const int* pin_module,
+                                                                const int8_t* turn, double2* offset) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < count) offset[p] = transformed(raw[p], turn[pin_module[p]]);
+}
+
+// The least value of a set of pins, its owner and the least value of other owners' pins.  (An
+// unowned pin may count as the others' owner too: no window asks without it.)
+struct LeastTwo {
+    double first = kLargest;
+    double next = kLargest;
+    int owner = -2;
+    __device__ __forceinline__ void join(double f, double n, int o) {
+        if (o == owner) {
+            next = n < next ? n : next;
+            first = f < first ? f : first;
+        } else if (f < first) {
+            next = first < n ? first : n;
+            first = f;
+            owner = o;
+        } else {
+            next = f < next ? f : next;
+        }
+    }
+    __device__ __forceinline__ void joinLane(int lanes) {
+        const double f = __shfl_xor_sync(0xffffffffu, first, lanes);
+        const double n = __shfl_xor_sync(0xffffffffu, next, lanes);
+        join(f, n, __shfl_xor_sync(0xffffffffu, owner, lanes));
+    }
+};
+
+// Eight lanes per net; the greatest values as the least negated ones.
+__global__ void __launch_bounds__(kThreads) netExtremesKernel(int count, const int* start, const int* pin_module,
+                                                              const double2* offset, const double2* center,
+                                                              const int* owner, NetExtremes* out) {
+    const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int last = n < count ? start[n + 1] : 0;
+    LeastTwo low_x, low_y, high_x, high_y;
+    for (int p = (n < count ? start[n] : 0) + static_cast<int>(threadIdx.x & 7); p < last; p += 8) {
+        const int m = pin_module[p];
+        const double2 c = center[m];
+        const double2 o = offset[p];
+        const int w = owner[m];
+        const double x = c.x + o.x;
+        const double y = c.y + o.y;
+        low_x.join(x, kLargest, w);
+        low_y.join(y, kLargest, w);
+        high_x.join(-x, kLargest, w);
+        high_y.join(-y, kLargest, w);
+    }
+#pragma unroll
+    for (int lanes = 4; lanes > 0; lanes >>= 1) {
+        low_x.joinLane(lanes);
+        low_y.joinLane(lanes);
+        high_x.joinLane(lanes);
+        high_y.joinLane(lanes);
+    }
+    if (n < count && (threadIdx.x & 7) == 0) {
+        out[n] = NetExtremes{make_double2(low_x.first, low_y.first),    make_double2(-high_x.first, -high_y.first),
+                             make_double2(low_x.next, low_y.next),      make_double2(-high_x.next, -high_y.next),
+                             make_int2(low_x.owner, low_y.owner), make_int2(high_x.owner, high_y.owner)};
+    }
+}
+
+// One net's weighted HPWL (Placement::netTerm; zero below two pins), eight lanes per net.
+__global__ void __launch_bounds__(kThreads) netTermsKernel(int count, const int* start, const int* pin_module,
+                                                           const double2* offset, const double2* center,
+                                                           const double* weight, double* term) {
+    const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int first = n < count ? start[n] : 0;
+    const int last = n < count ? start[n + 1] : 0;
+    double min_x = INFINITY, max_x = -INFINITY, min_y = INFINITY, max_y = -INFINITY;
+    for (int p = first + static_cast<int>(threadIdx.x & 7); p < last; p += 8) {
+        const double2 c = center[pin_module[p]];
+        const double2 o = offset[p];
+        const double x = c.x + o.x;
+        const double y = c.y + o.y;
+        min_x = x < min_x ? x : min_x;
+        max_x = max_x < x ? x : max_x;
+        min_y = y < min_y ? y : min_y;
+        max_y = max_y < y ? y : max_y;
+    }
+#pragma unroll
+    for (int offset_lane = 4; offset_lane > 0; offset_lane >>= 1) {
+        min_x = fmin(min_x, __shfl_xor_sync(0xffffffffu, min_x, offset_lane));
+        max_x = fmax(max_x, __shfl_xor_sync(0xffffffffu, max_x, offset_lane));
+        min_y = fmin(min_y, __shfl_xor_sync(0xffffffffu, min_y, offset_lane));
+        max_y = fmax(max_y, __shfl_xor_sync(0xffffffffu, max_y, offset_lane));
+    }
+    if (n < count && (threadIdx.x & 7) == 0) {
+        term[n] = last - first < 2 ? 0.0 : __dmul_rn(weight[n], (max_x - min_x) + (max_y - min_y));
+    }
+}
+
+// Each standard cell's row (buildWindows: the nearest row by centre, if the cell sits on its
+// bottom) and sort keys; the other modules sort behind every row.
+__global__ void __launch_bounds__(kThreads) cellRowsKernel(int count, const uint8_t* standard, const double2* center,
+                                                           const double2* size, DeviceRows rows, double* x_key,
+                                                           int* cell, int* row) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= count) return;
+    int r = rows.count;
+    const double2 c = center[m];
+    const double2 s = size[m];
+    if (standard[m] != 0) {
+        int lo = 0, hi = rows.count;  // first sorted row whose centre is not below the cell's
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (rows.centre[mid] < c.y) {
+                lo = mid + 1;
+            } else {
+                hi = mid;
+            }
+        }
+        int at = lo;
+        if (lo == rows.count) {
+            at = rows.count - 1;
+        } else if (lo > 0 && fabs(rows.centre[lo - 1] - c.y) <= fabs(rows.centre[lo] - c.y)) {
+            at = lo - 1;
+        }
+        const int nearest = rows.index[at];
+        if (fabs(lowerLeft(c.y, s.y) - rows.bottom[nearest]) <= kSegmentEpsilon) r = nearest;
+    }
+    x_key[m] = lowerLeft(c.x, s.x);
+    cell[m] = m;
+    row[m] = r;
+}
+
+__global__ void __launch_bounds__(kThreads) rowKeysKernel(int count, const int* cell, const int* row, unsigned* key) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < count) key[i] = static_cast<unsigned>(row[cell[i]]);
+}
+
+// first[i] = i where a segment begins (the row's first cell, or one that does not abut the cell
+// before it), else 0; a running maximum then gives every cell its segment's first position.
+__global__ void __launch_bounds__(kThreads) segmentsKernel(int count, const int* cell, const unsigned* row,
+                                                           const double2* center, const double2* size, DeviceRows rows,
+                                                           int* first, PassCounts* counts) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const unsigned r = row[i];
+    bool begins = true;
+    if (i > 0 && row[i - 1] == r && r < static_cast<unsigned>(rows.count)) {
+        const int previous = cell[i - 1];
+        const int m = cell[i];
+        const double left = lowerLeft(center[previous].x, size[previous].x);
+        const double mine = lowerLeft(center[m].x, size[m].x);
+        const double expected = __dadd_rn(left, roundedWidthDevice(size[previous].x, rows.spacing[r]));
+        begins = fabs(mine - expected) > kSegmentEpsilon;
+        if (mine == left) counts->ties = 1;
+    }
+    first[i] = begins ? i : 0;
+}
+
+__device__ __forceinline__ bool sameSegment(const int* first, const unsigned* row, int i, int j) {
+    return first[i] == first[j] && row[i] == row[j];
+}
+
+// begins[i] = 1 where a window begins: every kWindow-th cell of a segment from `phase` on that
+// has a cell after it; begins[count] = 0.
+__global__ void __launch_bounds__(kThreads) windowBeginsKernel(int count, int phase, int rows, const int* first,
+                                                               const unsigned* row, int* begins) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > count) return;
+    int b = 0;
+    if (i + 1 < count && row[i] < static_cast<unsigned>(rows)) {
+        const int q = i - first[i] - phase;
+        b = q >= 0 && q % kWindow == 0 && sameSegment(first, row, i, i + 1) ? 1 : 0;
+    }
+    begins[i] = b;
+}
+
+// A pass's windows in the reference's order (rows, then x), whatever their kind.
+struct DeviceWindows {
+    int4* modules = nullptr;  // unused slots -1
+    int* count = nullptr;
+    double* start_x = nullptr;
+    double* bottom = nullptr;
+    double* spacing = nullptr;
+    int* net_start = nullptr;
+    int* nets = nullptr;
+    int* own = nullptr;       // per entry of nets: its first own pin among the sorted pins
+    uint8_t* kind = nullptr;
+    int* owner = nullptr;              // per module: its window, or -1
+    int8_t* moved_orientation = nullptr;  // per module: the orientation it takes when its window is reordered
+};
+
+__global__ void __launch_bounds__(kThreads) fillWindowsKernel(int count, const int* cell, const unsigned* row,
+                                                              const int* first, const int* begins, const int* id,
+                                                              const double2* center, const double2* size,
+                                                              const int8_t* turn, DeviceRows rows, DeviceWindows out,
+                                                              PassCounts* counts) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) counts->windows = id[count];
+    if (i >= count || begins[i] == 0) return;
+    const int w = id[i];
+    const unsigned r = row[i];
+    int module[kWindow] = {-1, -1, -1, -1};
+    int n = 0;
+#pragma unroll
+    for (int k = 0; k < kWindow; ++k) {
+        if (n == k && i + k < count && sameSegment(first, row, i, i + k)) {
+            module[k] = cell[i + k];
+            ++n;
+        }
+    }
+    out.modules[w] = make_int4(module[0], module[1], module[2], module[3]);
+    out.count[w] = n;
+    out.start_x[w] = lowerLeft(center[module[0]].x, size[module[0]].x);
+    out.bottom[w] = rows.bottom[r];
+    out.spacing[w] = rows.spacing[r];
+    const int turned = rows.turn[r];
+#pragma unroll
+    for (int k = 0; k < kWindow; ++k) {
+        if (module[k] < 0) continue;
+        out.owner[module[k]] = w;
+        out.moved_orientation[module[k]] = turned != kOrientationUnknown ? static_cast<int8_t>(turned) : turn[module[k]];
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) pinWindowsKernel(int pins, const int* pin_module, const int* owner,
+                                                             const PassCounts* counts, unsigned* key) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= pins) return;
+    const int w = owner[pin_module[p]];
+    key[p] = static_cast<unsigned>(w >= 0 ? w : counts->windows);  // behind every window
+}
+
+// head[i] = 1 where a net of a window appears first among the sorted pins; head[pins] = 0.
+__global__ void __launch_bounds__(kThreads) netHeadsKernel(int pins, const unsigned* key, const int* pin,
+                                                           const int* net, const PassCounts* counts, int* head) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > pins) return;
+    head[i] = i < pins && key[i] < static_cast<unsigned>(counts->windows) &&
+                      (i == 0 || key[i - 1] != key[i] || net[pin[i - 1]] != net[pin[i]])
+                  ? 1
+                  : 0;
+}
+
+__global__ void __launch_bounds__(kThreads) windowNetsKernel(int pins, const unsigned* key, const int* pin,
+                                                             const int* net, const int* head, const int* at, const PassCounts* counts,
+                                                             DeviceWindows out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > pins) return;
+    const int windows = counts->windows;
+    if (i < pins && head[i] != 0) {
+        out.nets[at[i]] = net[pin[i]];
+        out.own[at[i]] = i;
+    }
+    // The windows after the previous pin's up to this one's begin here (those between have no pins).
+    const int mine = i < pins ? static_cast<int>(key[i]) : windows;
+    const int before = i > 0 ? static_cast<int>(key[i - 1]) : -1;
+    for (int w = before + 1; w <= mine; ++w) out.net_start[w] = at[i];
+    if (mine == windows && before < windows) out.own[at[i]] = i;  // the end of the last entry
+}
+
+// Each window's kind: none without nets or with one above the degree limit.
+__global__ void __launch_bounds__(kThreads) windowKindsKernel(const int* net_pin_start, unsigned long long maximum_degree,
+                                                              DeviceWindows out, PassCounts* counts) {
+    const int w = blockIdx.x * blockDim.x + threadIdx.x;
+    int four = 0, tail = 0, orders = 0;
+    if (w < counts->windows) {
+        const int first = out.net_start[w];
+        const int last = out.net_start[w + 1];
+        bool takes = last > first;
+        for (int e = first; e < last && takes; ++e) {
+            const int n = out.nets[e];
+            takes = static_cast<unsigned long long>(net_pin_start[n + 1] - net_pin_start[n]) <= maximum_degree;
+        }
+        four = takes && out.count[w] == kWindow ? 1 : 0;
+        tail = takes && four == 0 ? 1 : 0;
+        orders = takes ? factorialOf(out.count[w]) : 0;
+        out.kind[w] = four != 0 ? kFourCells : (tail != 0 ? kTail : kNotEvaluated);
+    }
+    four = __reduce_add_sync(0xffffffffu, four);
+    tail = __reduce_add_sync(0xffffffffu, tail);
+    orders = __reduce_add_sync(0xffffffffu, orders);
+    if ((threadIdx.x & 31) == 0 && orders > 0) {
+        if (four > 0) atomicAdd(&counts->four, four);
+        if (tail > 0) atomicAdd(&counts->tails, tail);
+        atomicAdd(&counts->permutations, static_cast<unsigned long long>(orders));
+    }
+}
+
+// Moves the cells of the accepted windows of a kind (four-cell: decided, tails: an order taken).
+__global__ void __launch_bounds__(kThreads) applyWindowsKernel(int windows, WindowKind kind, const uint8_t* decided,
+                                                               const int8_t* order, DeviceWindows w,
+                                                               const double2* moved_center, double2* center,
+                                                               int8_t* turn, PassCounts* counts) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool accepted = k < windows && w.kind[k] == kind && (kind == kTail ? order[k] >= 0 : decided[k] != 0);
+    if (accepted) {
+        const int4 m4 = w.modules[k];
+        const int module[kWindow] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+        for (int i = 0; i < kWindow; ++i) {
+            if (module[i] < 0) continue;
+            center[module[i]] = moved_center[module[i]];
+            turn[module[i]] = w.moved_orientation[module[i]];
+        }
+    }
+    const unsigned all = __ballot_sync(0xffffffffu, accepted ? 1 : 0);
+    if ((threadIdx.x & 31) == 0 && all != 0u) {
+        atomicAdd(&counts->accepted, static_cast<unsigned long long>(__popc(all)));
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) resultKernel(int count, const double2* center, const int8_t* turn, double* x,
+                                                         double* y, int* orientation) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= count) return;
+    const double2 c = center[m];
+    x[m] = c.x;
+    y[m] = c.y;
+    orientation[m] = turn[m];
+}
+
+struct LargerOf {
+    __device__ __forceinline__ int operator()(int a, int b) const { return a < b ? b : a; }
+};
+
+// What the passes on the device hold: the arrays below (176 bytes per module, 88 per pin, 120 per
+// net, 32 per row) and the sorts' workspace (12 bytes per module or 8 per pin), with slack.
+uint64_t devicePassBytes(const mpgp_design& d) {
+    const uint64_t modules = static_cast<uint64_t>(d.module_count);
+    const uint64_t pins = static_cast<uint64_t>(d.pin_count);
+    const uint64_t nets = static_cast<uint64_t>(d.net_count);
+    return modules * 240 + pins * 112 + nets * 128 + static_cast<uint64_t>(d.row_count) * 32 + (uint64_t{8} << 20);
+}
+
+// The passes' arrays out of one block.
+class PassMemory {
+public:
+    PassMemory(cudaStream_t stream, uint64_t bytes)
+        : scratch_(stream, [bytes] { return bytes; }), block_(scratch_.array<unsigned char>(bytes)), bytes_(bytes) {}
+    template <typename T>
+    T* array(std::size_t count) {
+        const std::size_t at = (used_ + 255) / 256 * 256;
+        require(at + count * sizeof(T) <= bytes_, "The detailed-placement arrays exceed their block.");
+        used_ = at + count * sizeof(T);
+        return reinterpret_cast<T*>(block_ + at);
+    }
+
+private:
+    Scratch scratch_;
+    unsigned char* block_;
+    std::size_t bytes_;
+    std::size_t used_ = 0;
+};
+
+// Every pass on the device.  False, with nothing written, where the host has to look: an entry
+// that validation refuses, rows of which cells share an x (the host's sort decides their
+// order), rounds that do not end in kMaxRounds, or no memory for the arrays.
+bool placeOnDevice(const mpgp_design& d, const int32_t* row_orientation, const mpgp_detailed_options& options,
+                   double* module_x, double* module_y, int32_t* module_orientation, mpgp_detailed_result& result) {
+    for (int32_t r = 0; r < d.row_count; ++r) {
+        const bool good = std::isfinite(d.row_bottom[r]) && std::isfinite(d.row_height[r]) &&
+                          std::isfinite(d.row_site_spacing[r]) && std::isfinite(d.row_x_start[r]) &&
+                          d.row_site_count[r] >= 0 &&
+                          (row_orientation == nullptr ||
+                           (row_orientation[r] >= 0 && row_orientation[r] <= kOrientationUnknown));
+        if (!good) return false;
+    }
+    const auto started = std::chrono::steady_clock::now();
+    const int modules = d.module_count;
+    const int pins = static_cast<int>(d.pin_count);
+    const int nets = d.net_count;
+    const std::size_t rows = static_cast<std::size_t>(d.row_count);
+    Stream owned_stream;
+    const cudaStream_t stream = owned_stream.get();
+    Stream side;  // the HPWL terms' way to the host
+    Event terms;
+    std::unique_ptr<PassMemory> memory;
+    try {
+        memory = std::make_unique<PassMemory>(stream, devicePassBytes(d));
+    } catch (const Error&) {
+        cudaGetLastError();
+        return false;  // the host's path says what is missing
+    }
+    PassMemory& scratch = *memory;
+    HostTransfer transfer(stream, static_cast<std::size_t>(std::max(modules, pins)) * sizeof(double));
+    const HostTransfer::Call call(&transfer);
+    const auto put = [&](const auto* host, std::size_t count) {
+        using T = std::remove_const_t<std::remove_pointer_t<decltype(host)>>;
+        T* device = scratch.array<T>(count);
+        transfer.send(host, device, count * sizeof(T));
+        return device;
+    };
+
+    // The rows in bottom order (buildWindows).
+    std::vector<std::size_t> sorted_rows(rows);
+    std::iota(sorted_rows.begin(), sorted_rows.end(), 0U);
+    std::sort(sorted_rows.begin(), sorted_rows.end(),
+              [&](std::size_t a, std::size_t b) { return d.row_bottom[a] < d.row_bottom[b]; });
+    std::vector<double> centres(rows);
+    std::vector<int> indices(rows), turns(rows);
+    for (std::size_t k = 0; k < rows; ++k) {
+        const std::size_t r = sorted_rows[k];
+        centres[k] = d.row_bottom[r] + d.row_height[r] * 0.5;
+        indices[k] = static_cast<int>(r);
+        turns[k] = row_orientation != nullptr ? row_orientation[k] : 0;
+    }
+    DeviceRows row_data;
+    row_data.count = d.row_count;
+    row_data.centre = put(centres.data(), rows);
+    row_data.index = put(indices.data(), rows);
+    row_data.bottom = put(d.row_bottom, rows);
+    row_data.spacing = put(d.row_site_spacing, rows);
+    row_data.turn = put(turns.data(), rows);
+
+    const std::size_t m_count = static_cast<std::size_t>(modules);
+    const std::size_t p_count = static_cast<std::size_t>(pins);
+    const std::size_t n_count = static_cast<std::size_t>(nets);
+    const std::size_t w_count = m_count / 2 + 1;  // every window holds two cells at least
+    static_assert(sizeof(long long) == sizeof(int64_t), "net offsets are 64-bit");
+    RawDesign raw;
+    raw.modules = modules;
+    raw.nets = nets;
+    raw.pins = pins;
+    double* x = put(d.module_x, m_count);
+    double* y = put(d.module_y, m_count);
+    raw.x = x;
+    raw.y = y;
+    raw.width = put(d.module_width, m_count);
+    raw.height = put(d.module_height, m_count);
+    raw.flags = put(d.module_flags, m_count);
+    if (d.module_orientation != nullptr) raw.orientation = put(d.module_orientation, m_count);
+    raw.net_start = put(reinterpret_cast<const long long*>(d.net_pin_start), n_count + 1);
+    raw.net_weight = put(d.net_weight, n_count);
+    raw.pin_module = put(d.pin_module, p_count);
+    raw.offset_x = put(d.pin_offset_x, p_count);
+    raw.offset_y = put(d.pin_offset_y, p_count);
+    const int* pin_module = raw.pin_module;
+    const double* net_weight = raw.net_weight;
+    int* changed = scratch.array<int>(kMaxRounds + kRoundsPerCheck + 1);
+    PassCounts* counts = scratch.array<PassCounts>(1);
+    const PinnedBlock readback(sizeof(PassCounts) + sizeof(int), "detailed-placement counters");
+    PassCounts* const host_counts = reinterpret_cast<PassCounts*>(readback.data());
+    int* const host_changed = reinterpret_cast<int*>(readback.data() + sizeof(PassCounts));
+    // The checks, before any kernel follows an index.
+    checkCuda(cudaMemsetAsync(changed, 0, sizeof(int), stream), "check the design");
+    checkDesignKernel<<<threadBlocks(std::max({m_count, n_count, p_count})), kThreads, 0, stream>>>(raw, changed);
+    checkCuda(cudaMemcpyAsync(host_changed, changed, sizeof(int), cudaMemcpyDeviceToHost, stream), "check the design");
+    checkCuda(cudaStreamSynchronize(stream), "check the design");
+    transfer.settled();
+    if (*host_changed != 0) return false;
+
+    double2* center = scratch.array<double2>(m_count);
+    double2* moved_center = scratch.array<double2>(m_count);
+    double2* size = scratch.array<double2>(m_count);
+    int8_t* turn = scratch.array<int8_t>(m_count);
+    uint8_t* is_standard = scratch.array<uint8_t>(m_count);
+    detailedModulesKernel<<<threadBlocks(m_count), kThreads, 0, stream>>>(raw, nominalRowHeight(d), center, size, turn,
+                                                                          is_standard);
+    checkCuda(cudaGetLastError(), "detailed placement on the device");
+    int* net_pin_start = scratch.array<int>(n_count + 1);
+    int* pin_net = scratch.array<int>(p_count);
+    int* pin_index = scratch.array<int>(p_count);
+    detailedNetsKernel<<<threadBlocks(8 * (n_count + 1)), kThreads, 0, stream>>>(nets, raw.net_start, net_pin_start, pin_net,
+                                                                                pin_index);
+    double2* raw_offset = scratch.array<double2>(p_count);
+    double2* pin_offset = scratch.array<double2>(p_count);
+    rawOffsetsKernel<<<threadBlocks(p_count), kThreads, 0, stream>>>(pins, raw.offset_x, raw.offset_y, raw_offset);
+    double* term_before = scratch.array<double>(n_count);
+    double* term_after = scratch.array<double>(n_count);
+    const auto turnOffsets = [&] {
+        turnedOffsetsKernel<<<threadBlocks(p_count), kThreads, 0, stream>>>(pins, raw_offset, pin_module, turn, pin_offset);
+    };
+    const auto netTerms = [&](double* term) {
+        netTermsKernel<<<threadBlocks(8 * n_count), kThreads, 0, stream>>>(nets, net_pin_start, pin_module, pin_offset,
+                                                                           center, net_weight, term);
+        checkCuda(cudaGetLastError(), "net terms");
+    };
+    turnOffsets();
+    netTerms(term_before);
+    checkCuda(cudaEventRecord(terms.get(), stream), "net terms");
+    checkCuda(cudaStreamWaitEvent(side.get(), terms.get(), 0), "net terms");
+
+    double* x_key = scratch.array<double>(m_count);
+    double* x_sorted = scratch.array<double>(m_count);
+    int* cell = scratch.array<int>(m_count);
+    int* cell_by_x = scratch.array<int>(m_count);
+    int* row = scratch.array<int>(m_count);
+    unsigned* row_key = scratch.array<unsigned>(m_count);
+    unsigned* row_sorted = scratch.array<unsigned>(m_count);
+    int* first = scratch.array<int>(m_count);
+    int* segment = scratch.array<int>(m_count);
+    int* begins = scratch.array<int>(m_count + 1);
+    int* window_id = scratch.array<int>(m_count + 1);
+    unsigned* pin_key = scratch.array<unsigned>(p_count);
+    unsigned* pin_key_sorted = scratch.array<unsigned>(p_count);
+    int* pin_sorted = scratch.array<int>(p_count);
+    int* head = scratch.array<int>(p_count + 1);
+    int* head_at = scratch.array<int>(p_count + 1);
+    DeviceWindows windows;
+    windows.modules = scratch.array<int4>(w_count);
+    windows.count = scratch.array<int>(w_count);
+    windows.start_x = scratch.array<double>(w_count);
+    windows.bottom = scratch.array<double>(w_count);
+    windows.spacing = scratch.array<double>(w_count);
+    windows.net_start = scratch.array<int>(w_count + 1);
+    windows.nets = scratch.array<int>(p_count);
+    windows.own = scratch.array<int>(p_count + 1);
+    windows.kind = scratch.array<uint8_t>(w_count);
+    windows.owner = scratch.array<int>(m_count);
+    windows.moved_orientation = scratch.array<int8_t>(m_count);
+    int* best_order = scratch.array<int>(w_count);
+    uint8_t* decided[2] = {scratch.array<uint8_t>(w_count), scratch.array<uint8_t>(w_count)};
+    int8_t* taken[2] = {scratch.array<int8_t>(w_count), scratch.array<int8_t>(w_count)};
+    NetExtremes* extremes = scratch.array<NetExtremes>(n_count);
+    int* stamp = scratch.array<int>(n_count);
+
+    const auto bitsFor = [](uint64_t largest) {
+        int bits = 1;
+        while ((largest >> bits) != 0) ++bits;
+        return bits;
+    };
+    const int row_bits = bitsFor(rows);
+    const int window_bits = bitsFor(w_count);
+    std::size_t workspace_bytes = 0;
+    const auto grow = [&](cudaError_t status, std::size_t bytes) {
+        checkCuda(status, "size a sort's workspace");
+        workspace_bytes = std::max(workspace_bytes, bytes);
+    };
+    std::size_t bytes = 0;
+    grow(cub::DeviceRadixSort::SortPairs(nullptr, bytes, x_key, x_sorted, cell, cell_by_x, modules, 0, 64, stream), bytes);
+    grow(cub::DeviceRadixSort::SortPairs(nullptr, bytes, row_key, row_sorted, cell_by_x, cell, modules, 0, row_bits, stream),
+         bytes);
+    grow(cub::DeviceRadixSort::SortPairs(nullptr, bytes, pin_key, pin_key_sorted, pin_index, pin_sorted, pins, 0, window_bits,
+                                         stream),
+         bytes);
+    grow(cub::DeviceScan::InclusiveScan(nullptr, bytes, first, segment, LargerOf{}, modules, stream), bytes);
+    grow(cub::DeviceScan::ExclusiveSum(nullptr, bytes, head, head_at, pins + 1, stream), bytes);
+    grow(cub::DeviceScan::ExclusiveSum(nullptr, bytes, begins, window_id, modules + 1, stream), bytes);
+    void* workspace = scratch.array<unsigned char>(workspace_bytes);
+    result.cuda_reserved_memory_bytes = devicePassBytes(d);
+    const auto readCounts = [&] {
+        checkCuda(cudaMemcpyAsync(host_counts, counts, sizeof(PassCounts), cudaMemcpyDeviceToHost, stream), "pass counts");
+        checkCuda(cudaStreamSynchronize(stream), "detailed-placement pass");
+    };
+    // Rounds until one changes nothing; launch(rounds, in) launches round `rounds.round` from
+    // decisions `in` (0 or 1) into the other.
+    const auto settle = [&](const auto& launch) {
+        checkCuda(cudaMemsetAsync(stamp, 0, n_count * sizeof(int), stream), "clear the rounds");
+        checkCuda(cudaMemsetAsync(changed, 0, (kMaxRounds + kRoundsPerCheck + 1) * sizeof(int), stream), "clear the rounds");
+        for (int round = 1; round <= kMaxRounds; round += kRoundsPerCheck) {
+            for (int k = round; k < round + kRoundsPerCheck; ++k) launch(Rounds{k, stamp, changed}, (k - 1) & 1);
+            checkCuda(cudaGetLastError(), "re-decide the windows");
+            checkCuda(cudaMemcpyAsync(host_changed, changed + round + kRoundsPerCheck - 1, sizeof(int),
+                                      cudaMemcpyDeviceToHost, stream),
+                      "read the rounds");
+            checkCuda(cudaStreamSynchronize(stream), "re-decide the windows");
+            if (*host_changed == 0) return true;
+        }
+        return false;
+    };
+
+    // calculateHpwl (Metrics.cpp:128-147): the nets' terms in net order.
+    const auto sum = [&](const double* term, cudaStream_t on) {
+        double total = 0.0;
+        readDown(term, n_count,
+                 [&](const double* v, std::size_t count) {
+                     for (std::size_t k = 0; k < count; ++k) total += v[k];
+                 },
+                 on);
+        return total;
+    };
+    double hpwl_before = 0.0;
+    uint64_t evaluated = 0, permutations = 0, accepted = 0;
+    for (int pass = 0; pass < options.passes; ++pass) {
+        const int phase = (pass % 2) * (kWindow / 2);
+        checkCuda(cudaMemsetAsync(counts, 0, sizeof(PassCounts), stream), "clear the counts");
+        checkCuda(cudaMemsetAsync(windows.owner, 0xFF, m_count * sizeof(int), stream), "clear the owners");
+        const int module_blocks = threadBlocks(m_count + 1);
+        const int pin_blocks = threadBlocks(p_count + 1);
+        cellRowsKernel<<<module_blocks, kThreads, 0, stream>>>(modules, is_standard, center, size, row_data, x_key, cell, row);
+        bytes = workspace_bytes;
+        checkCuda(cub::DeviceRadixSort::SortPairs(workspace, bytes, x_key, x_sorted, cell, cell_by_x, modules, 0, 64, stream),
+                  "sort the cells by x");
+        rowKeysKernel<<<module_blocks, kThreads, 0, stream>>>(modules, cell_by_x, row, row_key);
+        bytes = workspace_bytes;
+        checkCuda(cub::DeviceRadixSort::SortPairs(workspace, bytes, row_key, row_sorted, cell_by_x, cell, modules, 0, row_bits,
+                                                  stream),
+                  "sort the cells by row");
+        segmentsKernel<<<module_blocks, kThreads, 0, stream>>>(modules, cell, row_sorted, center, size, row_data, first, counts);
+        bytes = workspace_bytes;
+        checkCuda(cub::DeviceScan::InclusiveScan(workspace, bytes, first, segment, LargerOf{}, modules, stream), "segments");
+        windowBeginsKernel<<<module_blocks, kThreads, 0, stream>>>(modules, phase, row_data.count, segment, row_sorted, begins);
+        bytes = workspace_bytes;
+        checkCuda(cub::DeviceScan::ExclusiveSum(workspace, bytes, begins, window_id, modules + 1, stream), "windows");
+        fillWindowsKernel<<<module_blocks, kThreads, 0, stream>>>(modules, cell, row_sorted, segment, begins, window_id, center,
+                                                                  size, turn, row_data, windows, counts);
+        pinWindowsKernel<<<pin_blocks, kThreads, 0, stream>>>(pins, pin_module, windows.owner, counts, pin_key);
+        bytes = workspace_bytes;
+        checkCuda(cub::DeviceRadixSort::SortPairs(workspace, bytes, pin_key, pin_key_sorted, pin_index, pin_sorted, pins, 0,
+                                                  window_bits, stream),
+                  "sort the pins by window");
+        netHeadsKernel<<<pin_blocks, kThreads, 0, stream>>>(pins, pin_key_sorted, pin_sorted, pin_net, counts, head);
+        bytes = workspace_bytes;
+        checkCuda(cub::DeviceScan::ExclusiveSum(workspace, bytes, head, head_at, pins + 1, stream), "window nets");
+        windowNetsKernel<<<pin_blocks, kThreads, 0, stream>>>(pins, pin_key_sorted, pin_sorted, pin_net, head, head_at, counts,
+                                                              windows);
+        windowKindsKernel<<<threadBlocks(w_count), kThreads, 0, stream>>>(net_pin_start, options.maximum_net_degree, windows,
+                                                                          counts);
+        checkCuda(cudaGetLastError(), "build the windows");
+        if (pass == 0) hpwl_before = sum(term_before, side.get());  // while the device builds the windows
+        readCounts();
+        if (host_counts->ties != 0) return false;
+        const int total = host_counts->windows;
+        evaluated += static_cast<uint64_t>(total);
+        permutations += host_counts->permutations;
+        const unsigned warps = static_cast<unsigned>((total + kWindowsPerBlock - 1) / kWindowsPerBlock);
+        if (host_counts->four > 0) {
+            if (pass > 0) turnOffsets();
+            const WindowArrays arrays{windows.modules, windows.start_x, windows.bottom,
+                                      windows.spacing, windows.net_start, windows.nets};
+            netExtremesKernel<<<threadBlocks(8 * n_count), kThreads, 0, stream>>>(nets, net_pin_start, pin_module, pin_offset,
+                                                                                  center, windows.owner, extremes);
+            windowOrdersKernel<true><<<warps, 32 * kWindowsPerBlock, 0, stream>>>(
+                center, size, pin_module, pin_offset, net_pin_start, net_weight, arrays, total, windows.kind,
+                options.improvement_epsilon, best_order, decided[0], moved_center,
+                OwnPins{windows.own, pin_sorted, extremes});
+            const bool settled = settle([&](const Rounds& rounds, int in) {
+                speculativeValuesKernel<<<warps, 32 * kWindowsPerBlock, 0, stream>>>(
+                    center, moved_center, windows.owner, windows.moved_orientation, raw_offset, pin_offset, pin_module,
+                    net_pin_start, net_weight, arrays, total, best_order, options.improvement_epsilon, decided[in],
+                    decided[in ^ 1], nullptr, nullptr, rounds);
+            });
+            if (!settled) return false;
+            applyWindowsKernel<<<threadBlocks(static_cast<std::size_t>(total)), kThreads, 0, stream>>>(
+                total, kFourCells, decided[0], nullptr, windows, moved_center, center, turn, counts);
+        }
+        if (host_counts->tails > 0) {
+            const TailArrays tail{windows.modules, windows.count, windows.start_x, windows.bottom,
+                                  windows.spacing, windows.net_start, windows.nets};
+            checkCuda(cudaMemsetAsync(taken[0], 0xFF, static_cast<std::size_t>(total), stream), "tail orders");
+            const bool settled = settle([&](const Rounds& rounds, int in) {
+                if (rounds.round > 1) {
+                    tailPlacementKernel<<<threadBlocks(static_cast<std::size_t>(total)), kThreads, 0, stream>>>(
+                        tail, total, size, taken[in], moved_center, rounds);
+                }
+                tailOrdersKernel<<<warps, 32 * kWindowsPerBlock, 0, stream>>>(
+                    center, turn, moved_center, windows.owner, 0, windows.moved_orientation, raw_offset, size, pin_module,
+                    net_pin_start, net_weight, tail, total, windows.kind, options.improvement_epsilon, taken[in],
+                    taken[in ^ 1], rounds);
+            });
+            if (!settled) return false;
+            applyWindowsKernel<<<threadBlocks(static_cast<std::size_t>(total)), kThreads, 0, stream>>>(
+                total, kTail, nullptr, taken[0], windows, moved_center, center, turn, counts);
+        }
+        checkCuda(cudaGetLastError(), "detailed-placement pass");
+        if (pass + 1 == options.passes) break;
+        readCounts();
+        accepted += host_counts->accepted;
+    }
+    turnOffsets();
+    netTerms(term_after);
+    int* orientation_out = row;  // the arrays of the cell sort are free again
+    resultKernel<<<threadBlocks(m_count), kThreads, 0, stream>>>(modules, center, turn, x, y, orientation_out);
+    checkCuda(cudaGetLastError(), "detailed-placement result");
+    readCounts();
+    accepted += host_counts->accepted;
+    std::vector<HostTransfer::Piece> pieces{{x, module_x, m_count * sizeof(double)}, {y, module_y, m_count * sizeof(double)}};
+    if (module_orientation != nullptr) pieces.push_back({orientation_out, module_orientation, m_count * sizeof(int32_t)});
+    transfer.startDownload(pieces);
+    result.hpwl_before = hpwl_before;
+    result.hpwl_after = sum(term_after, side.get());
+    transfer.finishDownload();
+    result.cuda_device_used = options.cuda_device;
+    result.evaluated_windows = evaluated;
+    result.evaluated_permutations = permutations;
+    result.accepted_operations = accepted;
+    result.completed_passes = options.passes;
+    result.elapsed_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - started).count();
+    return true;
+}
+
+// The bytes the host's lists reserve on the device (detailedPlace).
+uint64_t hostListBytes(const mpgp_design& d) {
+    const auto of = [](uint64_t count, uint64_t size) { return std::max<uint64_t>(count, 1) * size; };
+    const uint64_t modules = static_cast<uint64_t>(d.module_count);
+    const uint64_t pins = static_cast<uint64_t>(d.pin_count);
+    const uint64_t nets = static_cast<uint64_t>(d.net_count);
+    const uint64_t windows = modules / kWindow + 1;
+    const uint64_t tails = modules / 2 + 1;
+    return of(modules, 16 + 16 + 4 + 1 + 16 + 1) + of(pins, 16 + 16 + 4 + 4) + of(nets + 1, 4) + of(nets, 8) +
+           windows * (16 + 3 * 8 + 4 + 2 * 8 + 2) + (windows + 1) * 4 + tails * (16 + 4 + 3 * 8 + 2) + (tails + 1) * 4;
+}
+
 }  // namespace
 
 bool detailedPlace(const mpgp_design& d, const int32_t* row_orientation, const mpgp_detailed_options& options,
@@ -781,19 +1917,23 @@ bool detailedPlace(const mpgp_design& d, const int32_t* row_orientation, const m
         reason = "CUDA detailed-placement options are outside their valid range.";
         return false;
     }
-    validateDesign(d);
-    for (int32_t m = 0; d.module_orientation != nullptr && m < d.module_count; ++m) {
-        require(d.module_orientation[m] >= 0 && d.module_orientation[m] <= kOrientationUnknown,
-                "Module orientations must be Orientation values (0-8).");
-    }
-    for (int32_t r = 0; row_orientation != nullptr && r < d.row_count; ++r) {
-        require(row_orientation[r] >= 0 && row_orientation[r] <= kOrientationUnknown,
-                "Row orientations must be Orientation values (0-8).");
-    }
+    validateDesignShape(d);
+    const auto validate = [&] {
+        validateDesign(d);
+        for (int32_t m = 0; d.module_orientation != nullptr && m < d.module_count; ++m) {
+            require(d.module_orientation[m] >= 0 && d.module_orientation[m] <= kOrientationUnknown,
+                    "Module orientations must be Orientation values (0-8).");
+        }
+        for (int32_t r = 0; row_orientation != nullptr && r < d.row_count; ++r) {
+            require(row_orientation[r] >= 0 && row_orientation[r] <= kOrientationUnknown,
+                    "Row orientations must be Orientation values (0-8).");
+        }
+    };
     int device_count = 0;
     if (cudaGetDeviceCount(&device_count) != cudaSuccess || options.cuda_device < 0 ||
         options.cuda_device >= device_count) {
         cudaGetLastError();
+        validate();
         reason = "Requested CUDA device is unavailable on this host.";
         return false;
     }
@@ -801,6 +1941,7 @@ bool detailedPlace(const mpgp_design& d, const int32_t* row_orientation, const m
     cudaGetDevice(&previous_device);
     if (cudaSetDevice(options.cuda_device) != cudaSuccess) {
         cudaGetLastError();
+        validate();
         reason = "Unable to select the requested CUDA device.";
         return false;
     }
@@ -808,24 +1949,36 @@ bool detailedPlace(const mpgp_design& d, const int32_t* row_orientation, const m
         int device;
         ~RestoreDevice() { cudaSetDevice(device); }
     } restore{previous_device};
-    cudaDeviceProp properties{};
-    if (cudaGetDeviceProperties(&properties, options.cuda_device) != cudaSuccess || properties.major < 6) {
+    int major = 0;
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, options.cuda_device) != cudaSuccess || major < 6) {
+        validate();
         reason = "Requested CUDA device lacks required double-precision support.";
         return false;
     }
+    // The device takes every design it can (the rules above placeOnDevice) whose arrays, and
+    // those of the host's lists, the caller's budget allows.  Two passes, host's lists against
+    // device, a B200 with 16 host CPUs: 50 cells 1.9 / 0.8 ms, 500 2.2 / 1.0, 2,000 3.0 / 1.1, 8,000
+    // 5.3 / 1.4, 30,000 12.9 / 2.0, 210,000 61 / 5.3.
+    result = mpgp_detailed_result{};
+    const uint64_t budget = options.maximum_cuda_memory_bytes;
+    if (d.module_count > 0 && d.pin_count > 0 && d.net_count > 0 && d.row_count > 0 && hostListBytes(d) <= budget &&
+        devicePassBytes(d) <= budget &&
+        placeOnDevice(d, row_orientation, options, module_x, module_y, module_orientation, result)) {
+        return true;
+    }
+    result = mpgp_detailed_result{};
+    validate();
     std::size_t free_bytes = 0;
     std::size_t total_bytes = 0;
     checkCuda(cudaMemGetInfo(&free_bytes, &total_bytes), "cudaMemGetInfo");
-    const uint64_t limit = std::min<uint64_t>(options.maximum_cuda_memory_bytes, free_bytes);
+    const uint64_t limit = std::min<uint64_t>(budget, free_bytes);
 
-    const DerivedDesign derived = deriveDesign(d);
+    const DerivedDesign derived = deriveDesign(d, false);
     std::vector<uint8_t> standard(static_cast<std::size_t>(d.module_count));
     for (int32_t m = 0; m < d.module_count; ++m) standard[m] = derived.is_fixed[m] == 0 && derived.is_macro[m] == 0;
     const auto rowOrientation = [&](int r) { return row_orientation != nullptr ? row_orientation[r] : 0; };
-
     const Workers workers = Workers::all(16);
     Placement s(d);
-    result = mpgp_detailed_result{};
     result.hpwl_before = s.hpwl(workers);
     result.cuda_device_used = options.cuda_device;
     const auto started = std::chrono::steady_clock::now();
@@ -1018,9 +2171,10 @@ bool detailedPlace(const mpgp_design& d, const int32_t* row_orientation, const m
                                       window_spacing.get(), window_net_start.get(), window_nets.get()};
             const int n = static_cast<int>(count);
             const unsigned blocks = static_cast<unsigned>((count + kWindowsPerBlock - 1) / kWindowsPerBlock);
-            windowOrdersKernel<<<blocks, 32 * kWindowsPerBlock, 0, stream.get()>>>(
+            windowOrdersKernel<false><<<blocks, 32 * kWindowsPerBlock, 0, stream.get()>>>(
                 center.get(), size.get(), pin_module.get(), pin_offset.get(), net_pin_start.get(), net_weight.get(),
-                arrays, n, options.improvement_epsilon, best_order.get(), decided[0].get(), moved_center.get());
+                arrays, n, nullptr, options.improvement_epsilon, best_order.get(), decided[0].get(), moved_center.get(),
+                OwnPins{});
             checkCuda(cudaGetLastError(), "windowOrdersKernel launch");
             // Each iteration re-decides every window on the previous iteration's
             // decisions; the last one's input is the assumption its values rest on.
@@ -1030,7 +2184,7 @@ bool detailedPlace(const mpgp_design& d, const int32_t* row_orientation, const m
                     center.get(), moved_center.get(), owner.get(), moved_orientation.get(), raw_offset.get(),
                     pin_offset.get(), pin_module.get(), net_pin_start.get(), net_weight.get(), arrays, n,
                     best_order.get(), options.improvement_epsilon, decided[in].get(), decided[in ^ 1].get(),
-                    value_before.get(), value_after.get());
+                    value_before.get(), value_after.get(), Rounds{});
                 checkCuda(cudaGetLastError(), "speculativeValuesKernel launch");
             }
             best_order.download(best, stream.get());
@@ -1109,14 +2263,14 @@ bool detailedPlace(const mpgp_design& d, const int32_t* row_orientation, const m
             for (int iteration = 0; iteration < kSpeculations; ++iteration, in ^= 1) {
                 if (iteration > 0) {
                     tailPlacementKernel<<<blocks, 256, 0, stream.get()>>>(tail, n, size.get(), tail_decided[in].get(),
-                                                                         moved_center.get());
+                                                                         moved_center.get(), Rounds{});
                     checkCuda(cudaGetLastError(), "tailPlacementKernel launch");
                 }
                 tailOrdersKernel<<<warp_blocks, 32 * kWindowsPerBlock, 0, stream.get()>>>(
                     center.get(), orientation_now.get(), moved_center.get(), owner.get(), static_cast<int>(count),
                     moved_orientation.get(), raw_offset.get(), size.get(), pin_module.get(), net_pin_start.get(),
-                    net_weight.get(), tail, n, options.improvement_epsilon, tail_decided[in].get(),
-                    tail_decided[in ^ 1].get());
+                    net_weight.get(), tail, n, nullptr, options.improvement_epsilon, tail_decided[in].get(),
+                    tail_decided[in ^ 1].get(), Rounds{});
                 checkCuda(cudaGetLastError(), "tailOrdersKernel launch");
             }
             tail_decided[in].download(tail_result, stream.get());

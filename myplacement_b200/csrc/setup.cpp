@@ -178,7 +178,7 @@ void defaultOptions(mpgp_options& o) {
     o.maximum_cuda_memory_bytes = 40ULL * 1024ULL * 1024ULL * 1024ULL;
 }
 
-void validateDesign(const mpgp_design& d) {
+void validateDesignShape(const mpgp_design& d) {
     require(d.module_count >= 0 && d.net_count >= 0 && d.pin_count >= 0 && d.row_count >= 0,
             "Design counts must be non-negative.");
     require(d.module_count == 0 || (d.module_width && d.module_height && d.module_x && d.module_y && d.module_flags),
@@ -193,6 +193,10 @@ void validateDesign(const mpgp_design& d) {
             "net_pin_start must begin at 0 and end at pin_count.");
     require(d.pin_count < static_cast<int64_t>(std::numeric_limits<int32_t>::max()),
             "The engine indexes pins with 32-bit integers.");
+}
+
+void validateDesign(const mpgp_design& d) {
+    validateDesignShape(d);
     // The first net, then the first pin, that fails a check fails with that check's message.
     const std::size_t net = firstBad(static_cast<std::size_t>(d.net_count), [&](std::size_t n) {
         return !(d.net_pin_start[n + 1] >= d.net_pin_start[n]) || !finite(d.net_weight[n]);
@@ -259,12 +263,17 @@ void validateOptions(const mpgp_options& o) {
     require(o.maximum_cuda_memory_bytes > 0, "The device memory budget must be non-zero.");
 }
 
+double nominalRowHeight(const mpgp_design& d) {
+    if (d.row_count <= 0) return DerivedDesign{}.nominal_row_height;
+    std::vector<double> heights(d.row_height, d.row_height + d.row_count);
+    std::sort(heights.begin(), heights.end());
+    return heights[heights.size() / 2U];
+}
+
 DerivedDesign deriveDesign(const mpgp_design& d, bool with_pins) {
     DerivedDesign out;
+    out.nominal_row_height = nominalRowHeight(d);
     if (d.row_count > 0) {
-        std::vector<double> heights(d.row_height, d.row_height + d.row_count);
-        std::sort(heights.begin(), heights.end());
-        out.nominal_row_height = heights[heights.size() / 2U];
         const auto rowRect = [&](int r) {
             const double x_end = d.row_x_start[r] + static_cast<double>(d.row_site_count[r]) * d.row_site_spacing[r];
             return R{d.row_x_start[r], d.row_bottom[r], x_end, d.row_bottom[r] + d.row_height[r]};

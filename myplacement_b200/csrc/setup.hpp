@@ -60,9 +60,13 @@ struct DerivedDesign {
 
 // Without `with_pins` the pin counts stay empty.
 DerivedDesign deriveDesign(const mpgp_design& design, bool with_pins = true);
+// The median row height (zero without rows): a standard cell's height.
+double nominalRowHeight(const mpgp_design& design);
 
 // Validates the design arrays (sizes, indices, finiteness).
 void validateDesign(const mpgp_design& design);
+// Its first part: counts, missing arrays and the pin total, without a pass over the arrays.
+void validateDesignShape(const mpgp_design& design);
 
 // validateAdaptiveOptions (AdaptiveGlobalPlacer.cpp:413-454) plus the engine's own limits.
 void validateOptions(const mpgp_options& options);
