@@ -1541,11 +1541,25 @@ uint64_t devicePassBytes(const mpgp_design& d) {
     return modules * 240 + pins * 112 + nets * 128 + static_cast<uint64_t>(d.row_count) * 32 + (uint64_t{8} << 20);
 }
 
-// The passes' arrays out of one block.
+// The passes' arrays out of one block of the device's pool.  The pool keeps up to kKeptBytes
+// of what is free for the next call; a larger design's memory goes back to the device.
+constexpr uint64_t kKeptBytes = uint64_t{1} << 29;
 class PassMemory {
 public:
-    PassMemory(cudaStream_t stream, uint64_t bytes)
-        : scratch_(stream, [bytes] { return bytes; }), block_(scratch_.array<unsigned char>(bytes)), bytes_(bytes) {}
+    PassMemory(cudaStream_t stream, uint64_t bytes) : stream_(stream), bytes_(bytes) {
+        scratch_ = std::make_unique<Scratch>(stream, [bytes] { return bytes; });
+        block_ = scratch_->array<unsigned char>(bytes);
+    }
+    ~PassMemory() {
+        scratch_.reset();
+        int device = 0;
+        if (bytes_ <= kKeptBytes || cudaStreamSynchronize(stream_) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess) {
+            return;
+        }
+        cudaMemPoolTrimTo(devicePool(device), kKeptBytes);
+    }
+    PassMemory(const PassMemory&) = delete;
+    PassMemory& operator=(const PassMemory&) = delete;
     template <typename T>
     T* array(std::size_t count) {
         const std::size_t at = (used_ + 255) / 256 * 256;
@@ -1555,8 +1569,9 @@ public:
     }
 
 private:
-    Scratch scratch_;
-    unsigned char* block_;
+    cudaStream_t stream_;
+    std::unique_ptr<Scratch> scratch_;
+    unsigned char* block_ = nullptr;
     std::size_t bytes_;
     std::size_t used_ = 0;
 };
