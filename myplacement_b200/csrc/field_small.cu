@@ -15,7 +15,7 @@
 //   data A   S -> phi_hat -> T             data B   X^T -> phi_hat^T -> U^T
 //   basis A  Cy -> Dy -> Syw               basis B  Cx -> Dxc -> Sxwt (-> Dxc)
 // The next basis is fetched as soon as the contraction that read the last one is done,
-// behind its epilogue.  Thread 0 issues the TMA loads and the tcgen05.mma (the products
+// behind its epilogue.  One thread issues the TMA loads and the tcgen05.mma (the products
 // of the error-corrected fp16 split, as dct_tc.cu); every K-block has accumulators of
 // its own, so one commit covers a step.  All 16 warps run the epilogues: warp w reads
 // TMEM lanes 32 (w % 4) .. (tile rows) and the (w / 4)-th quarter of the columns.
@@ -56,6 +56,9 @@ constexpr int kSmallThreads = 512;
 constexpr int kSmallWarps = kSmallThreads / 32;
 constexpr int kAPlane = kTileM * kBlockK * 2;   // 16 KB: 128 rows of one K-block
 constexpr int kABlock = kSplit * kAPlane;       // both planes
+// The thread that issues the loads and products: in a warp whose TMEM lanes hold no rows of a
+// grid of at most 64, so that it does so beside the epilogues there.
+constexpr unsigned kIssuer = 64;
 constexpr uint32_t kSecondTask = 128;           // TMEM columns of a step's first task
 constexpr uint32_t kSmallTmem = 256;
 
@@ -69,20 +72,19 @@ struct SmallLayout {
     static constexpr int kBasisA = kDataA + kBlocks * kABlock;
     static constexpr int kDataB = kBasisA + kBlocks * kABlock;
     static constexpr int kBasisB = kDataB + kBlocks * kBBlock;
-    static constexpr int kTail = kBasisB + kBlocks * kBBlock;  // 4 barriers, TMEM address, 2 maxima, warp energies
+    static constexpr int kScale = kBasisB + kBlocks * kBBlock;  // the spectral scale, a column of values per thread
+    static constexpr int kTail = kScale + N / 4 * kSmallThreads * 4;  // 4 barriers, TMEM address, 2 maxima, warp energies
+    static constexpr int kFieldPitch = 2 * N + 1;  // floats per staged field row (odd: no bank conflicts)
     static constexpr int kBytes = kTail + 4 * 8 + 16 + kSmallWarps * 8 + 1024 /* alignment slack */;
 };
 static_assert(SmallLayout<32>::kBytes <= 227 * 1024 && SmallLayout<64>::kBytes <= 227 * 1024, "one CTA's shared memory");
+static_assert(SmallLayout<64>::kFieldPitch * 4 * 64 <= kABlock + SmallLayout<64>::kBBlock &&
+                  SmallLayout<32>::kFieldPitch * 4 * 128 <= 2 * kABlock,
+              "the staged field fits where the basis and data operands of the last contraction along y were");
 static_assert(SmallLayout<32>::kBBlock % 1024 == 0 && kABlock % 1024 == 0, "swizzled tiles stay 1024-byte aligned");
 
 __device__ __forceinline__ int planeExponentOf(float bound) {
     return min(120, max(-120, exponentOf(bound) - kPlaneTop));
-}
-
-__device__ __forceinline__ void loadColumns(uint32_t main_at, uint32_t corr_at, uint32_t (&m)[16], uint32_t (&c)[16]) {
-    tmemLoad16(main_at, m);
-    tmemLoad16(corr_at, c);
-    tmemWait(m, c);
 }
 
 __device__ __forceinline__ void loadColumns(uint32_t main_at, uint32_t corr_at, uint32_t (&m)[8], uint32_t (&c)[8]) {
@@ -132,21 +134,29 @@ __device__ __forceinline__ void readResult(uint32_t at, int k_blocks, int shift,
     for (int j = 0; j < kCols; ++j) v[j] = static_cast<float>(acc[j] * unscale);
 }
 
-// Writes row r of a result, columns n0 .. n0 + kCols - 1 of this CTA's N, as column r of
-// a K-major operand (128-byte swizzle: chunk c of operand row n sits at chunk c ^ (n % 8)).
-template <int N, int kCols>
-__device__ __forceinline__ void writeTransposed(unsigned char* operand, int r, int n0, const float (&v)[kCols],
-                                                float inv_scale) {
-    unsigned char* tile = operand + (r >> 6) * (kSplit * N * kBlockK * 2);
-    const int kk = r & 63;
+// The planes of eight values, packed two halves to a word.
+__device__ __forceinline__ void splitEight(const float (&v)[8], float inv_scale, uint4& h, uint4& l) {
+    __half hi[8], lo[8];
 #pragma unroll
-    for (int j = 0; j < kCols; ++j) {
-        __half hi, lo;
-        splitScaled(v[j], inv_scale, hi, lo);
-        const int n = n0 + j;
-        const int offset = n * 128 + (((kk >> 3) ^ (n & 7)) << 4) + (kk & 7) * 2;
-        *reinterpret_cast<__half*>(tile + offset) = hi;
-        *reinterpret_cast<__half*>(tile + N * 128 + offset) = lo;
+    for (int i = 0; i < 8; ++i) splitScaled(v[i], inv_scale, hi[i], lo[i]);
+    h = make_uint4(packHalves(hi[0], hi[1]), packHalves(hi[2], hi[3]), packHalves(hi[4], hi[5]), packHalves(hi[6], hi[7]));
+    l = make_uint4(packHalves(lo[0], lo[1]), packHalves(lo[2], lo[3]), packHalves(lo[4], lo[5]), packHalves(lo[6], lo[7]));
+}
+
+// Writes row r of a result, columns n0 .. n0 + 7 of this CTA's N (n0 a multiple of 8), as
+// column r of a K-major operand (128-byte swizzle: chunk c of operand row n sits at chunk
+// c ^ (n % 8)).
+template <int N>
+__device__ __forceinline__ void writeTransposed(unsigned char* operand, int r, int n0, const uint4& h, const uint4& l) {
+    unsigned char* tile = operand + (r >> 6) * (kSplit * N * kBlockK * 2) + n0 * 128 + (r & 7) * 2;
+    const int chunk = (r & 63) >> 3;
+    const uint32_t hi[4] = {h.x, h.y, h.z, h.w};
+    const uint32_t lo[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        unsigned char* at = tile + j * 128 + ((chunk ^ j) << 4);
+        *reinterpret_cast<unsigned short*>(at) = static_cast<unsigned short>(hi[j / 2] >> (16 * (j & 1)));
+        *reinterpret_cast<unsigned short*>(at + N * 128) = static_cast<unsigned short>(lo[j / 2] >> (16 * (j & 1)));
     }
 }
 
@@ -161,31 +171,19 @@ __device__ __forceinline__ void storeCluster16(uint32_t address, const uint4& v)
                  : "memory");
 }
 
-// Writes row r, columns column .. column + kCols - 1 (of the whole grid) of a result as a
-// K-major A operand in every CTA of the cluster.
-template <int kCols>
-__device__ __forceinline__ void writeRows(uint32_t operand, int rank, int cluster, int r, int column,
-                                          const float (&v)[kCols], float inv_scale) {
-    const uint32_t row = operand + static_cast<uint32_t>((column >> 6) * kABlock + r * 128);
-#pragma unroll
-    for (int j = 0; j < kCols; j += 8) {
-        __half hi[8], lo[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) splitScaled(v[j + i], inv_scale, hi[i], lo[i]);
-        const uint4 h = make_uint4(packHalves(hi[0], hi[1]), packHalves(hi[2], hi[3]), packHalves(hi[4], hi[5]),
-                                   packHalves(hi[6], hi[7]));
-        const uint4 l = make_uint4(packHalves(lo[0], lo[1]), packHalves(lo[2], lo[3]), packHalves(lo[4], lo[5]),
-                                   packHalves(lo[6], lo[7]));
-        const int chunk = ((column + j) & 63) >> 3;
-        const uint32_t at = row + static_cast<uint32_t>((chunk ^ (r & 7)) << 4);
-        storeOwn16(at, h);
-        storeOwn16(at + kAPlane, l);
-        for (int peer = 0; peer < cluster; ++peer) {
-            if (peer == rank) continue;
-            const uint32_t there = clusterAddress(at, static_cast<uint32_t>(peer));
-            storeCluster16(there, h);
-            storeCluster16(there + kAPlane, l);
-        }
+// Writes row r, columns column .. column + 7 (of the whole grid, a multiple of 8) of a result
+// as a K-major A operand in every CTA of the cluster.
+__device__ __forceinline__ void writeRows(uint32_t operand, int rank, int cluster, int r, int column, const uint4& h,
+                                          const uint4& l) {
+    const int chunk = (column & 63) >> 3;
+    const uint32_t at = operand + static_cast<uint32_t>((column >> 6) * kABlock + r * 128 + ((chunk ^ (r & 7)) << 4));
+    storeOwn16(at, h);
+    storeOwn16(at + kAPlane, l);
+    for (int peer = 0; peer < cluster; ++peer) {
+        if (peer == rank) continue;
+        const uint32_t there = clusterAddress(at, static_cast<uint32_t>(peer));
+        storeCluster16(there, h);
+        storeCluster16(there + kAPlane, l);
     }
 }
 
@@ -200,6 +198,8 @@ __device__ __forceinline__ void foldMaximum(float v, uint32_t slot, int cluster)
     }
 }
 
+// A writer's stores before the barrier that hands them to the tensor cores or the copy engine
+// (about 800 cycles: the readers need none of their own).
 __device__ __forceinline__ void asyncFence() { asm volatile("fence.proxy.async;" ::: "memory"); }
 __device__ __forceinline__ void tcBefore() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tcAfter() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -277,7 +277,7 @@ __device__ __forceinline__ void fieldSmall(const FieldSmall& f, int mode, int lo
     const uint32_t here = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(c0);
     clusterArrive();  // this CTA's maxima are cleared; peers wait for it before their first remote store
 
-    // Thread 0's loads and products.  Each barrier completes once per use.
+    // The issuer's loads and products.  Each barrier completes once per use.
     bool ok = true;
     uint32_t parity_a = 0, parity_b = 0, parity_data = 0, parity_products = 0;
     bool pending_a = false, pending_b = false, pending_data = false, pending_products = false;
@@ -314,10 +314,6 @@ __device__ __forceinline__ void fieldSmall(const FieldSmall& f, int mode, int lo
             }
         }
     };
-    const auto commit = [&] {
-        ummaCommit(products);
-        pending_products = true;
-    };
     // Every thread: this step's products are complete.
     const auto awaitProducts = [&] {
         __syncwarp();
@@ -340,237 +336,194 @@ __device__ __forceinline__ void fieldSmall(const FieldSmall& f, int mode, int lo
         tcAfter();
     };
 
-    if (threadIdx.x == 0) {  // fixed tables: before the predecessor has finished
+    if (threadIdx.x == kIssuer) {  // fixed tables: before the predecessor has finished
         fetchA(forward ? &f.map_cy : &f.map_dy);
         fetchB(forward ? &f.map_cx : &f.map_dxc);
+        for (const CUtensorMap* map : {&f.map_s, &f.map_dy, &f.map_dxc, &f.map_syw, &f.map_sxwt}) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+        }
     }
-    float scale[kCols];
+    float* const scale = reinterpret_cast<float*>(smem + L::kScale) + threadIdx.x;  // read back by this thread only
     if (forward) {
 #pragma unroll
         for (int j = 0; j < kCols; ++j) {
-            scale[j] = r < f.ny && column + j < f.nx ? __ldg(f.scale + static_cast<size_t>(r) * f.nx + column + j) : 0.0f;
+            scale[j * kSmallThreads] =
+                r < f.ny && column + j < f.nx ? __ldg(f.scale + static_cast<size_t>(r) * f.nx + column + j) : 0.0f;
         }
     }
     waitForPrior();
     __syncwarp();
     clusterWait();
-    const volatile TcScales* known = f.scales;
-    const int exp_cx = known->exp_basis[0], exp_cy = known->exp_basis[1], exp_dy = known->exp_basis[2];
-    const int exp_dxc = known->exp_basis[3], exp_sxwt = known->exp_basis[4], exp_syw = known->exp_basis[5];
     // The kept phi_hat: its A operand (every K-block), then each CTA's B operand.
     unsigned char* const kept_b = f.phi_store + static_cast<size_t>(kx_blocks) * kABlock +
                                   static_cast<size_t>(rank) * ky_blocks * L::kBBlock;
-    int exp_phi = 0;
-    float top_phi = 0.0f;
-
-    if (forward) {
-        // X = S Cx^T.
-        if (threadIdx.x == 0) {
+    if (threadIdx.x == kIssuer) {
+        if (forward) {
             mbarExpectTx(full_data, static_cast<uint32_t>(kx_blocks * kABlock));
             for (int kb = 0; kb < kx_blocks; ++kb) {
                 tmaLoad3d(data_a + kb * kABlock, &f.map_s, full_data, kb * kBlockK, 0, 0);
             }
-            pending_data = true;
-            landed(full_b, parity_b, pending_b);
-            landed(full_data, parity_data, pending_data);
-            tcAfter();
-            if (ok) {
-                multiply(data_a, basis_b, kx_blocks, tmem);
-                commit();
-            }
-        }
-        const int exp_x = planeExponentOf(__uint_as_float(known->max_source) * f.gain_x);
-        const int exp_row = r < f.ny ? __ldg(f.row_exp + r) : 0;
-        awaitProducts();
-        if (threadIdx.x == 0 && ok && gradient) fetchB(&f.map_dxc);
-        __syncwarp();
-        float top = 0.0f;
-        if (active) {
-            float v[kCols];
-            readResult<N, kCols>(here, kx_blocks, exp_cx + exp_row, v);
-#pragma unroll
-            for (int j = 0; j < kCols; ++j) top = fmaxf(top, fabsf(v[j]));
-            writeTransposed<N, kCols>(smem + L::kDataB, r, c0, v, static_cast<float>(pow2(-exp_x)));
-            foldMaximum(top, smemAddress(tail + 1), cluster);
-            asyncFence();
-        }
-        exchange();
-        const float top_x = __uint_as_float(*reinterpret_cast<volatile uint32_t*>(tail + 1));
-        exp_phi = planeExponentOf(top_x * f.gain_phi);
-
-        // rho_hat = Cy X; phi_hat = rho_hat .* scale (ElectrostaticField.cpp:212-221).
-        if (threadIdx.x == 0) {
-            landed(full_a, parity_a, pending_a);
-            tcAfter();
-            asyncFence();
-            if (ok) {
-                multiply(basis_a, data_b, ky_blocks, tmem);
-                commit();
-            }
-            if (rank == 0) f.scales->max_source = 0u;  // every CTA has read it
-        }
-        awaitProducts();
-        if (threadIdx.x == 0 && ok && gradient) fetchA(&f.map_dy);
-        __syncwarp();
-        double energy = 0.0;
-        top = 0.0f;
-        if (active) {
-            float v[kCols];
-            readResult<N, kCols>(here, ky_blocks, exp_cy + exp_x, v);
-            const double wr = parsevalWeight(r);
-#pragma unroll
-            for (int j = 0; j < kCols; ++j) {
-                const float phi = v[j] * scale[j];
-                if (r < f.ny && column + j < f.nx) {
-                    energy += static_cast<double>(phi) * static_cast<double>(v[j]) * wr * parsevalWeight(column + j);
-                }
-                v[j] = phi;
-                top = fmaxf(top, fabsf(phi));
-            }
-            const float inv_scale = static_cast<float>(pow2(-exp_phi));
-            writeRows<kCols>(data_a, rank, cluster, r, column, v, inv_scale);
-            writeTransposed<N, kCols>(smem + L::kDataB, r, c0, v, inv_scale);
-            foldMaximum(top, smemAddress(tail + 2), cluster);
-            asyncFence();
-        }
-        energy = warpSum(energy);
-        if ((threadIdx.x & 31) == 0) energies[warp] = energy;
-        exchange();
-        top_phi = __uint_as_float(*reinterpret_cast<volatile uint32_t*>(tail + 2));
-        if (threadIdx.x == 0) {
-            // phi_hat is kept for a later launch without the forward transform: each K-block
-            // of the A operand by the CTA that owns its first column, the B operand by its CTA.
-            asyncFence();
-            if (n0 % kBlockK == 0) {
-                bulkToGlobal(f.phi_store + static_cast<size_t>(n0 / kBlockK) * kABlock, data_a + n0 / kBlockK * kABlock,
-                             kABlock);
-            }
-            bulkToGlobal(kept_b, data_b, static_cast<uint32_t>(ky_blocks * L::kBBlock));
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
-        if (threadIdx.x == 32) {
-            double sum = 0.0;
-            for (int w = 0; w < kSmallWarps; ++w) sum += energies[w];
-            if (f.energy_partials != nullptr) f.energy_partials[local_block] = sum;
-            if (rank == 0) {
-                f.scales->max_phi = __float_as_uint(top_phi);
-                f.scales->exp_phi = exp_phi;
-            }
-        }
-    } else {
-        if (threadIdx.x == 0) {
+        } else {
             mbarExpectTx(full_data, static_cast<uint32_t>(kx_blocks * kABlock + ky_blocks * L::kBBlock));
             bulkFromGlobal(data_a, f.phi_store, static_cast<uint32_t>(kx_blocks * kABlock), full_data);
             bulkFromGlobal(data_b, kept_b, static_cast<uint32_t>(ky_blocks * L::kBBlock), full_data);
-            pending_data = true;
-            landed(full_data, parity_data, pending_data);
         }
-        exp_phi = known->exp_phi;
-        top_phi = __uint_as_float(known->max_phi);
+        pending_data = true;
     }
+    const volatile TcScales* known = f.scales;
+    const int exp_cx = known->exp_basis[0], exp_cy = known->exp_basis[1], exp_dy = known->exp_basis[2];
+    const int exp_dxc = known->exp_basis[3], exp_sxwt = known->exp_basis[4], exp_syw = known->exp_basis[5];
+    const int exp_row = forward && r < f.ny ? __ldg(f.row_exp + r) : 0;
+    const int exp_x = forward ? planeExponentOf(__uint_as_float(known->max_source) * f.gain_x) : 0;
+    int exp_phi = forward ? 0 : known->exp_phi;
+    float top_phi = forward ? 0.0f : __uint_as_float(known->max_phi);
+    int exp_t = planeExponentOf(top_phi * f.gain_t);
+    int exp_u = planeExponentOf(top_phi * f.gain_u);
 
-    if (gradient) {
-        // T = Dy phi_hat and U = phi_hat Dxc^T.
-        if (threadIdx.x == 0) {
-            landed(full_a, parity_a, pending_a);
-            landed(full_b, parity_b, pending_b);
+    // The steps of the chain share one loop body: code that runs once is fetched as it runs, and
+    // a step is a few thousand cycles (X 3,500 for the source, 250 after the last product, 2,400
+    // for the epilogue; T and U 5,100 of epilogue).  Unrolled, with a fence on the readers' side
+    // and the loads issued by an epilogue warp, an evaluation took 2 us more (94.8 us against 93
+    // at 64 x 64, 104.4 against 102.5 at 128 x 128).
+    enum { kX = 0, kPhi, kTU, kField, kPotential };
+    const int last = !gradient ? kPhi : (potential ? kPotential : kField);
+#pragma unroll 1
+    for (int step = forward ? kX : kTU; step <= last; ++step) {
+        const int tasks = step == kTU || step == kField ? 2 : 1;
+        // Task 0 of T/U and phi_hat contract along y: A = basis A, B = data B.  The others
+        // contract along x: A = data A, B = basis B.
+        const auto alongX = [&](int task) {
+            return step == kX || step == kPotential || (step == kTU && task == 1) || (step == kField && task == 0);
+        };
+        if (threadIdx.x == kIssuer) {
+            if (pending_data) landed(full_data, parity_data, pending_data);
+            if (step != kX && step != kPotential) landed(full_a, parity_a, pending_a);
+            if (step != kPhi) landed(full_b, parity_b, pending_b);
             tcAfter();
-            asyncFence();
             if (ok) {
-                multiply(basis_a, data_b, ky_blocks, tmem);
-                multiply(data_a, basis_b, kx_blocks, tmem + kSecondTask);
-                commit();
+#pragma unroll 1
+                for (int task = 0; task < tasks; ++task) {
+                    const bool x = alongX(task);
+                    multiply(x ? data_a : basis_a, x ? basis_b : data_b, x ? kx_blocks : ky_blocks,
+                             tmem + static_cast<uint32_t>(task) * kSecondTask);
+                }
+                ummaCommit(products);
+                pending_products = true;
             }
-        }
-        const int exp_t = planeExponentOf(top_phi * f.gain_t);
-        const int exp_u = planeExponentOf(top_phi * f.gain_u);
-        awaitProducts();
-        if (threadIdx.x == 0) {
-            if (ok) {
-                fetchA(&f.map_syw);
-                fetchB(&f.map_sxwt);
-            }
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the kept copies have read the operands
-        }
-        __syncwarp();
-        // The operands may be overwritten once every CTA's products (and copies) have read
-        // them; the results are read from TMEM meanwhile.
-        if (cluster > 1) {
-            clusterArrive();
-        } else {
-            __syncthreads();
-        }
-        float t[kCols], u[kCols];
-        if (active) {
-            readResult<N, kCols>(here, ky_blocks, exp_dy + exp_phi, t);
-            readResult<N, kCols>(here + kSecondTask, kx_blocks, exp_phi + exp_dxc, u);
-        }
-        if (cluster > 1) clusterWait();
-        if (active) {
-            writeRows<kCols>(data_a, rank, cluster, r, column, t, static_cast<float>(pow2(-exp_t)));
-            writeTransposed<N, kCols>(smem + L::kDataB, r, c0, u, static_cast<float>(pow2(-exp_u)));
-            asyncFence();
-        }
-        exchange();
-
-        // Ex = T Sxwt^T and Ey = Syw U.
-        if (threadIdx.x == 0) {
-            landed(full_a, parity_a, pending_a);
-            landed(full_b, parity_b, pending_b);
-            tcAfter();
-            asyncFence();
-            if (ok) {
-                multiply(data_a, basis_b, kx_blocks, tmem);
-                multiply(basis_a, data_b, ky_blocks, tmem + kSecondTask);
-                commit();
-            }
+            if (step == kPhi && rank == 0) f.scales->max_source = 0u;  // every CTA has read it
         }
         awaitProducts();
-        if (threadIdx.x == 0 && ok && potential) fetchB(&f.map_dxc);
-        __syncwarp();
+        if (threadIdx.x == kIssuer) {
+            // The next basis, behind this step's epilogue.
+            if (ok && gradient) {
+                if (step == kPhi || step == kTU) fetchA(step == kPhi ? &f.map_dy : &f.map_syw);
+                if (step == kX || step == kTU) fetchB(step == kX ? &f.map_dxc : &f.map_sxwt);
+                if (step == kField && potential) fetchB(&f.map_dxc);
+            }
+            if (step == kTU) {
+                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the kept copies have read the operands
+            }
+        }
+        // T and U replace operands that every CTA's products (and copies) have to have read.
+        if (step == kTU) exchange();
+
+        float top = 0.0f;
+        double energy = 0.0;
         if (active) {
-            float ex[kCols], ey[kCols];
-            readResult<N, kCols>(here, kx_blocks, exp_t + exp_sxwt, ex);
-            readResult<N, kCols>(here + kSecondTask, ky_blocks, exp_syw + exp_u, ey);
-            if (r < f.ny) {
-                float2* out = f.field + static_cast<size_t>(r) * f.nx + column;
-                if ((f.nx & 1) == 0 && column + kCols <= f.nx) {  // an even width: pairs of bins are 16-byte aligned
+#pragma unroll 1
+            for (int unit = 0; unit < tasks * (kCols / 8); ++unit) {
+                const int task = unit / (kCols / 8);
+                const int j0 = unit % (kCols / 8) * 8;
+                const int shift = step == kX     ? exp_cx + exp_row
+                                  : step == kPhi ? exp_cy + exp_x
+                                  : step == kTU  ? (task == 0 ? exp_dy : exp_dxc) + exp_phi
+                                  : step == kField ? (task == 0 ? exp_t + exp_sxwt : exp_syw + exp_u)
+                                                   : exp_t + exp_dxc;
+                float v[8];
+                readResult<N, 8>(here + static_cast<uint32_t>(task) * kSecondTask + static_cast<uint32_t>(j0),
+                                 alongX(task) ? kx_blocks : ky_blocks, shift, v);
+                if (step == kPhi) {
+                    const double wr = parsevalWeight(r);
 #pragma unroll
-                    for (int j = 0; j < kCols; j += 2) {
-                        *reinterpret_cast<float4*>(out + j) = make_float4(ex[j], ey[j], ex[j + 1], ey[j + 1]);
+                    for (int j = 0; j < 8; ++j) {
+                        const float phi = v[j] * scale[(j0 + j) * kSmallThreads];
+                        if (r < f.ny && column + j0 + j < f.nx) {
+                            energy += static_cast<double>(phi) * static_cast<double>(v[j]) * wr *
+                                      parsevalWeight(column + j0 + j);
+                        }
+                        v[j] = phi;
                     }
-                } else {
+                }
+                if (step <= kTU) {
+                    const int e = step == kX ? exp_x : step == kPhi ? exp_phi : task == 0 ? exp_t : exp_u;
+                    const float inv_scale = static_cast<float>(pow2(-e));
 #pragma unroll
-                    for (int j = 0; j < kCols; ++j) {
-                        if (column + j < f.nx) out[j] = make_float2(ex[j], ey[j]);
+                    for (int j = 0; j < 8; ++j) top = fmaxf(top, fabsf(v[j]));
+                    uint4 h, l;
+                    splitEight(v, inv_scale, h, l);
+                    if (step != kX && task == 0) writeRows(data_a, rank, cluster, r, column + j0, h, l);
+                    if (step != kTU || task == 1) writeTransposed<N>(smem + L::kDataB, r, c0 + j0, h, l);
+                } else if (step == kField) {
+                    float* staged = reinterpret_cast<float*>(smem + L::kBasisA) + r * L::kFieldPitch + 2 * (c0 + j0) + task;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) staged[2 * j] = v[j];
+                } else if (r < f.ny) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        if (column + j0 + j < f.nx) f.potential[static_cast<size_t>(r) * f.nx + column + j0 + j] = v[j];
                     }
                 }
             }
+            if (step <= kPhi) foldMaximum(top, smemAddress(tail + 1 + step), cluster);
+            if (step <= kTU) asyncFence();
         }
-        if (potential) {
-            // phi = T Dxc^T.
+        if (step == kPhi) {
+            energy = warpSum(energy);
+            if ((threadIdx.x & 31) == 0) energies[warp] = energy;
+        }
+        if (step <= kTU) {
+            exchange();
+        } else {
             tcBefore();
             __syncthreads();
-            if (threadIdx.x == 0) {
-                landed(full_b, parity_b, pending_b);
-                tcAfter();
-                if (ok) {
-                    multiply(data_a, basis_b, kx_blocks, tmem);
-                    commit();
+        }
+        if (step == kX) {
+            const float top_x = __uint_as_float(*reinterpret_cast<volatile uint32_t*>(tail + 1));
+            exp_phi = planeExponentOf(top_x * f.gain_phi);
+        } else if (step == kPhi) {
+            top_phi = __uint_as_float(*reinterpret_cast<volatile uint32_t*>(tail + 2));
+            exp_t = planeExponentOf(top_phi * f.gain_t);
+            exp_u = planeExponentOf(top_phi * f.gain_u);
+            if (threadIdx.x == kIssuer) {
+                // phi_hat is kept for a later launch without the forward transform: each K-block
+                // of the A operand by the CTA that owns its first column, the B operand by its CTA.
+                if (n0 % kBlockK == 0) {
+                    bulkToGlobal(f.phi_store + static_cast<size_t>(n0 / kBlockK) * kABlock,
+                                 data_a + n0 / kBlockK * kABlock, kABlock);
+                }
+                bulkToGlobal(kept_b, data_b, static_cast<uint32_t>(ky_blocks * L::kBBlock));
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+            if (threadIdx.x == kIssuer + 32) {
+                double sum = 0.0;
+                for (int w = 0; w < kSmallWarps; ++w) sum += energies[w];
+                if (f.energy_partials != nullptr) f.energy_partials[local_block] = sum;
+                if (rank == 0) {
+                    f.scales->max_phi = __float_as_uint(top_phi);
+                    f.scales->exp_phi = exp_phi;
                 }
             }
-            awaitProducts();
-            if (active) {
-                float v[kCols];
-                readResult<N, kCols>(here, kx_blocks, exp_t + exp_dxc, v);
-#pragma unroll
-                for (int j = 0; j < kCols; ++j) {
-                    if (r < f.ny && column + j < f.nx) f.potential[static_cast<size_t>(r) * f.nx + column + j] = v[j];
-                }
+        } else if (step == kField) {
+            // Whole rows of the CTA's columns, a warp per row.
+            const int floats = 2 * max(0, min(N, f.nx - n0));
+            for (int row = warp; row < f.ny; row += kSmallWarps) {
+                const float* staged = reinterpret_cast<const float*>(smem + L::kBasisA) + row * L::kFieldPitch;
+                float* out = reinterpret_cast<float*>(f.field + static_cast<size_t>(row) * f.nx + n0);
+                for (int c = threadIdx.x & 31; c < floats; c += 32) out[c] = staged[c];
             }
         }
     }
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == kIssuer) {
         // Drain: nothing this CTA issued lands after it exits (all done already unless a wait ran out).
         if (pending_a) mbarWait(full_a, parity_a, nullptr);
         if (pending_b) mbarWait(full_b, parity_b, nullptr);
