@@ -943,8 +943,9 @@ EvalPlan Engine::plan(const EvalRequest& q) {
     sa.layers = layers_;
     sa.totals = totals_;
     sa.partials = partials_sc_;
+    const bool scatter_direct = scatter_blocks_ <= kDirectRows;
     sa.group_partials = sc_groups_.partials;
-    sa.group_counters = sc_groups_.counters;
+    sa.group_counters = scatter_direct ? nullptr : sc_groups_.counters;
     p.scatter = !q.reuse_density && particle_count_ > 0;
     p.scatter_blocks = scatter_blocks_;
     // The wirelength pass needs the positions only: it runs beside the density
@@ -989,7 +990,8 @@ EvalPlan Engine::plan(const EvalRequest& q) {
     ma.source = source_;
     ma.partials = partials_m_;
     ma.group_partials = m_groups_.partials;
-    ma.group_counters = m_groups_.counters;
+    const bool metrics_direct = metrics_blocks_ <= kDirectRows;
+    ma.group_counters = metrics_direct ? nullptr : m_groups_.counters;
     int kernels = 1;  // the wirelength pass
     if (!q.reuse_density) {
         p.metrics = true;
@@ -1018,13 +1020,18 @@ EvalPlan Engine::plan(const EvalRequest& q) {
     };
     add(wl_group_, wl_blocks_ > 0 ? wl_groups_ : 0, 1, 0, false, kSmooth);
     add(wl_group_, wl_blocks_ > 0 ? wl_groups_ : 0, 1, wl_groups_, false, kHpwl);
-    // The scatter, metrics and gather partials, folded per 32 blocks by the producers.
-    const int scatter_rows = particle_count_ > 0 && q.mode == kPropose ? sc_groups_.count : 0;
+    // The scatter, metrics and gather partials: folded per 32 blocks by the producers, those of
+    // few blocks (kDirectRows) as they are.
+    const double* const scatter_partials = scatter_direct ? partials_sc_ : sc_groups_.partials;
+    const int scatter_count = scatter_direct ? scatter_blocks_ : sc_groups_.count;
+    const int scatter_rows = particle_count_ > 0 && q.mode == kPropose ? scatter_count : 0;
+    const double* const metrics_partials = metrics_direct ? partials_m_ : m_groups_.partials;
+    const int metrics_count = metrics_direct ? metrics_blocks_ : m_groups_.count;
     if (!q.reuse_density) {  // otherwise the density scalars of the previous evaluation stand
-        add(sc_groups_.partials, scatter_rows, 1, 0, false, kPredicted);
-        add(sc_groups_.partials, scatter_rows, 1, sc_groups_.count, true, kMaxDisplacement);
+        add(scatter_partials, scatter_rows, 1, 0, false, kPredicted);
+        add(scatter_partials, scatter_rows, 1, scatter_count, true, kMaxDisplacement);
         for (int k = 0; k < 9; ++k) {
-            add(m_groups_.partials, m_groups_.count, 1, k * m_groups_.count, k >= 7, kOverflowWith + k);
+            add(metrics_partials, metrics_count, 1, k * metrics_count, k >= 7, kOverflowWith + k);
         }
         add(partials_e_, energy_blocks_, 1, 0, false, kEnergy);
     }

@@ -97,7 +97,7 @@ __device__ __forceinline__ void finishReduce(const ReduceArgs& a) {
 // error flag are also published to host memory.
 __device__ void reduceAllSources(const ReduceArgs& a) {
     constexpr int kSourcesPerWarp = 4;  // sources a warp handles per pass, loads issued together
-    constexpr int kRowsPerLane = 4;     // rows lane + 32 j prefetched per source
+    constexpr int kRowsPerLane = kDirectRows / 32;  // rows lane + 32 j prefetched per source
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int warps = blockDim.x >> 5;

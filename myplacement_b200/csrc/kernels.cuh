@@ -188,6 +188,13 @@ void launchRudyGradient(const RudyArgs& args, cudaStream_t stream);
 void launchRudyGather(const int* particle_pin_start, const double2* pin_gradient, int movable_count,
                       int particle_count, double2* out, cudaStream_t stream);
 
+// Partials of up to this many blocks are reduced directly: the reduction loads that many rows of
+// a source at once, and the producers' blocks end without folding theirs (two atomics and a
+// load, on the way to the next kernel).  Evaluations of 5,000 cells (24 and 64 blocks) 94 -> 91
+// us, iterations 76.6 -> 74.4; with up to 1,024 rows 210,000 cells gain nothing (1,016 and 512
+// blocks: 241 us either way).
+constexpr int kDirectRows = 128;
+
 // ---- deterministic reduction of all partials into the scalar block ----------------------
 // Source row r is partials[r * stride + column]; the producers write their
 // partials column-major (partial k of block b at k * grid + b), so stride is 1
