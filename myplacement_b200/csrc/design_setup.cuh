@@ -17,8 +17,8 @@ namespace mpgp {
 
 // The rule of a session's set-up: the device takes designs of at least this many modules and
 // pins whose scratch fits the budget (deviceSetupBytes).  Whole placements of two iterations
-// on a B200 with 16 host CPUs, host set-up against device set-up: 25,000 items 1.7 / 1.8 ms,
-// 51,000 1.96 / 1.72, 101,000 2.57 / 2.17, 226,000 5.9 / 2.8, 1.06 million 20.2 / 6.5.  The
+// on a B200 with 16 host CPUs, host set-up against device set-up: 25,000 items 1.49 / 1.47
+// ms, 51,000 1.80 / 1.62, 101,000 2.54 / 2.02, 226,000 5.9 / 2.87, 1.06 million 20.6 / 6.6.  The
 // host's part that is left is the validation, the module lists and sums that must be added in
 // order; below the line both are launch and allocation latency.
 constexpr int64_t kDeviceSetupItems = int64_t{1} << 15;

@@ -1015,8 +1015,9 @@ EvalPlan Engine::plan(const EvalRequest& q) {
 
     ReduceArgs& ra = p.reduce_args;
     int s = 0;
-    const auto add = [&](const double* partials, int rows, int stride, int column, bool is_max, int target) {
-        ra.sources[s++] = ReduceSource{partials, rows, stride, column, is_max ? 1 : 0, target};
+    const auto add = [&](const double* partials, int rows, int stride, int column, bool is_max, int target,
+                         bool direct = false) {
+        ra.sources[s++] = ReduceSource{partials, rows, stride, column, is_max ? 1 : 0, target, direct ? 1 : 0};
     };
     add(wl_group_, wl_blocks_ > 0 ? wl_groups_ : 0, 1, 0, false, kSmooth);
     add(wl_group_, wl_blocks_ > 0 ? wl_groups_ : 0, 1, wl_groups_, false, kHpwl);
@@ -1028,10 +1029,10 @@ EvalPlan Engine::plan(const EvalRequest& q) {
     const double* const metrics_partials = metrics_direct ? partials_m_ : m_groups_.partials;
     const int metrics_count = metrics_direct ? metrics_blocks_ : m_groups_.count;
     if (!q.reuse_density) {  // otherwise the density scalars of the previous evaluation stand
-        add(scatter_partials, scatter_rows, 1, 0, false, kPredicted);
+        add(scatter_partials, scatter_rows, 1, 0, false, kPredicted, scatter_direct);
         add(scatter_partials, scatter_rows, 1, scatter_count, true, kMaxDisplacement);
         for (int k = 0; k < 9; ++k) {
-            add(metrics_partials, metrics_count, 1, k * metrics_count, k >= 7, kOverflowWith + k);
+            add(metrics_partials, metrics_count, 1, k * metrics_count, k >= 7, kOverflowWith + k, metrics_direct);
         }
         add(partials_e_, energy_blocks_, 1, 0, false, kEnergy);
     }

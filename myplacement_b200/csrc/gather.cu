@@ -106,7 +106,7 @@ __device__ void reduceAllSources(const ReduceArgs& a) {
 #pragma unroll
         for (int i = 0; i < kSourcesPerWarp; ++i) {
             const int s = first + i * warps;
-            const ReduceSource src = s < a.source_count ? a.sources[s] : ReduceSource{nullptr, 0, 0, 0, 0, 0};
+            const ReduceSource src = s < a.source_count ? a.sources[s] : ReduceSource{nullptr, 0, 0, 0, 0, 0, 0};
 #pragma unroll
             for (int j = 0; j < kRowsPerLane; ++j) {
                 const int row = lane + 32 * j;
@@ -121,7 +121,14 @@ __device__ void reduceAllSources(const ReduceArgs& a) {
             const ReduceSource src = a.sources[s];
             double value = src.is_max ? -1.0e308 : 0.0;
 #pragma unroll
-            for (int j = 0; j < kRowsPerLane; ++j) value = src.is_max ? fmax(value, x[i][j]) : value + x[i][j];
+            for (int j = 0; j < kRowsPerLane; ++j) {
+                if (src.direct != 0 && src.is_max == 0) {
+                    const double group = warpSum(x[i][j]);
+                    if (lane == j) value = group;
+                } else {
+                    value = src.is_max ? fmax(value, x[i][j]) : value + x[i][j];
+                }
+            }
             for (int row = lane + 32 * kRowsPerLane; row < src.rows; row += 32) {
                 const double y = __ldcg(src.partials + static_cast<size_t>(row) * src.stride + src.column);
                 value = src.is_max ? fmax(value, y) : value + y;
@@ -234,7 +241,8 @@ __global__ void __launch_bounds__(kThreads) gatherBatchKernel(const GatherArgs* 
 // The scalar reduction as its own kernel: every partial of every source is
 // first staged in shared memory with all loads in flight together (eight per
 // thread at a time), then warp w sums sources w, w + 32, ... from shared memory,
-// lane l taking rows l, l + 32, ... in order and a fixed shuffle tree.
+// lane l taking rows l, l + 32, ... in order and a fixed shuffle tree (direct
+// sources: 32 rows at a time, as reduceGroups would have folded them).
 __device__ __forceinline__ void reduceBlock(const ReduceArgs& a) {
     extern __shared__ double staged[];
     const int total = a.offsets[a.source_count];
@@ -279,9 +287,16 @@ __device__ __forceinline__ void reduceBlock(const ReduceArgs& a) {
         const ReduceSource& src = a.sources[s];
         const int first = offset_of[s];
         double value = src.is_max ? -1.0e308 : 0.0;
-        for (int row = lane; row < src.rows; row += 32) {
-            const double y = staged[first + row];
-            value = src.is_max ? fmax(value, y) : value + y;
+        if (src.direct != 0 && src.is_max == 0) {
+            for (int j = 0; 32 * j < src.rows; ++j) {
+                const double group = warpSum(32 * j + lane < src.rows ? staged[first + 32 * j + lane] : 0.0);
+                if (lane == j) value = group;
+            }
+        } else {
+            for (int row = lane; row < src.rows; row += 32) {
+                const double y = staged[first + row];
+                value = src.is_max ? fmax(value, y) : value + y;
+            }
         }
         value = src.is_max ? warpMax(value) : warpSum(value);
         if (lane == 0) {

@@ -206,6 +206,7 @@ struct ReduceSource {
     int column;  // offset of row 0
     int is_max;
     int target;  // Scalar slot
+    int direct;  // rows of blocks (at most kDirectRows), summed 32 at a time as reduceGroups folds them
 };
 struct ReduceArgs {
     ReduceSource sources[kScalarCount];
