@@ -48,7 +48,6 @@
 #include "ingest.cuh"
 #include "pinned.hpp"
 #include "setup.hpp"
-#include "transfer.hpp"
 #include "workers.hpp"
 
 namespace mpgp {
@@ -1606,12 +1605,10 @@ bool placeOnDevice(const mpgp_design& d, const int32_t* row_orientation, const m
         return false;  // the host's path says what is missing
     }
     PassMemory& scratch = *memory;
-    HostTransfer transfer(stream, static_cast<std::size_t>(std::max(modules, pins)) * sizeof(double));
-    const HostTransfer::Call call(&transfer);
     const auto put = [&](const auto* host, std::size_t count) {
         using T = std::remove_const_t<std::remove_pointer_t<decltype(host)>>;
         T* device = scratch.array<T>(count);
-        transfer.send(host, device, count * sizeof(T));
+        checkCuda(cudaMemcpyAsync(device, host, count * sizeof(T), cudaMemcpyHostToDevice, stream), "upload the design");
         return device;
     };
 
@@ -1670,7 +1667,6 @@ bool placeOnDevice(const mpgp_design& d, const int32_t* row_orientation, const m
     checkDesignKernel<<<threadBlocks(std::max({m_count, n_count, p_count})), kThreads, 0, stream>>>(raw, changed);
     checkCuda(cudaMemcpyAsync(host_changed, changed, sizeof(int), cudaMemcpyDeviceToHost, stream), "check the design");
     checkCuda(cudaStreamSynchronize(stream), "check the design");
-    transfer.settled();
     if (*host_changed != 0) return false;
 
     double2* center = scratch.array<double2>(m_count);
@@ -1888,12 +1884,15 @@ bool placeOnDevice(const mpgp_design& d, const int32_t* row_orientation, const m
     checkCuda(cudaGetLastError(), "detailed-placement result");
     readCounts();
     accepted += host_counts->accepted;
-    std::vector<HostTransfer::Piece> pieces{{x, module_x, m_count * sizeof(double)}, {y, module_y, m_count * sizeof(double)}};
-    if (module_orientation != nullptr) pieces.push_back({orientation_out, module_orientation, m_count * sizeof(int32_t)});
-    transfer.startDownload(pieces);
     result.hpwl_before = hpwl_before;
     result.hpwl_after = sum(term_after, side.get());
-    transfer.finishDownload();
+    const auto bring = [&](const auto* device, auto* host) {
+        checkCuda(cudaMemcpyAsync(host, device, m_count * sizeof(*host), cudaMemcpyDeviceToHost, stream), "detailed-placement result");
+    };
+    bring(x, module_x);
+    bring(y, module_y);
+    if (module_orientation != nullptr) bring(orientation_out, module_orientation);
+    checkCuda(cudaStreamSynchronize(stream), "detailed-placement result");
     result.cuda_device_used = options.cuda_device;
     result.evaluated_windows = evaluated;
     result.evaluated_permutations = permutations;

@@ -192,15 +192,6 @@ bool HostTransfer::upload(const double* source, double* destination, std::size_t
                 count * sizeof(double), check);
 }
 
-void HostTransfer::send(const void* source, void* destination, std::size_t bytes) {
-    if (bytes == 0) return;
-    if (helped_ && bytes >= kLargeBytes) {
-        move(static_cast<const unsigned char*>(source), static_cast<unsigned char*>(destination), bytes, false);
-    } else {
-        checkCuda(cudaMemcpyAsync(destination, source, bytes, cudaMemcpyHostToDevice, stream_), "Upload to the device");
-    }
-}
-
 bool HostTransfer::move(const unsigned char* source, unsigned char* destination, std::size_t bytes, bool check) {
     // Slots that an earlier move of this call still uses: its last copies, from the last slots' events.
     if (in_flight_) {

@@ -83,9 +83,6 @@ public:
     // Copies `count` doubles to the device on the stream.  With `check`, returns whether all
     // are finite.  The source has been read when this returns.
     bool upload(const double* source, double* destination, std::size_t count, bool check);
-    // Copies bytes to the device on the stream; the source has been read when this returns.
-    // Bytes that are few, or beside another thread's call, take the driver's own staging.
-    void send(const void* source, void* destination, std::size_t bytes);
 
     struct Piece {
         const void* device = nullptr;
