@@ -23,10 +23,10 @@
 // Bound by latency: a chain of four products with an epilogue, an operand write and a barrier
 // each, on one to four SMs.  As four launches against one (a backend evaluation, and one
 // iteration of a placement, microseconds):
-//   32 x 32    91.2 ->  81.3   110.1 ->  89.9      65 x 65    108.0 -> 103.3   110.2 -> 103.6
-//   64 x 64   109.6 ->  93.2    95.6 ->  78.8      128 x 64   131.3 -> 114.6   103.7 ->  82.6
-//   96 x 96   121.9 -> 114.6   121.6 -> 114.4      128 x 128  148.6 -> 142.6   128.6 -> 122.6
-// and 24 to 200 placements in shared launches 3 to 12 % faster.  Two K-blocks along an axis
+//   32 x 32    90.6 ->  76.3   107.9 ->  86.7      65 x 65    101.5 ->  93.6   106.8 ->  91.6
+//   64 x 64   101.5 ->  90.2    91.9 ->  74.5      128 x 64   128.7 -> 109.5    99.0 ->  78.2
+//   96 x 96   118.6 -> 111.9   113.8 -> 105.3      128 x 128  143.3 -> 135.7   120.1 -> 114.3
+// and 24 to 200 placements in shared launches 6 to 13 % faster.  Two K-blocks along an axis
 // gain less: the FP64 sums of its epilogues are the larger part then.
 //
 // The arithmetic is that of dct_tc.cu: K-block partials summed in FP64 and rounded once
