@@ -20,7 +20,10 @@ namespace mpgp {
 // on a B200 with 16 host CPUs, host set-up against device set-up: 25,000 items 1.49 / 1.47
 // ms, 51,000 1.80 / 1.62, 101,000 2.54 / 2.02, 226,000 5.9 / 2.87, 1.06 million 20.6 / 6.6.  The
 // host's part that is left is the validation, the module lists and sums that must be added in
-// order; below the line both are launch and allocation latency.
+// order; below the line both are launch and allocation latency.  Sessions of several threads
+// at once (45,000 cells, 16 iterations each): 4 threads 15 / 9.7 ms, 6 16.5 / 14.9, 10 27 / 25;
+// at 16, as many as host CPUs, the device's read-backs wait for one another's kernels and the
+// host's set-ups are the faster ones, 42 / 44-60.
 constexpr int64_t kDeviceSetupItems = int64_t{1} << 15;
 // In a batch the set-ups of several sessions and the running rounds share one stream, so every
 // read-back of a set-up on the device waits for them, while the host's set-ups run on threads of
