@@ -320,6 +320,13 @@ void Engine::loadDesign(const mpgp_design& d, const DerivedDesign& derived, cons
     };
     // Declared before the threads that use it.
     Scratch scratch(stream_, [this] { return arena_.headroom(); });
+    // The scratch is given back in the order of the engine's stream, and the second thread's kernels
+    // run on the side stream: whichever way the set-up ends, they are done before that.
+    const cudaStream_t side = stream_wl_ != nullptr ? stream_wl_ : stream_;
+    struct SideDone {
+        cudaStream_t side;
+        ~SideDone() { cudaStreamSynchronize(side); }
+    } side_done{side};
     DeviceModules m;
     m.count = d.module_count;
     Join areas_thread{std::thread([&] {
@@ -357,7 +364,6 @@ void Engine::loadDesign(const mpgp_design& d, const DerivedDesign& derived, cons
     checkCuda(cudaMemsetAsync(m.pins, 0, modules * sizeof(int), stream_), "Clear the pin counts");
     launchMapModules(m, movable, stream_);
     allocateDensity();
-    const cudaStream_t side = stream_wl_ != nullptr ? stream_wl_ : stream_;
     checkCuda(cudaEventRecord(fork_, stream_), "Modules on the device");
     checkCuda(cudaStreamWaitEvent(side, fork_, 0), "Modules on the device");
     Join side_thread{std::thread([&] {
