@@ -551,9 +551,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) fieldSmallBatchKernel(const 
     releaseNext();
     const FieldSmallItem item = items[blockIdx.x / static_cast<unsigned>(cluster)];
     const FieldSmall& field = *item.field;
-    if (threadIdx.x == 0) {
-        // Uploaded by a copy, possibly into memory an earlier engine's maps used: make the
-        // TMA proxy see their current bytes.
+    if (threadIdx.x == kIssuer) {
+        // Uploaded by a copy, possibly into memory an earlier engine's maps used: the thread that
+        // prefetches them and issues the loads makes the TMA proxy see their current bytes.
         for (const CUtensorMap* map : {&field.map_s, &field.map_cy, &field.map_dy, &field.map_syw, &field.map_cx,
                                        &field.map_dxc, &field.map_sxwt}) {
             asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
