@@ -143,39 +143,46 @@ struct EntryLists {
     std::vector<int> start;
 };
 
-// The rectangles' entries by bin row: each rectangle that overlaps the region goes to every bin
-// row it spans (Grid::span), in the given order.
 struct Rectangle {
     double llx, lly, urx, ury;
 };
 
-EntryLists entryLists(const std::vector<Rectangle>& rectangles, const Rect2& region, int columns, int rows) {
+// A rectangle's entry and the bin rows it goes to: those it spans (Grid::span).
+struct Span {
+    StaticEntry entry;
+    int first_row, last_row;
+};
+
+// False for a rectangle that does not overlap the region.
+bool spanOf(const Rectangle& r, const Rect2& region, int columns, int rows, Span& s) {
     const double bin_width = region.width() / static_cast<double>(columns);
     const double bin_height = region.height() / static_cast<double>(rows);
-    struct Span {
-        StaticEntry entry;
-        int first_row, last_row;
+    const Rectangle c{std::max(r.llx, region.llx), std::max(r.lly, region.lly), std::min(r.urx, region.urx),
+                      std::min(r.ury, region.ury)};
+    const double area = std::max(0.0, c.urx - c.llx) * std::max(0.0, c.ury - c.lly);
+    if (area <= kEpsilon) return false;
+    const auto first = [](double offset, double length, int count) {
+        return std::max(0, std::min(count - 1, static_cast<int>(std::floor(offset / length))));
     };
+    const auto last = [](double offset, double length, int count) {
+        return std::max(0, std::min(count - 1, static_cast<int>(std::ceil(offset / length) - 1.0)));
+    };
+    s.entry = StaticEntry{c.llx, c.lly, c.urx, c.ury, first(c.llx - region.llx, bin_width, columns),
+                          last(c.urx - region.llx, bin_width, columns)};
+    s.first_row = first(c.lly - region.lly, bin_height, rows);
+    s.last_row = last(c.ury - region.lly, bin_height, rows);
+    return true;
+}
+
+// The rectangles' entries by bin row, in the given order.
+EntryLists entryLists(const std::vector<Rectangle>& rectangles, const Rect2& region, int columns, int rows) {
     std::vector<Span> spans;
     spans.reserve(rectangles.size());
     EntryLists out;
     out.start.assign(static_cast<std::size_t>(rows) + 1, 0);
     for (const Rectangle& r : rectangles) {
-        const Rectangle c{std::max(r.llx, region.llx), std::max(r.lly, region.lly), std::min(r.urx, region.urx),
-                          std::min(r.ury, region.ury)};
-        const double area = std::max(0.0, c.urx - c.llx) * std::max(0.0, c.ury - c.lly);
-        if (area <= kEpsilon) continue;
-        const auto first = [](double offset, double length, int count) {
-            return std::max(0, std::min(count - 1, static_cast<int>(std::floor(offset / length))));
-        };
-        const auto last = [](double offset, double length, int count) {
-            return std::max(0, std::min(count - 1, static_cast<int>(std::ceil(offset / length) - 1.0)));
-        };
         Span s{};
-        s.entry = StaticEntry{c.llx, c.lly, c.urx, c.ury, first(c.llx - region.llx, bin_width, columns),
-                              last(c.urx - region.llx, bin_width, columns)};
-        s.first_row = first(c.lly - region.lly, bin_height, rows);
-        s.last_row = last(c.ury - region.lly, bin_height, rows);
+        if (!spanOf(r, region, columns, rows, s)) continue;
         for (int row = s.first_row; row <= s.last_row; ++row) ++out.start[static_cast<std::size_t>(row) + 1];
         spans.push_back(s);
     }
@@ -190,16 +197,42 @@ EntryLists entryLists(const std::vector<Rectangle>& rectangles, const Rect2& reg
     return out;
 }
 
+Rectangle rowRectangle(const mpgp_design& d, int r) {
+    const double x_end = d.row_x_start[r] + static_cast<double>(d.row_site_count[r]) * d.row_site_spacing[r];
+    return {d.row_x_start[r], d.row_bottom[r], x_end, d.row_bottom[r] + d.row_height[r]};
+}
+
+Rectangle moduleRectangle(const mpgp_design& d, int32_t m) {
+    const double x = d.module_x[m], y = d.module_y[m], w = d.module_width[m], h = d.module_height[m];
+    return {x - w * 0.5, y - h * 0.5, x + w * 0.5, y + h * 0.5};
+}
+
 }  // namespace
 
-uint64_t deviceSetupBytes(const mpgp_design& d, int bins) {
+uint64_t staticEntryCount(const mpgp_design& d, const DerivedDesign& derived, int bins_x, int bins_y) {
+    uint64_t entries = 0;
+    Span s{};
+    const auto add = [&](const Rectangle& r) {
+        if (spanOf(r, derived.core, bins_x, bins_y, s)) entries += static_cast<uint64_t>(s.last_row - s.first_row) + 1;
+    };
+    for (int r = 0; r < d.row_count; ++r) add(rowRectangle(d, r));
+    if (derived.movable.size() < static_cast<std::size_t>(d.module_count)) {
+        for (int32_t m = 0; m < d.module_count; ++m) {
+            if (derived.is_fixed[m]) add(moduleRectangle(d, m));
+        }
+    }
+    return entries;
+}
+
+uint64_t deviceSetupBytes(const mpgp_design& d, uint64_t static_entries, int bins_x, int bins_y) {
     const uint64_t pins = static_cast<uint64_t>(d.pin_count), modules = static_cast<uint64_t>(d.module_count);
-    const uint64_t nets = static_cast<uint64_t>(d.net_count), rows = static_cast<uint64_t>(d.row_count);
+    const uint64_t nets = static_cast<uint64_t>(d.net_count);
+    const uint64_t bins = static_cast<uint64_t>(bins_x) * static_cast<uint64_t>(bins_y);
     // Per pin: the design's arrays (20), the layout's staging and sorting scratch (88) and its
     // lasting arrays (24); per module: geometry and maps, and the area sort (24); per net: the
     // offsets and weights, the net sort and the lasting arrays; the static layers and lists.
-    return 160 * pins + 96 * modules + 128 * nets + 64 * static_cast<uint64_t>(bins) + 256 * (rows + 1024) +
-           (uint64_t{32} << 20);
+    return 160 * pins + 96 * modules + 128 * nets + 64 * bins + sizeof(StaticEntry) * static_entries +
+           8 * (static_cast<uint64_t>(bins_y) + 1) + (uint64_t{32} << 20);
 }
 
 void launchMapModules(const DeviceModules& m, int movable, cudaStream_t stream) {
@@ -225,16 +258,11 @@ StaticSums staticLayersOnDevice(const mpgp_design& d, const DerivedDesign& deriv
             "DensityMap requires a valid region, positive dimensions, and target density.");
     std::vector<Rectangle> rectangles;
     rectangles.reserve(static_cast<std::size_t>(d.row_count));
-    for (int r = 0; r < d.row_count; ++r) {
-        const double x_end = d.row_x_start[r] + static_cast<double>(d.row_site_count[r]) * d.row_site_spacing[r];
-        rectangles.push_back({d.row_x_start[r], d.row_bottom[r], x_end, d.row_bottom[r] + d.row_height[r]});
-    }
+    for (int r = 0; r < d.row_count; ++r) rectangles.push_back(rowRectangle(d, r));
     const EntryLists rows = entryLists(rectangles, region, bins_x, bins_y);
     rectangles.clear();
     for (int32_t m = 0; m < d.module_count; ++m) {
-        if (!derived.is_fixed[m]) continue;
-        const double x = d.module_x[m], y = d.module_y[m], w = d.module_width[m], h = d.module_height[m];
-        rectangles.push_back({x - w * 0.5, y - h * 0.5, x + w * 0.5, y + h * 0.5});
+        if (derived.is_fixed[m]) rectangles.push_back(moduleRectangle(d, m));
     }
     const EntryLists modules = entryLists(rectangles, region, bins_x, bins_y);
 

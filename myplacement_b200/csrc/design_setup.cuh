@@ -31,8 +31,10 @@ constexpr int64_t kDeviceSetupItems = int64_t{1} << 15;
 // items) 38 / 65 ms, 16 of 30,000 (151,000) 43 / 43, 12 of 80,000 (404,000) 76 / 66.
 constexpr int64_t kBatchDeviceSetupItems = int64_t{1} << 18;
 
+// The static layers' list entries: one per SiteRow or fixed module and bin row that it spans.
+uint64_t staticEntryCount(const mpgp_design& design, const DerivedDesign& derived, int bins_x, int bins_y);
 // More than the set-up's transient device memory and the net layout's lasting arrays together.
-uint64_t deviceSetupBytes(const mpgp_design& design, int bins);
+uint64_t deviceSetupBytes(const mpgp_design& design, uint64_t static_entries, int bins_x, int bins_y);
 
 // The design's modules on the device: scratch that lives until the set-up is done.
 struct DeviceModules {

@@ -285,10 +285,10 @@ void Engine::uploadStatic(const Problem& p) {
     allocatePartials();
 }
 
-bool Engine::setsUpOnDevice(const mpgp_design& d) const {
+bool Engine::setsUpOnDevice(const mpgp_design& d, const DerivedDesign& derived) const {
     const int64_t least = batch_ == nullptr ? kDeviceSetupItems : kBatchDeviceSetupItems;
     return static_cast<int64_t>(d.module_count) + d.pin_count >= least &&
-           deviceSetupBytes(d, bin_count_) <= arena_.headroom();
+           deviceSetupBytes(d, staticEntryCount(d, derived, bins_x_, bins_y_), bins_x_, bins_y_) <= arena_.headroom();
 }
 
 // The session's set-up on the device (design_setup.cuh).  The caller's arrays are uploaded as

@@ -174,7 +174,7 @@ public:
     void loadParticles(const Problem& problem);
     // Or from a session's design, set up on the device where setsUpOnDevice says so; the
     // initial positions are then in scratchPositions().
-    [[nodiscard]] bool setsUpOnDevice(const mpgp_design& design) const;
+    [[nodiscard]] bool setsUpOnDevice(const mpgp_design& design, const DerivedDesign& derived) const;
     void loadDesign(const mpgp_design& design, const DerivedDesign& derived, const mpgp_options& options);
     // out = positions moved into the region as far as the particles' sizes allow (applyPositions,
     // AdaptiveGlobalPlacer.cpp:185-198).

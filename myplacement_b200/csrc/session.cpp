@@ -131,7 +131,7 @@ Session::Session(const mpgp_design& design, const mpgp_options& options, Batch* 
     bool on_device = false;
     if (large) {
         makeEngine();
-        on_device = engine_->setsUpOnDevice(design);
+        on_device = engine_->setsUpOnDevice(design, derived_);
         if (on_device) {
             engine_->loadDesign(design, derived_, options_);
         } else {

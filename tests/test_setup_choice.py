@@ -1,0 +1,49 @@
+"""Which path sets a session up: nothing that the host's set-up takes is refused (needs a GPU).
+
+The device's set-up needs scratch beside the session's arrays: the design as it is, and per bin
+row a list of the SiteRows and fixed modules that span it.  A design whose scratch does not fit
+its memory budget is set up on the host.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import myplacement_b200 as mp
+from myplacement_b200 import _abi
+
+pytestmark = pytest.mark.gpu
+
+
+def _with_blocks(blocks: int, height: float, seed: int = 3, cells: int = 12_000) -> mp.Design:
+    """A design with fixed blocks of `height` (a share of the core) that are a small part of a bin wide."""
+    design = mp.synthetic_design(cells=cells, nets=cells, terminals=16, seed=seed)
+    design = design.copy_with_positions(*mp.random_placement(design, seed))
+    rng = np.random.default_rng(seed)
+    llx, lly, urx, ury = design.core
+    fields = {k: getattr(design, k) for k in design.__dataclass_fields__ if not k.startswith("_")}
+    fields["module_width"] = np.concatenate([design.module_width, np.full(blocks, 1e-4 * (urx - llx))])
+    fields["module_height"] = np.concatenate([design.module_height, np.full(blocks, height * (ury - lly))])
+    fields["module_x"] = np.concatenate([design.module_x, rng.uniform(llx, urx, blocks)])
+    fields["module_y"] = np.concatenate([design.module_y, rng.uniform(lly, ury, blocks)])
+    fields["module_flags"] = np.concatenate([design.module_flags, np.full(blocks, _abi.MODULE_FIXED)])
+    return mp.Design(**fields)
+
+
+def _place(design: mp.Design, **overrides):
+    options = mp.default_options(bins_x=256, bins_y=256, target_density=0.9, iterations=2, **overrides)
+    return mp.GlobalPlacer().run(design, options)
+
+
+@pytest.mark.parametrize("blocks,height", [(20_000, 1.0), (60_000, 0.3)])
+def test_lists_beyond_the_budget(gpu, blocks, height):
+    design = _with_blocks(blocks, height)
+    # Every block is listed in each of the bin rows it spans, 40 bytes a time: about 200 MB, far more
+    # than the rest of the set-up.
+    options = mp.default_options(bins_x=256, bins_y=256, target_density=0.9, iterations=2)
+    budget = mp.estimate_bytes(design, options) + (100 << 20)
+    tight = _place(design, maximum_cuda_memory_bytes=budget)
+    free = _place(design)
+    assert tight.result["cuda_reserved_memory_bytes"] <= budget
+    assert np.array_equal(tight.module_x, free.module_x) and np.array_equal(tight.module_y, free.module_y)
+    assert tight.history == free.history
