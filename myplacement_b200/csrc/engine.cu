@@ -285,10 +285,23 @@ void Engine::uploadStatic(const Problem& p) {
     allocatePartials();
 }
 
-bool Engine::setsUpOnDevice(const mpgp_design& d, const DerivedDesign& derived) const {
-    const int64_t least = batch_ == nullptr ? kDeviceSetupItems : kBatchDeviceSetupItems;
-    return static_cast<int64_t>(d.module_count) + d.pin_count >= least &&
-           deviceSetupBytes(d, staticEntryCount(d, derived, bins_x_, bins_y_), bins_x_, bins_y_) <= arena_.headroom();
+uint64_t Engine::gridBytes(int bins_x, int bins_y) {
+    const uint64_t nx = static_cast<uint64_t>(bins_x), ny = static_cast<uint64_t>(bins_y);
+    const uint64_t ldx = static_cast<uint64_t>(paddedLd(bins_x)), ldy = static_cast<uint64_t>(paddedLd(bins_y));
+    // The bases, the source and the stages' planes (two of 2 bytes each) and the banded solve's
+    // two more and kept coefficients; scale, field and potential; everything else.
+    return 4 * (3 * nx * ldx + 3 * ny * ldy + 5 * ny * ldx + 3 * nx * ldy) + 4 * ldx * (ny + kTileM) + 16 * nx * ny +
+           (uint64_t{1} << 20);
+}
+
+bool Engine::setsUpOnDevice(const mpgp_design& d, const DerivedDesign& derived, const mpgp_options& o, bool batched) {
+    const int64_t least = batched ? kBatchDeviceSetupItems : kDeviceSetupItems;
+    if (static_cast<int64_t>(d.module_count) + d.pin_count < least) return false;
+    const uint64_t budget = o.maximum_cuda_memory_bytes;
+    const auto fits = [&](uint64_t entries) {
+        return gridBytes(o.bins_x, o.bins_y) + deviceSetupBytes(d, entries, o.bins_x, o.bins_y) <= budget;
+    };
+    return fits(0) && fits(staticEntryCount(d, derived, o.bins_x, o.bins_y));
 }
 
 // The session's set-up on the device (design_setup.cuh).  The caller's arrays are uploaded as

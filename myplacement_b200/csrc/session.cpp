@@ -107,9 +107,7 @@ Session::Session(const mpgp_design& design, const mpgp_options& options, Batch* 
     module_x_.assign(design.module_x, design.module_x + design.module_count);
     module_y_.assign(design.module_y, design.module_y + design.module_count);
     result_.compute_backend_used = MPGP_BACKEND_CUDA;
-    // A large design is set up on the device, which counts its modules' pins itself.
-    const bool large = static_cast<int64_t>(design.module_count) + design.pin_count >= kDeviceSetupItems;
-    derived_ = deriveDesign(design, !large);
+    derived_ = deriveDesign(design, false);  // the set-up counts the modules' pins
     if (derived_.movable.empty()) {  // AdaptiveGlobalPlacer.cpp:653
         empty_ = true;
         done_ = true;
@@ -125,20 +123,14 @@ Session::Session(const mpgp_design& design, const mpgp_options& options, Batch* 
         }
         require(options_.cuda_device >= 0 && options_.cuda_device < device_count,
                 "Requested CUDA device does not exist on this host.");
-        engine_ = std::make_unique<Engine>(grid, options_.cuda_device, options_.maximum_cuda_memory_bytes,
-                                           rudy_requested_ ? nullptr : batch);
+        engine_ = std::make_unique<Engine>(grid, options_.cuda_device, options_.maximum_cuda_memory_bytes, batch);
     };
-    bool on_device = false;
-    if (large) {
+    if (rudy_requested_) batch = nullptr;
+    const bool on_device = Engine::setsUpOnDevice(design, derived_, options_, batch != nullptr);
+    if (on_device) {
         makeEngine();
-        on_device = engine_->setsUpOnDevice(design, derived_);
-        if (on_device) {
-            engine_->loadDesign(design, derived_, options_);
-        } else {
-            derived_ = deriveDesign(design);  // with the pin counts
-        }
-    }
-    if (!on_device) {
+        engine_->loadDesign(design, derived_, options_);
+    } else {
         // The host problem is built on two threads while this one sets up the engine's grid
         // part on the device (the field solve's bases and buffers need only the grid): the
         // pin and net arrays, whose device layout then starts at once, and the static
@@ -153,6 +145,7 @@ Session::Session(const mpgp_design& design, const mpgp_options& options, Batch* 
         });
         std::thread particles_thread([&] {
             try {
+                derived_.pin_count = countPins(design);
                 buildProblemParticles(design, derived_, options_, problem_, fillers_);
             } catch (...) {
                 particles_error = std::current_exception();
@@ -164,7 +157,7 @@ Session::Session(const mpgp_design& design, const mpgp_options& options, Batch* 
                 if (t.joinable()) t.join();
             }
         } join_pins{pins_thread}, join_particles{particles_thread};
-        if (engine_ == nullptr) makeEngine();
+        makeEngine();
         pins_thread.join();
         if (pins_error) std::rethrow_exception(pins_error);
         engine_->loadNets(problem_, static_cast<int64_t>(derived_.movable.size()));

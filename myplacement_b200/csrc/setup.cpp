@@ -289,14 +289,11 @@ DerivedDesign deriveDesign(const mpgp_design& d, bool with_pins) {
         out.core = {core.llx, core.lly, core.urx, core.ury};
     }
     const std::size_t modules = static_cast<std::size_t>(d.module_count);
-    const std::size_t pins = with_pins ? static_cast<std::size_t>(d.pin_count) : 0;
     out.is_fixed.resize(modules);
     out.is_macro.resize(modules);
-    if (with_pins) out.pin_count.assign(modules, 0);
-    // Module flags and the movable list (in module order: each piece's movable
-    // modules go after those of the pieces before it), then the pin counts (integer
-    // sums, so the pieces' order does not matter), on up to eight host threads.
-    const Workers workers = setupWorkers(modules + pins);
+    // Module flags, then the movable list (in module order: each piece's movable modules go
+    // after those of the pieces before it), on up to eight host threads.
+    const Workers workers = setupWorkers(modules);
     const std::size_t pieces = static_cast<std::size_t>(workers.threads());
     const auto bound = [&](std::size_t k, std::size_t n) { return n * k / pieces; };
     std::vector<std::size_t> movable_in(pieces + 1, 0);
@@ -316,30 +313,39 @@ DerivedDesign deriveDesign(const mpgp_design& d, bool with_pins) {
     });
     for (std::size_t k = 0; k < pieces; ++k) movable_in[k + 1] += movable_in[k];
     out.movable.resize(movable_in[pieces]);
-    std::vector<std::vector<int32_t>> counts(pieces > 1 ? pieces : 0);
     workers.run(pieces, [&](std::size_t k) {
         std::size_t at = movable_in[k];
         for (std::size_t m = bound(k, modules); m < bound(k + 1, modules); ++m) {
             if (!out.is_fixed[m]) out.movable[at++] = static_cast<int32_t>(m);
         }
-        if (pieces > 1 && with_pins) {
-            std::vector<int32_t>& mine = counts[k];
-            mine.assign(modules, 0);
-            for (std::size_t p = bound(k, pins); p < bound(k + 1, pins); ++p) ++mine[d.pin_module[p]];
+    });
+    if (with_pins) out.pin_count = countPins(d);
+    return out;
+}
+
+std::vector<int32_t> countPins(const mpgp_design& d) {
+    const std::size_t modules = static_cast<std::size_t>(d.module_count);
+    const std::size_t pins = static_cast<std::size_t>(d.pin_count);
+    std::vector<int32_t> out(modules, 0);
+    const Workers workers = setupWorkers(modules + pins);
+    const std::size_t pieces = static_cast<std::size_t>(workers.threads());
+    if (pieces <= 1) {
+        for (std::size_t p = 0; p < pins; ++p) ++out[d.pin_module[p]];
+        return out;
+    }
+    // Integer sums, so the pieces' order does not matter.
+    const auto bound = [&](std::size_t k, std::size_t n) { return n * k / pieces; };
+    std::vector<std::vector<int32_t>> counts(pieces);
+    workers.run(pieces, [&](std::size_t k) {
+        std::vector<int32_t>& mine = counts[k];
+        mine.assign(modules, 0);
+        for (std::size_t p = bound(k, pins); p < bound(k + 1, pins); ++p) ++mine[d.pin_module[p]];
+    });
+    workers.run(pieces, [&](std::size_t k) {
+        for (std::size_t m = bound(k, modules); m < bound(k + 1, modules); ++m) {
+            for (std::size_t j = 0; j < pieces; ++j) out[m] += counts[j][m];
         }
     });
-    if (!with_pins) return out;
-    if (pieces <= 1) {
-        for (std::size_t p = 0; p < pins; ++p) ++out.pin_count[d.pin_module[p]];
-    } else {
-        workers.run(pieces, [&](std::size_t k) {
-            for (std::size_t m = bound(k, modules); m < bound(k + 1, modules); ++m) {
-                int32_t sum = 0;
-                for (std::size_t j = 0; j < pieces; ++j) sum += counts[j][m];
-                out.pin_count[m] = sum;
-            }
-        });
-    }
     return out;
 }
 

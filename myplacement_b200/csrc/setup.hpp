@@ -60,6 +60,8 @@ struct DerivedDesign {
 
 // Without `with_pins` the pin counts stay empty.
 DerivedDesign deriveDesign(const mpgp_design& design, bool with_pins = true);
+// The pins per module.
+std::vector<int32_t> countPins(const mpgp_design& design);
 // The median row height (zero without rows): a standard cell's height.
 double nominalRowHeight(const mpgp_design& design);
 

@@ -47,3 +47,17 @@ def test_lists_beyond_the_budget(gpu, blocks, height):
     assert tight.result["cuda_reserved_memory_bytes"] <= budget
     assert np.array_equal(tight.module_x, free.module_x) and np.array_equal(tight.module_y, free.module_y)
     assert tight.history == free.history
+
+
+@pytest.mark.parametrize("bins", [(64, 64), (257, 320), (130, 96)])
+def test_budgets_between_the_paths(gpu, bins):
+    """From the budget that the host's set-up needs to one that the device's fits: no budget is
+    refused, and the path makes no difference."""
+    design = _with_blocks(500, 0.2, seed=5, cells=20_000)
+    overrides = {"bins_x": bins[0], "bins_y": bins[1], "target_density": 0.9, "iterations": 2}
+    need = mp.estimate_bytes(design, mp.default_options(**overrides))
+    runs = [mp.GlobalPlacer().run(design, mp.default_options(maximum_cuda_memory_bytes=need + (extra << 20), **overrides))
+            for extra in range(0, 56, 4)]
+    for run in runs[1:]:
+        assert np.array_equal(run.module_x, runs[0].module_x) and np.array_equal(run.module_y, runs[0].module_y)
+        assert run.history == runs[0].history
