@@ -31,6 +31,14 @@ constexpr int64_t kDeviceSetupItems = int64_t{1} << 15;
 // items) 38 / 65 ms, 16 of 30,000 (151,000) 43 / 43, 12 of 80,000 (404,000) 76 / 66.
 constexpr int64_t kBatchDeviceSetupItems = int64_t{1} << 18;
 
+// Whether the static layers' lists, which the host builds and uploads, cost less than what the
+// device saves otherwise.  Whole placements of two iterations, device against host, by (entries
+// + 2 x fixed modules) / items: 30,000 cells 0.50: 3.3 / 4.1 ms, 0.71: 3.5 / 4.1, 0.92: 5.0 / 4.9,
+// 1.7: 5.2 / 4.6, 6.6: 18 / 5.8; 210,000 cells 0.22: 9.0 / 14.9, 0.44: 17.4 / 17.1, 0.50: 13.8 /
+// 17.7, 0.70: 24 / 18, 1.0: 28 / 19.6, 1.9: 55 / 23; 8,000 cells 0.16: 1.64 / 1.62, 1.0: 2.0 / 1.6.
+inline bool listsPay(uint64_t entries, uint64_t fixed, int64_t items) {
+    return entries + 2 * fixed <= static_cast<uint64_t>(items) / 2;
+}
 // The static layers' list entries: one per SiteRow or fixed module and bin row that it spans.
 uint64_t staticEntryCount(const mpgp_design& design, const DerivedDesign& derived, int bins_x, int bins_y);
 // More than the set-up's transient device memory and the net layout's lasting arrays together.

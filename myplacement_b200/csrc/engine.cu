@@ -295,13 +295,17 @@ uint64_t Engine::gridBytes(int bins_x, int bins_y) {
 }
 
 bool Engine::setsUpOnDevice(const mpgp_design& d, const DerivedDesign& derived, const mpgp_options& o, bool batched) {
-    const int64_t least = batched ? kBatchDeviceSetupItems : kDeviceSetupItems;
-    if (static_cast<int64_t>(d.module_count) + d.pin_count < least) return false;
+    const int64_t items = static_cast<int64_t>(d.module_count) + d.pin_count;
+    if (items < (batched ? kBatchDeviceSetupItems : kDeviceSetupItems)) return false;
     const uint64_t budget = o.maximum_cuda_memory_bytes;
     const auto fits = [&](uint64_t entries) {
         return gridBytes(o.bins_x, o.bins_y) + deviceSetupBytes(d, entries, o.bins_x, o.bins_y) <= budget;
     };
-    return fits(0) && fits(staticEntryCount(d, derived, o.bins_x, o.bins_y));
+    // The cheap limits first: counting the entries is a pass over the fixed modules.
+    const uint64_t fixed = static_cast<uint64_t>(d.module_count) - derived.movable.size();
+    if (!fits(0) || !listsPay(0, fixed, items)) return false;
+    const uint64_t entries = staticEntryCount(d, derived, o.bins_x, o.bins_y);
+    return fits(entries) && listsPay(entries, fixed, items);
 }
 
 // The session's set-up on the device (design_setup.cuh).  The caller's arrays are uploaded as
