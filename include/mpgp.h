@@ -552,7 +552,7 @@ typedef struct mpgp_server_stats {
     int32_t workers;
     int32_t peak_running;           /* most jobs on the device at once */
     uint64_t memory_budget;
-    uint64_t peak_reserved;         /* largest sum of admitted footprints */
+    uint64_t peak_reserved;         /* largest sum of admitted footprints and of set-up scratch beyond them */
     double seconds;                 /* since the server was created */
     int32_t batched;                /* 1: the running jobs' evaluations share batched launches */
     int32_t batch_peak_round;       /* most evaluations one batched round carried */

@@ -294,18 +294,19 @@ uint64_t Engine::gridBytes(int bins_x, int bins_y) {
            (uint64_t{1} << 20);
 }
 
-bool Engine::setsUpOnDevice(const mpgp_design& d, const DerivedDesign& derived, const mpgp_options& o, bool batched) {
+uint64_t Engine::deviceSetupNeed(const mpgp_design& d, const DerivedDesign& derived, const mpgp_options& o,
+                                 bool batched) {
     const int64_t items = static_cast<int64_t>(d.module_count) + d.pin_count;
-    if (items < (batched ? kBatchDeviceSetupItems : kDeviceSetupItems)) return false;
-    const uint64_t budget = o.maximum_cuda_memory_bytes;
-    const auto fits = [&](uint64_t entries) {
-        return gridBytes(o.bins_x, o.bins_y) + deviceSetupBytes(d, entries, o.bins_x, o.bins_y) <= budget;
+    if (items < (batched ? kBatchDeviceSetupItems : kDeviceSetupItems)) return 0;
+    const auto need = [&](uint64_t entries) {
+        return gridBytes(o.bins_x, o.bins_y) + deviceSetupBytes(d, entries, o.bins_x, o.bins_y);
     };
     // The cheap limits first: counting the entries is a pass over the fixed modules.
     const uint64_t fixed = static_cast<uint64_t>(d.module_count) - derived.movable.size();
-    if (!fits(0) || !listsPay(0, fixed, items)) return false;
+    const uint64_t budget = o.maximum_cuda_memory_bytes;
+    if (need(0) > budget || !listsPay(0, fixed, items)) return 0;
     const uint64_t entries = staticEntryCount(d, derived, o.bins_x, o.bins_y);
-    return fits(entries) && listsPay(entries, fixed, items);
+    return need(entries) <= budget && listsPay(entries, fixed, items) ? need(entries) : 0;
 }
 
 // The session's set-up on the device (design_setup.cuh).  The caller's arrays are uploaded as

@@ -172,11 +172,12 @@ public:
     void load(const Problem& problem);
     void loadNets(const Problem& problem, int64_t movable_count);
     void loadParticles(const Problem& problem);
-    // Or from a session's design, set up on the device where setsUpOnDevice says so; the
-    // initial positions are then in scratchPositions().  The choice needs no engine: the host's
-    // set-up begins beside the engine's grid part.
-    static bool setsUpOnDevice(const mpgp_design& design, const DerivedDesign& derived, const mpgp_options& options,
-                               bool batched);
+    // Or from a session's design, set up on the device; the initial positions are then in
+    // scratchPositions().  deviceSetupNeed: the bytes that this holds at most, the engine's grid
+    // part among them, or 0 where the host sets the session up.  The choice needs no engine: the
+    // host's set-up begins beside the engine's grid part.
+    static uint64_t deviceSetupNeed(const mpgp_design& design, const DerivedDesign& derived,
+                                    const mpgp_options& options, bool batched);
     // At least what an engine of this grid holds before its nets and particles are loaded.
     static uint64_t gridBytes(int bins_x, int bins_y);
     void loadDesign(const mpgp_design& design, const DerivedDesign& derived, const mpgp_options& options);

@@ -212,9 +212,37 @@ void Server::work() {
         int status = MPGP_OK;
         std::string error;
         uint64_t reserved_bytes = 0;
+        // A set-up on the device holds more than the job was admitted for: the rest comes out of
+        // the budget while it lasts, and without room for it the host sets the job up.
+        uint64_t setup_extra = 0;
+        const auto grant = [&](uint64_t bytes) {
+            if (bytes <= job->estimate) return true;
+            const std::lock_guard<std::mutex> lock(mutex_);
+            if (bytes - job->estimate > budget_ - std::min(budget_, reserved_)) return false;
+            setup_extra = bytes - job->estimate;
+            reserved_ += setup_extra;
+            stats_.peak_reserved = std::max(stats_.peak_reserved, reserved_);
+            return true;
+        };
+        struct GiveBack {
+            Server& server;
+            uint64_t& bytes;
+            ~GiveBack() { now(); }
+            void now() {
+                if (bytes == 0) return;
+                {
+                    const std::lock_guard<std::mutex> lock(server.mutex_);
+                    server.reserved_ -= bytes;
+                    bytes = 0;
+                }
+                server.ready_.notify_all();
+            }
+        };
         try {
             checkCuda(cudaSetDevice(device_), "Select CUDA device");
-            Session session(job->design, job->options, batch_.get());
+            GiveBack extra{*this, setup_extra};
+            Session session(job->design, job->options, batch_.get(), grant);
+            extra.now();
             reserved_bytes = session.engine() != nullptr ? session.engine()->reservedBytes() : 0;
             int completed = 0;
             while (!session.step(64, &completed)) {

@@ -96,7 +96,8 @@ mpgp_history_row makeHistoryRow(int iteration, const ObjectiveMetrics& m, double
 
 }  // namespace
 
-Session::Session(const mpgp_design& design, const mpgp_options& options, Batch* batch) : options_(options) {
+Session::Session(const mpgp_design& design, const mpgp_options& options, Batch* batch, const SetupGrant& grant)
+    : options_(options) {
     started_ = std::chrono::steady_clock::now();
     validateDesign(design);
     {
@@ -126,7 +127,8 @@ Session::Session(const mpgp_design& design, const mpgp_options& options, Batch* 
         engine_ = std::make_unique<Engine>(grid, options_.cuda_device, options_.maximum_cuda_memory_bytes, batch);
     };
     if (rudy_requested_) batch = nullptr;
-    const bool on_device = Engine::setsUpOnDevice(design, derived_, options_, batch != nullptr);
+    const uint64_t setup_bytes = Engine::deviceSetupNeed(design, derived_, options_, batch != nullptr);
+    const bool on_device = setup_bytes > 0 && (!grant || grant(setup_bytes));
     if (on_device) {
         makeEngine();
         engine_->loadDesign(design, derived_, options_);

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <chrono>
+#include <functional>
 #include <memory>
 #include <vector>
 
@@ -53,7 +54,11 @@ class Session {
 public:
     // With a batch, the session's evaluations run in the batch's shared rounds
     // (a routability run, which the batched launches do not cover, runs on its own).
-    Session(const mpgp_design& design, const mpgp_options& options, Batch* batch = nullptr);
+    // `grant`, if given, is asked before a set-up on the device, with the bytes that it holds at
+    // most (the engine's among them); false sends the session down the host's path.
+    using SetupGrant = std::function<bool(uint64_t bytes)>;
+    Session(const mpgp_design& design, const mpgp_options& options, Batch* batch = nullptr,
+            const SetupGrant& grant = {});
     // Runs up to `iterations` controller iterations; returns true once the run is done.
     bool step(int iterations, int* completed);
     void finish(double* module_x, double* module_y, mpgp_result* result, mpgp_history_row* history, int capacity);

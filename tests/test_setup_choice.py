@@ -61,3 +61,21 @@ def test_budgets_between_the_paths(gpu, bins):
     for run in runs[1:]:
         assert np.array_equal(run.module_x, runs[0].module_x) and np.array_equal(run.module_y, runs[0].module_y)
         assert run.history == runs[0].history
+
+
+@pytest.mark.parametrize("room", [0, 8 << 20, 1 << 30])
+def test_served_set_ups_stay_within_the_budget(gpu, room):
+    """A served job is admitted by its estimate; what a set-up on the device holds beyond that is
+    taken out of the server's budget too, or the host sets the job up."""
+    design = _with_blocks(100, 0.1, seed=6)  # short lists: the device takes it where memory allows
+    options = mp.default_options(bins_x=256, bins_y=256, target_density=0.9, iterations=3)
+    estimate = mp.estimate_bytes(design, options)
+    with mp.PlacementServer(device=0, workers=1, memory_budget=estimate + room, batched=False) as server:
+        job = server.submit(design, options)
+        assert server.wait(job, 120.0)
+        placed, stats = server.take(job)
+        peak = server.stats()["peak_reserved"]
+    assert stats["estimated_bytes"] == estimate and peak <= estimate + room
+    assert (peak > estimate) == (room == 1 << 30)  # 32 MB of slack alone is more than 8 MB
+    alone = mp.GlobalPlacer().run(design, options)
+    assert np.array_equal(placed.module_x, alone.module_x) and np.array_equal(placed.module_y, alone.module_y)
