@@ -20,11 +20,16 @@ namespace mpgp {
 // on a B200 with 16 host CPUs, host set-up against device set-up: 25,000 items 1.49 / 1.47
 // ms, 51,000 1.80 / 1.62, 101,000 2.54 / 2.02, 226,000 5.9 / 2.87, 1.06 million 20.6 / 6.6.  The
 // host's part that is left is the validation, the module lists and sums that must be added in
-// order; below the line both are launch and allocation latency.  Sessions of several threads
-// at once (45,000 cells, 16 iterations each): 4 threads 15 / 9.7 ms, 6 16.5 / 14.9, 10 27 / 25;
-// at 16, as many as host CPUs, the device's read-backs wait for one another's kernels and the
-// host's set-ups are the faster ones, 42 / 44-60.
+// order; below the line both are launch and allocation latency.
 constexpr int64_t kDeviceSetupItems = int64_t{1} << 15;
+// Set-ups on the device at once in a process; a session that finds as many under way is set up
+// on the host.  With many, each one's read-backs wait for the others' kernels and copies, and the
+// helper threads of all of them for host CPUs (16 of these).  Placements of 16 iterations from
+// several threads, without a limit / with 6 / with 4 / all on the host, ms a round of calls: 45,000
+// cells 6 threads 14.4 / 14.3 / 14.9 / 16.7, 10 threads 28 / 22 / 22 / 22, 16 threads 55 / 32.7 /
+// 33.4 / 34, 24 threads 85-108 / 49 / 50 / 51; 16 threads of 100,000 cells 88-129 / 59 / 58 / 65, of
+// 20,000 39-47 / 25 / 25 / 24.5; 8 threads of 210,000 58-64 / 54 / 52 / 63, 4 threads 30 / 29 / 28 / 37.
+constexpr int kDeviceSetupsAtOnce = 6;
 // In a batch the set-ups of several sessions and the running rounds share one stream, so every
 // read-back of a set-up on the device waits for them, while the host's set-ups run on threads of
 // their own.  Batches of 16 iterations, host against device: 24 sessions of 12,000 cells (60,000

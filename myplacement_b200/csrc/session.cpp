@@ -14,6 +14,7 @@
 #include "session.hpp"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <exception>
@@ -94,6 +95,31 @@ mpgp_history_row makeHistoryRow(int iteration, const ObjectiveMetrics& m, double
     return row;
 }
 
+// One of the process's set-ups on the device, if fewer than kDeviceSetupsAtOnce are under way.
+class DeviceSetupSlot {
+public:
+    explicit DeviceSetupSlot(bool wanted) {
+        if (!wanted) return;
+        taken_ = running().fetch_add(1) < kDeviceSetupsAtOnce;
+        if (!taken_) running().fetch_sub(1);
+    }
+    ~DeviceSetupSlot() { release(); }
+    DeviceSetupSlot(const DeviceSetupSlot&) = delete;
+    DeviceSetupSlot& operator=(const DeviceSetupSlot&) = delete;
+    [[nodiscard]] bool taken() const { return taken_; }
+    void release() {
+        if (taken_) running().fetch_sub(1);
+        taken_ = false;
+    }
+
+private:
+    static std::atomic<int>& running() {
+        static std::atomic<int> count{0};
+        return count;
+    }
+    bool taken_ = false;
+};
+
 }  // namespace
 
 Session::Session(const mpgp_design& design, const mpgp_options& options, Batch* batch, const SetupGrant& grant)
@@ -128,10 +154,13 @@ Session::Session(const mpgp_design& design, const mpgp_options& options, Batch* 
     };
     if (rudy_requested_) batch = nullptr;
     const uint64_t setup_bytes = Engine::deviceSetupNeed(design, derived_, options_, batch != nullptr);
-    const bool on_device = setup_bytes > 0 && (!grant || grant(setup_bytes));
+    DeviceSetupSlot slot(setup_bytes > 0);
+    if (slot.taken() && grant && !grant(setup_bytes)) slot.release();
+    const bool on_device = slot.taken();
     if (on_device) {
         makeEngine();
         engine_->loadDesign(design, derived_, options_);
+        slot.release();
     } else {
         // The host problem is built on two threads while this one sets up the engine's grid
         // part on the device (the field solve's bases and buffers need only the grid): the

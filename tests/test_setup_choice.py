@@ -6,6 +6,8 @@ its memory budget is set up on the host.
 """
 from __future__ import annotations
 
+import threading
+
 import numpy as np
 import pytest
 
@@ -79,3 +81,26 @@ def test_served_set_ups_stay_within_the_budget(gpu, room):
     assert (peak > estimate) == (room == 1 << 30)  # 32 MB of slack alone is more than 8 MB
     alone = mp.GlobalPlacer().run(design, options)
     assert np.array_equal(placed.module_x, alone.module_x) and np.array_equal(placed.module_y, alone.module_y)
+
+
+def test_more_sessions_at_once_than_device_set_ups(gpu):
+    """Sessions beyond the set-ups that run on the device at once are set up on the host: each
+    placement is the one it is alone."""
+    options = mp.default_options(bins_x=64, bins_y=64, target_density=0.9, iterations=3)
+    designs = [_with_blocks(50, 0.1, seed=20 + k % 3) for k in range(14)]
+    alone = [mp.GlobalPlacer().run(design, options) for design in designs[:3]]
+    placed = [None] * len(designs)
+
+    def work(k: int) -> None:
+        for _ in range(3):
+            placed[k] = mp.GlobalPlacer().run(designs[k], options)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(designs))]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    for k, run in enumerate(placed):
+        assert np.array_equal(run.module_x, alone[k % 3].module_x)
+        assert np.array_equal(run.module_y, alone[k % 3].module_y)
+        assert run.history == alone[k % 3].history
