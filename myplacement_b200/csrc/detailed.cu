@@ -1160,11 +1160,26 @@ struct RawDesign {
     const double* offset_y = nullptr;
 };
 
-// Raises *bad where validateDesign, or the check of the orientations, would refuse an entry.
-__global__ void __launch_bounds__(kThreads) checkDesignKernel(RawDesign d, int* bad) {
+// Kernels that walk the nets give each eight lanes, and a net of more than kLongNet pins a block
+// of kLongThreads in a launch of its own: eight lanes follow one chain of dependent loads after
+// another.  Two passes over 210,000 cells with a net of 420,000 pins beside the others took 95 ms
+// with eight lanes (72 from the host's lists) and take 5-6, with one of 210,000 pins 15 and 4-4.6.
+constexpr int kLongNet = 512;
+constexpr int kLongThreads = 1024;
+
+// Sets flags[0] where validateDesign, or the check of the orientations, would refuse an entry, and
+// lists the long nets (flags[1] of them; their list has room for one per kLongNet pins).
+__global__ void __launch_bounds__(kThreads) checkDesignKernel(RawDesign d, int* flags, int* long_nets) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     bool good = true;
-    if (i < d.nets) good = d.net_start[i + 1] >= d.net_start[i] && isfinite(d.net_weight[i]);
+    if (i < d.nets) {
+        const long long degree = d.net_start[i + 1] - d.net_start[i];
+        good = degree >= 0 && isfinite(d.net_weight[i]);
+        if (degree > kLongNet) {
+            const int at = atomicAdd(flags + 1, 1);
+            if (at <= d.pins / kLongNet) long_nets[at] = i;  // more only of offsets that are refused
+        }
+    }
     if (i < d.pins) {
         const int m = d.pin_module[i];
         good = good && m >= 0 && m < d.modules && isfinite(d.offset_x[i]) && isfinite(d.offset_y[i]);
@@ -1174,7 +1189,60 @@ __global__ void __launch_bounds__(kThreads) checkDesignKernel(RawDesign d, int* 
         good = good && w >= 0.0 && h >= 0.0 && isfinite(w) && isfinite(h) && isfinite(d.x[i]) && isfinite(d.y[i]);
         if (d.orientation != nullptr) good = good && d.orientation[i] >= 0 && d.orientation[i] <= kOrientationUnknown;
     }
-    if (!good) *bad = 1;
+    if (!good) flags[0] = 1;
+}
+
+// A thread's part of a net: pins first + lane, first + lane + lanes, ... below last.  In the form
+// for long nets a block's, otherwise eight lanes', whose long nets are empty here.
+struct NetShare {
+    int net = -1;  // none: nothing to write either
+    int first = 0, last = 0;
+    int lane = 0;
+};
+template <bool kLong>
+constexpr int kNetLanes = kLong ? kLongThreads : 8;
+template <bool kLong, class Start>
+__device__ __forceinline__ NetShare netShare(int count, const Start* start, const int* long_nets) {
+    NetShare s;
+    const int n = kLong ? long_nets[blockIdx.x] : static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 3);
+    s.lane = static_cast<int>(kLong ? threadIdx.x : threadIdx.x & 7);
+    if (n >= count) return s;
+    s.first = static_cast<int>(start[n]);
+    s.last = static_cast<int>(start[n + 1]);
+    if (!kLong && s.last - s.first > kLongNet) {
+        s.last = s.first;
+    } else {
+        s.net = n;
+    }
+    return s;
+}
+
+// Joins the parts of the net's threads; the first lane has the whole.
+template <bool kLong, class T>
+__device__ __forceinline__ void joinNet(T& v) {
+#pragma unroll
+    for (int lanes = kLong ? 16 : 4; lanes > 0; lanes >>= 1) v.joinLane(lanes);
+    if constexpr (kLong) {
+        static_assert(kLongThreads == 32 * 32, "a warp joins the warps' parts");
+        __shared__ __align__(16) unsigned char parts[32 * sizeof(T)];
+        T* const of_warp = reinterpret_cast<T*>(parts);
+        const int lane = threadIdx.x & 31;
+        if (lane == 0) of_warp[threadIdx.x >> 5] = v;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            v = of_warp[lane];
+#pragma unroll
+            for (int lanes = 16; lanes > 0; lanes >>= 1) v.joinLane(lanes);
+        }
+    }
+}
+
+// Calls launch(whether the form for long nets, blocks, threads) for the nets of at most kLongNet pins and,
+// if there are any, for the longer ones.
+template <class Launch>
+void launchNets(int nets, int long_nets, const Launch& launch) {
+    launch(std::false_type{}, threadBlocks(8 * (static_cast<std::size_t>(nets) + 1)), kThreads);
+    if (long_nets > 0) launch(std::true_type{}, long_nets, kLongThreads);
 }
 
 // deriveDesign's fixed and macro rules: a standard cell is neither.
@@ -1192,16 +1260,18 @@ __global__ void __launch_bounds__(kThreads) detailedModulesKernel(RawDesign d, d
     standard[m] = !fixed && !macro ? 1 : 0;
 }
 
-__global__ void __launch_bounds__(kThreads) detailedNetsKernel(int count, const long long* start, int* start32,
-                                                               int* pin_net, int* pin_index) {
-    const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;  // eight lanes per net
-    if (n > count) return;
-    const long long first = start[n];
-    if ((threadIdx.x & 7) == 0) start32[n] = static_cast<int>(first);
-    if (n == count) return;
-    for (long long p = first + (threadIdx.x & 7); p < start[n + 1]; p += 8) {
-        pin_net[p] = n;
-        pin_index[p] = static_cast<int>(p);
+template <bool kLong>
+__global__ void __launch_bounds__(kNetLanes<kLong> * (kLong ? 1 : kThreads / 8))
+    detailedNetsKernel(int count, const long long* start, const int* long_nets, int* start32, int* pin_net,
+                       int* pin_index) {
+    const NetShare s = netShare<kLong>(count, start, long_nets);
+    if constexpr (!kLong) {
+        const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+        if (s.lane == 0 && n <= count) start32[n] = static_cast<int>(start[n]);
+    }
+    for (int p = s.first + s.lane; p < s.last; p += kNetLanes<kLong>) {
+        pin_net[p] = s.net;
+        pin_index[p] = p;
     }
 }
 
@@ -1241,66 +1311,80 @@ struct LeastTwo {
     }
 };
 
-// Eight lanes per net; the greatest values as the least negated ones.
-__global__ void __launch_bounds__(kThreads) netExtremesKernel(int count, const int* start, const int* pin_module,
-                                                              const double2* offset, const double2* center,
-                                                              const int* owner, NetExtremes* out) {
-    const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-    const int last = n < count ? start[n + 1] : 0;
+// The greatest values as the least negated ones.  Nets of more than `longest` pins are left out: a
+// window with one of them is not evaluated.
+struct LeastFour {
     LeastTwo low_x, low_y, high_x, high_y;
-    for (int p = (n < count ? start[n] : 0) + static_cast<int>(threadIdx.x & 7); p < last; p += 8) {
+    __device__ __forceinline__ void joinLane(int lanes) {
+        low_x.joinLane(lanes);
+        low_y.joinLane(lanes);
+        high_x.joinLane(lanes);
+        high_y.joinLane(lanes);
+    }
+};
+template <bool kLong>
+__global__ void __launch_bounds__(kNetLanes<kLong> * (kLong ? 1 : kThreads / 8))
+    netExtremesKernel(int count, const int* start, const int* long_nets, int longest, const int* pin_module,
+                      const double2* offset, const double2* center, const int* owner, NetExtremes* out) {
+    const NetShare s = netShare<kLong>(count, start, long_nets);
+    if (kLong && s.last - s.first > longest) return;  // the whole block
+    const int last = s.last - s.first > longest ? s.first : s.last;
+    LeastFour v;
+#pragma unroll (kLong ? 4 : 1)
+    for (int p = s.first + s.lane; p < last; p += kNetLanes<kLong>) {
         const int m = pin_module[p];
         const double2 c = center[m];
         const double2 o = offset[p];
         const int w = owner[m];
         const double x = c.x + o.x;
         const double y = c.y + o.y;
-        low_x.join(x, kLargest, w);
-        low_y.join(y, kLargest, w);
-        high_x.join(-x, kLargest, w);
-        high_y.join(-y, kLargest, w);
+        v.low_x.join(x, kLargest, w);
+        v.low_y.join(y, kLargest, w);
+        v.high_x.join(-x, kLargest, w);
+        v.high_y.join(-y, kLargest, w);
     }
-#pragma unroll
-    for (int lanes = 4; lanes > 0; lanes >>= 1) {
-        low_x.joinLane(lanes);
-        low_y.joinLane(lanes);
-        high_x.joinLane(lanes);
-        high_y.joinLane(lanes);
-    }
-    if (n < count && (threadIdx.x & 7) == 0) {
-        out[n] = NetExtremes{make_double2(low_x.first, low_y.first),    make_double2(-high_x.first, -high_y.first),
-                             make_double2(low_x.next, low_y.next),      make_double2(-high_x.next, -high_y.next),
-                             make_int2(low_x.owner, low_y.owner), make_int2(high_x.owner, high_y.owner)};
+    joinNet<kLong>(v);
+    if (s.net >= 0 && s.lane == 0) {
+        out[s.net] = NetExtremes{make_double2(v.low_x.first, v.low_y.first),
+                                 make_double2(-v.high_x.first, -v.high_y.first),
+                                 make_double2(v.low_x.next, v.low_y.next),
+                                 make_double2(-v.high_x.next, -v.high_y.next),
+                                 make_int2(v.low_x.owner, v.low_y.owner),
+                                 make_int2(v.high_x.owner, v.high_y.owner)};
     }
 }
 
-// One net's weighted HPWL (Placement::netTerm; zero below two pins), eight lanes per net.
-__global__ void __launch_bounds__(kThreads) netTermsKernel(int count, const int* start, const int* pin_module,
-                                                           const double2* offset, const double2* center,
-                                                           const double* weight, double* term) {
-    const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-    const int first = n < count ? start[n] : 0;
-    const int last = n < count ? start[n + 1] : 0;
+// One net's weighted HPWL (Placement::netTerm; zero below two pins).
+struct NetBox {
     double min_x = INFINITY, max_x = -INFINITY, min_y = INFINITY, max_y = -INFINITY;
-    for (int p = first + static_cast<int>(threadIdx.x & 7); p < last; p += 8) {
+    __device__ __forceinline__ void joinLane(int lanes) {
+        min_x = fmin(min_x, __shfl_xor_sync(0xffffffffu, min_x, lanes));
+        max_x = fmax(max_x, __shfl_xor_sync(0xffffffffu, max_x, lanes));
+        min_y = fmin(min_y, __shfl_xor_sync(0xffffffffu, min_y, lanes));
+        max_y = fmax(max_y, __shfl_xor_sync(0xffffffffu, max_y, lanes));
+    }
+};
+template <bool kLong>
+__global__ void __launch_bounds__(kNetLanes<kLong> * (kLong ? 1 : kThreads / 8))
+    netTermsKernel(int count, const int* start, const int* long_nets, const int* pin_module, const double2* offset,
+                   const double2* center, const double* weight, double* term) {
+    const NetShare s = netShare<kLong>(count, start, long_nets);
+    NetBox box;
+#pragma unroll (kLong ? 4 : 1)
+    for (int p = s.first + s.lane; p < s.last; p += kNetLanes<kLong>) {
         const double2 c = center[pin_module[p]];
         const double2 o = offset[p];
         const double x = c.x + o.x;
         const double y = c.y + o.y;
-        min_x = x < min_x ? x : min_x;
-        max_x = max_x < x ? x : max_x;
-        min_y = y < min_y ? y : min_y;
-        max_y = max_y < y ? y : max_y;
+        box.min_x = x < box.min_x ? x : box.min_x;
+        box.max_x = box.max_x < x ? x : box.max_x;
+        box.min_y = y < box.min_y ? y : box.min_y;
+        box.max_y = box.max_y < y ? y : box.max_y;
     }
-#pragma unroll
-    for (int offset_lane = 4; offset_lane > 0; offset_lane >>= 1) {
-        min_x = fmin(min_x, __shfl_xor_sync(0xffffffffu, min_x, offset_lane));
-        max_x = fmax(max_x, __shfl_xor_sync(0xffffffffu, max_x, offset_lane));
-        min_y = fmin(min_y, __shfl_xor_sync(0xffffffffu, min_y, offset_lane));
-        max_y = fmax(max_y, __shfl_xor_sync(0xffffffffu, max_y, offset_lane));
-    }
-    if (n < count && (threadIdx.x & 7) == 0) {
-        term[n] = last - first < 2 ? 0.0 : __dmul_rn(weight[n], (max_x - min_x) + (max_y - min_y));
+    joinNet<kLong>(box);
+    if (s.net >= 0 && s.lane == 0) {
+        const double span = (box.max_x - box.min_x) + (box.max_y - box.min_y);
+        term[s.net] = s.last - s.first < 2 ? 0.0 : __dmul_rn(weight[s.net], span);
     }
 }
 
@@ -1659,15 +1743,18 @@ bool placeOnDevice(const mpgp_design& d, const int32_t* row_orientation, const m
     const double* net_weight = raw.net_weight;
     int* changed = scratch.array<int>(kMaxRounds + kRoundsPerCheck + 1);
     PassCounts* counts = scratch.array<PassCounts>(1);
-    const PinnedBlock readback(sizeof(PassCounts) + sizeof(int), "detailed-placement counters");
+    int* long_nets = scratch.array<int>(p_count / kLongNet + 1);
+    const PinnedBlock readback(sizeof(PassCounts) + 2 * sizeof(int), "detailed-placement counters");
     PassCounts* const host_counts = reinterpret_cast<PassCounts*>(readback.data());
     int* const host_changed = reinterpret_cast<int*>(readback.data() + sizeof(PassCounts));
     // The checks, before any kernel follows an index.
-    checkCuda(cudaMemsetAsync(changed, 0, sizeof(int), stream), "check the design");
-    checkDesignKernel<<<threadBlocks(std::max({m_count, n_count, p_count})), kThreads, 0, stream>>>(raw, changed);
-    checkCuda(cudaMemcpyAsync(host_changed, changed, sizeof(int), cudaMemcpyDeviceToHost, stream), "check the design");
+    checkCuda(cudaMemsetAsync(changed, 0, 2 * sizeof(int), stream), "check the design");
+    checkDesignKernel<<<threadBlocks(std::max({m_count, n_count, p_count})), kThreads, 0, stream>>>(raw, changed,
+                                                                                                       long_nets);
+    checkCuda(cudaMemcpyAsync(host_changed, changed, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream), "check the design");
     checkCuda(cudaStreamSynchronize(stream), "check the design");
-    if (*host_changed != 0) return false;
+    if (host_changed[0] != 0) return false;
+    const int long_count = host_changed[1];
 
     double2* center = scratch.array<double2>(m_count);
     double2* moved_center = scratch.array<double2>(m_count);
@@ -1680,8 +1767,10 @@ bool placeOnDevice(const mpgp_design& d, const int32_t* row_orientation, const m
     int* net_pin_start = scratch.array<int>(n_count + 1);
     int* pin_net = scratch.array<int>(p_count);
     int* pin_index = scratch.array<int>(p_count);
-    detailedNetsKernel<<<threadBlocks(8 * (n_count + 1)), kThreads, 0, stream>>>(nets, raw.net_start, net_pin_start, pin_net,
-                                                                                pin_index);
+    launchNets(nets, long_count, [&](auto is_long, int blocks, int threads) {
+        detailedNetsKernel<decltype(is_long)::value><<<blocks, threads, 0, stream>>>(nets, raw.net_start, long_nets,
+                                                                                    net_pin_start, pin_net, pin_index);
+    });
     double2* raw_offset = scratch.array<double2>(p_count);
     double2* pin_offset = scratch.array<double2>(p_count);
     rawOffsetsKernel<<<threadBlocks(p_count), kThreads, 0, stream>>>(pins, raw.offset_x, raw.offset_y, raw_offset);
@@ -1691,8 +1780,10 @@ bool placeOnDevice(const mpgp_design& d, const int32_t* row_orientation, const m
         turnedOffsetsKernel<<<threadBlocks(p_count), kThreads, 0, stream>>>(pins, raw_offset, pin_module, turn, pin_offset);
     };
     const auto netTerms = [&](double* term) {
-        netTermsKernel<<<threadBlocks(8 * n_count), kThreads, 0, stream>>>(nets, net_pin_start, pin_module, pin_offset,
-                                                                           center, net_weight, term);
+        launchNets(nets, long_count, [&](auto is_long, int blocks, int threads) {
+            netTermsKernel<decltype(is_long)::value><<<blocks, threads, 0, stream>>>(
+                nets, net_pin_start, long_nets, pin_module, pin_offset, center, net_weight, term);
+        });
         checkCuda(cudaGetLastError(), "net terms");
     };
     turnOffsets();
@@ -1789,6 +1880,8 @@ bool placeOnDevice(const mpgp_design& d, const int32_t* row_orientation, const m
                  on);
         return total;
     };
+    const int longest = static_cast<int>(
+        std::min<uint64_t>(options.maximum_net_degree, static_cast<uint64_t>(std::numeric_limits<int>::max())));
     double hpwl_before = 0.0;
     uint64_t evaluated = 0, permutations = 0, accepted = 0;
     for (int pass = 0; pass < options.passes; ++pass) {
@@ -1838,8 +1931,10 @@ bool placeOnDevice(const mpgp_design& d, const int32_t* row_orientation, const m
             if (pass > 0) turnOffsets();
             const WindowArrays arrays{windows.modules, windows.start_x, windows.bottom,
                                       windows.spacing, windows.net_start, windows.nets};
-            netExtremesKernel<<<threadBlocks(8 * n_count), kThreads, 0, stream>>>(nets, net_pin_start, pin_module, pin_offset,
-                                                                                  center, windows.owner, extremes);
+            launchNets(nets, longest > kLongNet ? long_count : 0, [&](auto is_long, int blocks, int threads) {
+                netExtremesKernel<decltype(is_long)::value><<<blocks, threads, 0, stream>>>(
+                    nets, net_pin_start, long_nets, longest, pin_module, pin_offset, center, windows.owner, extremes);
+            });
             windowOrdersKernel<true><<<warps, 32 * kWindowsPerBlock, 0, stream>>>(
                 center, size, pin_module, pin_offset, net_pin_start, net_weight, arrays, total, windows.kind,
                 options.improvement_epsilon, best_order, decided[0], moved_center,
