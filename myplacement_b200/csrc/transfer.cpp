@@ -19,10 +19,12 @@ namespace {
 constexpr std::size_t kHubSlots = 16;
 constexpr std::size_t kHubSlotBytes = std::size_t{512} << 10;
 constexpr std::size_t kSmallestSlot = std::size_t{32} << 10;
-constexpr std::size_t kFallbackSlot = std::size_t{64} << 10;
 constexpr std::size_t kOwnSlots = 2;
-// Arrays from this size on move through the hub: below, waking helpers costs about as much as
-// one thread needs for the copy.
+// Arrays from this size on move through the hub: below, the hand-over to the helpers costs more
+// than they save.  Evaluations with a gradient (three arrays) and without (one), this object's
+// slots against the hub, us: 80 KB 98 / 105 and 57 / 63, 235 KB 121 / 128 and 65 / 70, 390 KB 158 /
+// 152 and 75 / 80, 510 KB 201 / 178 and 83 / 92, 780 KB 271 / 214 and 113 / 105, 1.25 MB 384 / 265
+// and 157 / 122.
 constexpr std::size_t kLargeBytes = std::size_t{512} << 10;
 constexpr int kHelpers = 6;
 constexpr std::chrono::microseconds kSpin{300};  // a helper's wait for the next job before it sleeps
@@ -145,10 +147,12 @@ void TransferHub::close() noexcept {
 }
 
 HostTransfer::HostTransfer(cudaStream_t stream, std::size_t bytes) : stream_(stream) {
-    // A small array takes one slot; a large one uses its own slots only beside another thread's call.
-    if (bytes >= kLargeBytes) hub_ = TransferHub::shared();
-    own_slot_bytes_ = hub_ != nullptr ? kFallbackSlot : std::max(kSmallestSlot, (bytes + 4095) / 4096 * 4096);
-    own_ = PinnedBlock(kOwnSlots * own_slot_bytes_, "pinned transfer slots");
+    if (bytes >= kLargeBytes) {
+        hub_ = TransferHub::shared();
+    } else {  // a small array takes one slot
+        own_slot_bytes_ = std::max(kSmallestSlot, (bytes + 4095) / 4096 * 4096);
+        own_ = PinnedBlock(kOwnSlots * own_slot_bytes_, "pinned transfer slots");
+    }
     events_.resize(hub_ != nullptr ? kHubSlots : kOwnSlots);
     for (cudaEvent_t& e : events_) checkCuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "Create event");
 }
@@ -163,6 +167,7 @@ HostTransfer::Call::Call(HostTransfer* transfer) : transfer_(transfer) {
     if (transfer_ == nullptr) return;
     HostTransfer& t = *transfer_;
     t.helped_ = t.hub_ != nullptr && t.hub_->acquire();
+    t.direct_ = t.hub_ != nullptr && !t.helped_;
     t.moved_ = 0;
     t.ring_ = t.helped_ ? t.hub_->ring() : t.own_.data();
     t.slots_ = t.helped_ ? kHubSlots : kOwnSlots;
@@ -188,6 +193,12 @@ struct HostTransfer::Download {
 };
 
 bool HostTransfer::upload(const double* source, double* destination, std::size_t count, bool check) {
+    if (direct_) {
+        if (check && !allFinite(source, count)) return false;
+        checkCuda(cudaMemcpyAsync(destination, source, count * sizeof(double), cudaMemcpyHostToDevice, stream_),
+                  "Upload to the device");
+        return true;
+    }
     return move(reinterpret_cast<const unsigned char*>(source), reinterpret_cast<unsigned char*>(destination),
                 count * sizeof(double), check);
 }
@@ -274,6 +285,10 @@ bool HostTransfer::arrived(std::size_t k) {
 }
 
 void HostTransfer::startDownload(const std::vector<Piece>& pieces) {
+    if (direct_) {
+        pieces_ = pieces;
+        return;
+    }
     chunks_.clear();
     issued_ = 0;
     in_flight_ = true;
@@ -314,6 +329,13 @@ void HostTransfer::cancelDownload() noexcept {
 }
 
 void HostTransfer::finishDownload() {
+    if (direct_) {
+        for (const Piece& p : pieces_) {
+            checkCuda(cudaMemcpyAsync(p.host, p.device, p.bytes, cudaMemcpyDeviceToHost, stream_), "Download from the device");
+        }
+        checkCuda(cudaStreamSynchronize(stream_), "Download from the device");
+        return;
+    }
     Download& d = *download_;
     const std::size_t chunks = chunks_.size();
     std::size_t done = 0, out = 0;  // chunks that have arrived, and (in order) been copied
