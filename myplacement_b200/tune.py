@@ -9,14 +9,18 @@ doubles the CTAs a launch needs.  For every grid size this tuner runs the
 adaptive controller on a synthetic design (the mid design's structure at about
 16k cells) with that many bins per side, once with each split, times every
 contraction launch with CUDA events (the engine's own profiler) and keeps the
-split with the least device time per iteration.  With --write it stores the
-table in csrc/tuned_splits.inc, which the library compiles in (rebuild after).
+split with the least device time per iteration.  A square grid of at most 128 bins a
+side solves its field in one launch without them; other grids that contract over
+that length do not, so its splits are timed with the staged solve.  With --write it
+stores the table in csrc/tuned_splits.inc, which the library compiles in (rebuild
+after).
 """
 from __future__ import annotations
 
 import argparse
 import ctypes as C
 import json
+import os
 import sys
 from pathlib import Path
 
@@ -67,6 +71,25 @@ def contraction_us_per_iteration(design, bins: int, warmup: int, iterations: int
     return 1e3 * sum(stats[f][1] for f in FAMILIES) / iterations, launches
 
 
+def timed_contractions(design, bins: int, warmup: int, iterations: int) -> float:
+    """Device microseconds per iteration of the contractions at `bins`: as the engine runs them, or with
+    the staged field solve where it launches none."""
+    us, launches = contraction_us_per_iteration(design, bins, warmup, iterations)
+    if launches == 0:
+        chosen = os.environ.get("MPGP_FIELD_SOLVE")
+        os.environ["MPGP_FIELD_SOLVE"] = "staged"
+        try:
+            us, launches = contraction_us_per_iteration(design, bins, warmup, iterations)
+        finally:
+            if chosen is None:
+                del os.environ["MPGP_FIELD_SOLVE"]
+            else:
+                os.environ["MPGP_FIELD_SOLVE"] = chosen
+    if launches == 0:
+        raise RuntimeError(f"no contraction launches to time at {bins} bins")
+    return us
+
+
 def tune(sizes: list[int], warmup: int, iterations: int, repeats: int) -> dict:
     from . import placer
     from .design import workload
@@ -76,17 +99,19 @@ def tune(sizes: list[int], warmup: int, iterations: int, repeats: int) -> dict:
     design = design.copy_with_positions(x, y)
     start = get_splits()
     report = {}
-    for bins in sizes:
-        timings = {}
-        for split in (1, 2):
-            set_splits({**start, bins: split})
-            runs = [contraction_us_per_iteration(design, bins, warmup, iterations)[0] for _ in range(repeats)]
-            timings[split] = float(np.median(runs))
-        best = min(timings, key=timings.get)
-        report[bins] = {"split": best, "us_per_iteration": timings}
-        print(f"{bins:5d} bins: split 1 {timings[1]:9.1f} us, split 2 {timings[2]:9.1f} us per iteration -> {best}",
-              flush=True)
-    set_splits(start)
+    try:
+        for bins in sizes:
+            timings = {}
+            for split in (1, 2):
+                set_splits({**start, bins: split})
+                runs = [timed_contractions(design, bins, warmup, iterations) for _ in range(repeats)]
+                timings[split] = float(np.median(runs))
+            best = min(timings, key=timings.get)
+            report[bins] = {"split": best, "us_per_iteration": timings}
+            print(f"{bins:5d} bins: split 1 {timings[1]:9.1f} us, split 2 {timings[2]:9.1f} us per iteration -> {best}",
+                  flush=True)
+    finally:
+        set_splits(start)
     return report
 
 
