@@ -45,6 +45,9 @@ KERNEL_OF_FAMILY = {"dct_forward": "tcGemmKernel", "dct_inverse": "tcGemmKernel"
                     "wirelength": "wirelengthKernel", "scatter": "scatterKernel",
                     "metrics": "metricsSplitKernel", "gather": "gatherKernel", "reduce": "reduceKernel",
                     "vector": "velocityKernel", "dct_split": "splitSourceKernel", "rudy": "rudy kernels"}
+# Grids of at most this many bins a side solve their field in one launch (unless
+# MPGP_FIELD_SOLVE chooses another solve), which the engine times as the field families too.
+ONE_LAUNCH_BINS = 128
 # Iteration budget of the end-to-end runs (early stop on): large enough that the run stops on its
 # own once the design overflow is <= 0.10 (the reference's default budget of 280 iterations ends
 # this design at overflow 0.13).
@@ -155,6 +158,15 @@ class ClockSampler:
                            "(the steps, then the 256 MiB flush write as load)"}
 
 
+def one_launch_field(bins_x: int, bins_y: int) -> bool:
+    return max(bins_x, bins_y) <= ONE_LAUNCH_BINS and os.environ.get("MPGP_FIELD_SOLVE") not in ("staged", "banded")
+
+
+def kernel_of_family(family: str, bins_x: int, bins_y: int) -> str:
+    kernel = KERNEL_OF_FAMILY.get(family, family)
+    return "fieldSmallKernel" if kernel == "fieldKernel" and one_launch_field(bins_x, bins_y) else kernel
+
+
 def algorithmic_units(design, particles: int, bins_x: int, bins_y: int) -> dict:
     """Per-launch algorithmic bytes (HBM-bound families) or FLOPs (DCT) of each kernel family.
 
@@ -164,11 +176,15 @@ def algorithmic_units(design, particles: int, bins_x: int, bins_y: int) -> dict:
     two (inverse) M x N x K contractions at 2 flops per multiply-add (the transform's
     own work, not the three tensor-core products of the split); a banded field launch
     is the two forward contractions, and with a gradient the two inverse ones along y (an
-    inverse launch only those two);
+    inverse launch only those two); the one-launch solve of small grids runs the inverse ones
+    along x as well;
     the source split reads 4 B and writes two 2-byte planes per bin.
     """
     pins, nets, bins = design.pin_count, design.net_count, bins_x * bins_y
     m, n = bins_y, bins_x
+    # The inverse contractions inside a field launch: M1 and M2 (two m x n x m) in the banded one;
+    # T, U, Ex and Ey (two along each axis) in the one-launch solve.
+    inverse = 2 * 2.0 * m * n * ((m + n) if one_launch_field(bins_x, bins_y) else m)
     return {
         "wirelength": ("hbm", 20 * pins + 8 * nets + 8 * particles),
         "scatter": ("hbm", 20 * particles + 24 * bins),
@@ -176,10 +192,10 @@ def algorithmic_units(design, particles: int, bins_x: int, bins_y: int) -> dict:
         "gather": ("hbm", 80 * particles),
         "dct_forward": ("tensor", 2.0 * m * n * (n + m) / 2.0),
         "dct_inverse": ("tensor", 2 * 2.0 * m * n * (n + m) / 2.0),
-        # The banded solve: Q = S Cx^T and rho_hat = Cy Q, then M1 and M2 (two m x n x m) with a gradient.
+        # Q = S Cx^T and rho_hat = Cy Q, then the inverse ones with a gradient.
         "field_forward": ("tensor", 2.0 * m * n * (n + m)),
-        "field_gradient": ("tensor", 2.0 * m * n * (n + m) + 2 * 2.0 * m * n * m),
-        "field_inverse": ("tensor", 2 * 2.0 * m * n * m),
+        "field_gradient": ("tensor", 2.0 * m * n * (n + m) + inverse),
+        "field_inverse": ("tensor", inverse),
         "reduce": ("hbm", 8 * 64),
         "vector": ("hbm", 48 * particles),
         "dct_split": ("hbm", 4 * bins + 4 * bins),
@@ -309,7 +325,7 @@ def run_mine(args) -> None:
     groups = {}
     for name, (n, ms) in warm_stats.items():
         if n > 0:
-            groups.setdefault(KERNEL_OF_FAMILY.get(name, name), []).append(name)
+            groups.setdefault(kernel_of_family(name, bins, bins), []).append(name)
     dominant = max(groups, key=lambda g: sum(warm_stats[f][1] for f in groups[g])) if groups else "tcGemmKernel"
     families = groups.get(dominant, ["dct_forward", "dct_inverse"])
     session.set_profiling(families)
