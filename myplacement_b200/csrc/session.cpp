@@ -760,8 +760,8 @@ void Session::finish(double* module_x, double* module_y, mpgp_result* result, mp
             result_.best_checkpoint_overflow = chosen.overflow;
         }
         // applyPositions (AdaptiveGlobalPlacer.cpp:185-198); then calculateHpwl /
-        // calculateDensity at the restored placement (:938-940), which run while the movable
-        // modules' centres come back.
+        // calculateDensity at the restored placement (:938-940), and behind them on the stream the
+        // copy of the movable modules' centres.
         const std::size_t movable = derived_.movable.size();
         engine_->clampPositions(final_positions, cand_);
         EvalRequest q = givenRequest(cand_, false, penalty_, nullptr, nullptr, false, false, false, -1.0);
