@@ -408,6 +408,7 @@ __global__ void __launch_bounds__(kThreads) noAllocClearKernel(float2* pin_gradi
 // Degree classes of the net pass: lanes per net (a class of G lanes holds the nets of
 // degree <= G that no smaller class takes), 32 lanes and a pin loop above 32.
 constexpr int kNoAllocClasses = 6;
+constexpr int kNoAllocRun = 8;  // consecutive nets of a chunk: a sector of their offsets
 __device__ __forceinline__ int noAllocClass(int degree) {
     return degree <= 2 ? 0 : degree <= 4 ? 1 : degree <= 8 ? 2 : degree <= 16 ? 3 : degree <= 32 ? 4 : 5;
 }
@@ -532,8 +533,10 @@ __device__ __forceinline__ void callerGroup(const CallerNets& a, bool net_ok, in
     }
 }
 
-// The net pass.  A block takes chunks of `chunk` (at most 256) consecutive nets, sorts each
-// chunk's nets by degree class in shared memory (a stable counting sort, so the totals do
+// The net pass.  A block takes chunks of `chunk` (at most 256) nets, runs of kNoAllocRun consecutive
+// ones, each a grid's blocks after the one before: large nets that stand next to one another are
+// spread over the blocks (1,000 nets of 500 pins behind 200,000 of two: 77 us a call; with chunks
+// of consecutive nets 133 nets of 750 pins took 333 us, a warp per net 111).  It sorts each chunk's nets by degree class in shared memory (a stable counting sort, so the totals do
 // not depend on timing) and hands the classes' units -- 32 two-pin nets, 32 / G nets of a
 // G-lane class, one larger net -- to its warps.
 // Bound by the issue of the exponentials, divisions and shuffles (0.5 warp instructions a
@@ -557,12 +560,17 @@ __global__ void __launch_bounds__(kThreads) noAllocNetKernel(CallerNets a, int n
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     double values[2] = {0.0, 0.0};
-    for (int first = blockIdx.x * chunk; first < net_count; first += gridDim.x * chunk) {
+    const int blocks = static_cast<int>(gridDim.x);
+    for (int base = 0; base < net_count; base += blocks * chunk) {
+        const auto net_of = [&](int l) {
+            return base + (l / kNoAllocRun * blocks + static_cast<int>(blockIdx.x)) * kNoAllocRun + l % kNoAllocRun;
+        };
         const int local = static_cast<int>(threadIdx.x);
         int c = kNoAllocClasses;  // not evaluated
-        if (local < chunk && first + local < net_count) {
-            const int begin = a.net_pin_start[first + local];
-            const int end = a.net_pin_start[first + local + 1];
+        const int net = net_of(local);
+        if (local < chunk && net < net_count) {
+            const int begin = a.net_pin_start[net];
+            const int end = a.net_pin_start[net + 1];
             // Malformed CSR: never write outside scratch.  Single-pin nets contribute
             // nothing; their slots stay zero.
             if (begin >= 0 && end <= pin_count && end >= begin && end - begin >= 2) c = noAllocClass(end - begin);
@@ -601,7 +609,7 @@ __global__ void __launch_bounds__(kThreads) noAllocNetKernel(CallerNets a, int n
         }
         __syncthreads();
         int units_before = 0;
-        for (int k = 0; k < kNoAllocClasses; ++k) {
+        for (int k = 0; k < kNoAllocClasses - 1; ++k) {
             const int lanes = noAllocLanes(k);
             const int per_unit = 32 / lanes;
             const int low = class_first[k];
@@ -613,24 +621,52 @@ __global__ void __launch_bounds__(kThreads) noAllocNetKernel(CallerNets a, int n
                 const bool net_ok = i < nets;
                 const int l = net_ok ? order[low + i] : 0;
                 const int begin = begin_of[l], degree = degree_of[l];
+                const int of = net_of(l);
                 switch (k) {
-                    case 0: callerPair(a, net_ok, first + l, begin, values[0], values[1]); break;
-                    case 1: callerGroup<4>(a, net_ok, first + l, begin, degree, values[0], values[1]); break;
-                    case 2: callerGroup<8>(a, net_ok, first + l, begin, degree, values[0], values[1]); break;
-                    case 3: callerGroup<16>(a, net_ok, first + l, begin, degree, values[0], values[1]); break;
-                    case 4: callerGroup<32>(a, net_ok, first + l, begin, degree, values[0], values[1]); break;
-                    default:
-                        waitForPrior();  // the slots are cleared
-                        netOnWarp(a.load, begin, begin + degree, static_cast<float>(a.net_weight[first + l]), a.gamma,
-                                  a.inv_gamma, true, PinStore{a.pin_gradient}, values[0], values[1]);
-                        break;
+                    case 0: callerPair(a, net_ok, of, begin, values[0], values[1]); break;
+                    case 1: callerGroup<4>(a, net_ok, of, begin, degree, values[0], values[1]); break;
+                    case 2: callerGroup<8>(a, net_ok, of, begin, degree, values[0], values[1]); break;
+                    case 3: callerGroup<16>(a, net_ok, of, begin, degree, values[0], values[1]); break;
+                    default: callerGroup<32>(a, net_ok, of, begin, degree, values[0], values[1]); break;
                 }
             }
             units_before += units;
         }
+        const int large = class_first[kNoAllocClasses - 1];
+        for (int u = large + (warp - units_before % kWarps + kWarps) % kWarps; u < class_first[kNoAllocClasses]; u += kWarps) {
+            const int l = order[u];
+            const int begin = begin_of[l];
+            waitForPrior();  // the slots are cleared
+            netOnWarp(a.load, begin, begin + degree_of[l], static_cast<float>(a.net_weight[net_of(l)]), a.gamma,
+                      a.inv_gamma, true, PinStore{a.pin_gradient}, values[0], values[1]);
+        }
         __syncthreads();  // before the next chunk overwrites the lists
     }
     waitForPrior();  // every block: the grid completes after the clearing pass
+    const bool is_max[2] = {false, false};
+    blockReduce<2>(values, is_max);
+    if (threadIdx.x == 0) {
+        partials[2 * blockIdx.x + 0] = values[0];
+        partials[2 * blockIdx.x + 1] = values[1];
+    }
+}
+
+// A warp per net, for netlists whose nets have more than 32 pins on average: the sort finds
+// nothing to group there, and this kernel's 48 registers let an SM hold a fifth block (30,303
+// nets of 33 pins, the whole call: 62 us, 72 with the chunks).
+__global__ void __launch_bounds__(kThreads) noAllocWarpKernel(CallerNets a, int net_count, int pin_count,
+                                                             double* partials) {
+    releaseNext();
+    double values[2] = {0.0, 0.0};
+    const int warps = static_cast<int>((gridDim.x * blockDim.x) >> 5);
+    waitForPrior();  // the slots are cleared
+    for (int net = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5); net < net_count; net += warps) {
+        const int begin = a.net_pin_start[net];
+        const int end = a.net_pin_start[net + 1];
+        if (begin < 0 || end > pin_count || end < begin || end - begin < 2) continue;  // as the chunks' checks
+        netOnWarp(a.load, begin, end, static_cast<float>(a.net_weight[net]), a.gamma, a.inv_gamma, true,
+                  PinStore{a.pin_gradient}, values[0], values[1]);
+    }
     const bool is_max[2] = {false, false};
     blockReduce<2>(values, is_max);
     if (threadIdx.x == 0) {
@@ -703,10 +739,16 @@ __global__ void __launch_bounds__(kThreads) noAllocParticleKernel(const int* par
     }
 }
 
-// Nets per chunk of the net pass: 256, and fewer while that leaves SMs without a block.
-int noAllocChunk(int net_count) {
+// Nets per chunk of the net pass: 256, and fewer while that leaves SMs without a block, or while
+// nets of more than 32 pins, a warp each, may be more than the blocks' warps: with two pins in every
+// other net (pins - 2 nets) / 31 of them; four blocks fit an SM.
+int noAllocChunk(int net_count, int pin_count) {
     constexpr int kBlocksWanted = 2 * 148;
-    return std::min(kThreads, std::max(32, (ceilDiv(net_count, kBlocksWanted) + 31) / 32 * 32));
+    constexpr int kWave = 4 * 148;
+    const int chunk = std::min(kThreads, std::max(32, (ceilDiv(net_count, kBlocksWanted) + 31) / 32 * 32));
+    const int large = std::min(net_count, (pin_count - 2 * std::min(net_count, pin_count / 2)) / 31);
+    const int wanted = std::max(1, std::min(kWave, ceilDiv(large, kThreads / 32)));
+    return std::min(chunk, (ceilDiv(std::max(1, net_count), wanted) + kNoAllocRun - 1) / kNoAllocRun * kNoAllocRun);
 }
 
 }  // namespace
@@ -747,8 +789,10 @@ void launchWirelengthNoAlloc(const NoAllocWirelengthArgs& a) {
     const cudaStream_t stream = static_cast<cudaStream_t>(a.stream);
     const float gamma = static_cast<float>(std::max(a.smoothing, kEpsilon));
     const float inv_gamma = static_cast<float>(1.0 / std::max(a.smoothing, kEpsilon));
-    const int chunk = noAllocChunk(a.net_count);
-    const int net_blocks = std::min(kNoAllocMaxBlocks, std::max(1, ceilDiv(a.net_count, chunk)));
+    const int chunk = noAllocChunk(a.net_count, a.pin_count);
+    const bool large_nets = a.pin_count / 32 > a.net_count;  // on average
+    const int net_blocks =
+        std::min(kNoAllocMaxBlocks, std::max(1, ceilDiv(a.net_count, large_nets ? kThreads / 32 : chunk)));
     unsigned char* bytes = static_cast<unsigned char*>(scratch);
     float2* pin_gradient = reinterpret_cast<float2*>(bytes);
     const CallerNets nets{CallerPinLoader{reinterpret_cast<const double2*>(a.positions), a.pin_particle,
@@ -760,8 +804,14 @@ void launchWirelengthNoAlloc(const NoAllocWirelengthArgs& a) {
     const int clear_blocks = std::max(1, std::min(ceilDiv(a.pin_count, 8 * kThreads), 4 * 148));
     noAllocClearKernel<<<clear_blocks, kThreads, 0, stream>>>(pin_gradient, a.pin_count);
     checkCuda(cudaGetLastError(), "Launch the allocation-free clearing pass");
-    launchChained("Launch the allocation-free net pass", noAllocNetKernel, dim3(net_blocks), dim3(kThreads), 0, stream,
-                  nets, a.net_count, a.pin_count, chunk, reinterpret_cast<double*>(bytes + kNoAllocPinBytes));
+    double* const partials = reinterpret_cast<double*>(bytes + kNoAllocPinBytes);
+    if (large_nets) {
+        launchChained("Launch the allocation-free net pass", noAllocWarpKernel, dim3(net_blocks), dim3(kThreads), 0,
+                      stream, nets, a.net_count, a.pin_count, partials);
+    } else {
+        launchChained("Launch the allocation-free net pass", noAllocNetKernel, dim3(net_blocks), dim3(kThreads), 0,
+                      stream, nets, a.net_count, a.pin_count, chunk, partials);
+    }
     const int particle_blocks = std::max(1, ceilDiv(a.particle_count, kThreads));
     launchChained("Launch the allocation-free particle pass", noAllocParticleKernel, dim3(particle_blocks),
                   dim3(kThreads), 0, stream, a.particle_pin_start, a.particle_pins, a.pin_particle, a.particle_count,
