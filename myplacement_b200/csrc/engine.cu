@@ -1466,7 +1466,7 @@ RudyReport Engine::rudyEvaluate(const double2* positions, bool validation) {
     checkCuda(cudaMemcpyAsync(host_rudy_, rudy_scalars_, 5 * sizeof(double), cudaMemcpyDeviceToHost, stream_),
               "Download RUDY scalars");
     const std::size_t bins = static_cast<std::size_t>(g.columns) * static_cast<std::size_t>(g.rows);
-    std::vector<double> utilization;
+    std::vector<double>& utilization = rudy_utilization_;
     if (with_capacity) {
         utilization.resize(bins);
         checkCuda(cudaMemcpyAsync(utilization.data(), g.utilization, bins * sizeof(double), cudaMemcpyDeviceToHost,
