@@ -3,8 +3,9 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <iterator>
-#include <map>
+#include <list>
 #include <mutex>
 #include <utility>
 
@@ -13,11 +14,15 @@
 namespace mpgp {
 namespace {
 
-// The kept blocks by size.  Never destroyed: at process exit the driver may be gone
-// before a static destructor would run, and it releases the memory itself.
+// The kept blocks, the one given back last in front.  Never destroyed: at process exit the driver
+// may be gone before a static destructor would run, and it releases the memory itself.
 struct Kept {
+    struct Block {
+        std::size_t size;
+        unsigned char* data;
+    };
     std::mutex mutex;
-    std::multimap<std::size_t, unsigned char*> blocks;
+    std::list<Block> blocks;
     std::size_t bytes = 0;
 };
 
@@ -40,9 +45,9 @@ PinnedBlock::PinnedBlock(std::size_t bytes, const char* what) {
     Kept& k = kept();
     {
         const std::lock_guard<std::mutex> lock(k.mutex);
-        const auto found = k.blocks.find(size);
+        const auto found = std::find_if(k.blocks.begin(), k.blocks.end(), [&](const Kept::Block& b) { return b.size == size; });
         if (found != k.blocks.end()) {
-            data_ = found->second;
+            data_ = found->data;
             size_ = size;
             k.blocks.erase(found);
             k.bytes -= size;
@@ -68,18 +73,23 @@ void PinnedBlock::release() noexcept {
     if (data_ == nullptr) return;
     unsigned char* p = std::exchange(data_, nullptr);
     Kept& k = kept();
+    std::list<Kept::Block> freed;
     {
         const std::lock_guard<std::mutex> lock(k.mutex);
-        if (k.bytes + size_ <= kPinnedKept) {
-            try {
-                k.blocks.emplace(size_, p);
-                k.bytes += size_;
-                return;
-            } catch (...) {  // no memory for the entry: free the block below
-            }
+        try {
+            k.blocks.push_front({size_, p});
+            k.bytes += size_;
+            p = nullptr;
+        } catch (...) {  // no memory for the entry: free the block below
+        }
+        // The blocks that nobody has asked for the longest make room.
+        while (k.bytes > kPinnedKept) {
+            k.bytes -= k.blocks.back().size;
+            freed.splice(freed.end(), k.blocks, std::prev(k.blocks.end()));
         }
     }
-    cudaFreeHost(p);
+    for (const Kept::Block& b : freed) cudaFreeHost(b.data);
+    if (p != nullptr) cudaFreeHost(p);
 }
 
 }  // namespace mpgp

@@ -4,7 +4,11 @@
 // one is made and releases with the last one: a process that places one design after
 // another paid for that chunk (3 ms, and 0.7 ms to release it) in every session, for a
 // record of a few hundred bytes.  Blocks given back here stay pinned for the next
-// engine, up to kPinnedKept bytes in all; beyond that they are freed.
+// engine, up to kPinnedKept bytes in all; beyond that those that nobody has asked for the
+// longest are freed.  (The backends' 8 MB ring has to find room: with 16 MB, and the block that
+// came back freed instead, it was pinned anew with every first backend once others had left their
+// slots here.  Making a backend of 45,000 cells then took 11 ms and takes 3.3, from four threads
+// at once 28 and 5.2; 6.3 and 7.5 with allocations per backend.)
 //
 // Measured on one B200 box, whole placements with 16 iterations: 7.1 ms with allocations
 // per session and 3.8 ms with kept blocks for 5,000 cells, 28.9 and 25.6 ms for 210,000;
@@ -15,7 +19,7 @@
 
 namespace mpgp {
 
-constexpr std::size_t kPinnedKept = std::size_t{16} << 20;
+constexpr std::size_t kPinnedKept = std::size_t{32} << 20;
 
 // One block of at least `bytes` pinned bytes (portable: usable from every device, and
 // addressable by kernels), its contents undefined.  Movable; given back when destroyed.
